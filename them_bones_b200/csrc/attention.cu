@@ -22,137 +22,11 @@ namespace bones {
 constexpr float kQkEps = 1.1920928955078125e-07f;   // 2^-23
 
 // ---------------------------------------------------------------------------------------------------------------
-// RoPE + QK-norm pre-pass: qkv [M, 3A] -> qk [M, 2A]  (A = H * D; q-hat then k-hat).  One warp per (row, head, q|k).
+// RoPE + QK-norm pre-pass: qkv [M, 3A] -> qk [M, 2A]  (A = H * D; q-hat then k-hat), and its backward
+// (u = rope(x), r = rsqrt(mean(u^2)+eps), xhat = u r;  du = r (dxhat - xhat mean(dxhat xhat));  dx = rope^T(du)).
 // ---------------------------------------------------------------------------------------------------------------
-template <int D>
-__global__ void rope_qknorm_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
-                                       const float* __restrict__ sinT, __nv_bfloat16* __restrict__ qk, long long M, int T, int H) {
-  constexpr int HALF = D / 2, PER = HALF / 32;
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= M * H * 2) return;
-  const int which = (int)(w % 2), h = (int)((w / 2) % H);
-  const long long row = w / (2 * H);
-  const int t = (int)(row % T);
-  const long long A = (long long)H * D;
-  const __nv_bfloat16* src = qkv + row * 3 * A + which * A + (long long)h * D;
-  __nv_bfloat16* dst = qk + row * 2 * A + which * A + (long long)h * D;
-  float y1[PER], y2[PER], ss = 0.f;
-  float x1[PER], x2[PER], cs[PER], sn[PER];
-  if constexpr (PER == 2) {   // 4-byte / 8-byte vector accesses: a warp reads 128 contiguous bytes per half
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + 2 * lane));
-    const float2 c2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + HALF + 2 * lane));
-    const float2 cc = *reinterpret_cast<const float2*>(cosT + (long long)t * HALF + 2 * lane);
-    const float2 sc = *reinterpret_cast<const float2*>(sinT + (long long)t * HALF + 2 * lane);
-    x1[0] = a.x; x1[1] = a.y; x2[0] = c2.x; x2[1] = c2.y; cs[0] = cc.x; cs[1] = cc.y; sn[0] = sc.x; sn[1] = sc.y;
-  } else {
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int i = lane * PER + e;
-      x1[e] = __bfloat162float(src[i]); x2[e] = __bfloat162float(src[HALF + i]);
-      cs[e] = cosT[(long long)t * HALF + i]; sn[e] = sinT[(long long)t * HALF + i];
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < PER; ++e) {
-    y1[e] = x1[e] * cs[e] + x2[e] * sn[e];
-    y2[e] = -x1[e] * sn[e] + x2[e] * cs[e];
-    ss += y1[e] * y1[e] + y2[e] * y2[e];
-  }
-  ss = warp_sum(ss);
-  const float r = rsqrtf(ss / D + kQkEps);
-  if constexpr (PER == 2) {
-    *reinterpret_cast<__nv_bfloat162*>(dst + 2 * lane) = __floats2bfloat162_rn(y1[0] * r, y1[1] * r);
-    *reinterpret_cast<__nv_bfloat162*>(dst + HALF + 2 * lane) = __floats2bfloat162_rn(y2[0] * r, y2[1] * r);
-  } else {
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int i = lane * PER + e;
-      dst[i] = __float2bfloat16(y1[e] * r);
-      dst[HALF + i] = __float2bfloat16(y2[e] * r);
-    }
-  }
-}
-
-// Backward of the pre-pass: dq-hat/dk-hat (fp32 [M, 2A]) + dv (bf16 [M, A]) -> dqkv (bf16 [M, 3A]).
-// u = rope(x), r = rsqrt(mean(u^2)+eps), xhat = u r;  du = r (dxhat - xhat mean(dxhat xhat));  dx = rope^T(du).
-template <int D>
-__global__ void rope_qknorm_bwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
-                                       const float* __restrict__ sinT, const float* __restrict__ dqk,
-                                       const __nv_bfloat16* __restrict__ dv, __nv_bfloat16* __restrict__ dqkv, long long M, int T,
-                                       int H) {
-  constexpr int HALF = D / 2, PER = HALF / 32;
-  const long long w = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  const int lane = threadIdx.x & 31;
-  if (w >= M * H * 3) return;
-  const int which = (int)(w % 3), h = (int)((w / 3) % H);
-  const long long row = w / (3 * H);
-  const long long A = (long long)H * D;
-  __nv_bfloat16* out = dqkv + row * 3 * A + which * A + (long long)h * D;
-  if (which == 2) {   // values pass straight through
-    const __nv_bfloat16* g = dv + row * A + (long long)h * D;
-    if constexpr (D == 128) {
-      *reinterpret_cast<uint2*>(out + 4 * lane) = *reinterpret_cast<const uint2*>(g + 4 * lane);
-    } else {
-      for (int i = lane; i < D; i += 32) out[i] = g[i];
-    }
-    return;
-  }
-  const int t = (int)(row % T);
-  const __nv_bfloat16* src = qkv + row * 3 * A + which * A + (long long)h * D;
-  const float* g = dqk + row * 2 * A + which * A + (long long)h * D;
-  float y1[PER], y2[PER], g1[PER], g2[PER], cs[PER], sn[PER], x1[PER], x2[PER], ss = 0.f, dot = 0.f;
-  if constexpr (PER == 2) {
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + 2 * lane));
-    const float2 c2 = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(src + HALF + 2 * lane));
-    const float2 cc = *reinterpret_cast<const float2*>(cosT + (long long)t * HALF + 2 * lane);
-    const float2 sc = *reinterpret_cast<const float2*>(sinT + (long long)t * HALF + 2 * lane);
-    const float2 ga = *reinterpret_cast<const float2*>(g + 2 * lane);
-    const float2 gb = *reinterpret_cast<const float2*>(g + HALF + 2 * lane);
-    x1[0] = a.x; x1[1] = a.y; x2[0] = c2.x; x2[1] = c2.y; cs[0] = cc.x; cs[1] = cc.y; sn[0] = sc.x; sn[1] = sc.y;
-    g1[0] = ga.x; g1[1] = ga.y; g2[0] = gb.x; g2[1] = gb.y;
-  } else {
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int i = lane * PER + e;
-      x1[e] = __bfloat162float(src[i]); x2[e] = __bfloat162float(src[HALF + i]);
-      cs[e] = cosT[(long long)t * HALF + i]; sn[e] = sinT[(long long)t * HALF + i];
-      g1[e] = g[i]; g2[e] = g[HALF + i];
-    }
-  }
-#pragma unroll
-  for (int e = 0; e < PER; ++e) {
-    y1[e] = x1[e] * cs[e] + x2[e] * sn[e];
-    y2[e] = -x1[e] * sn[e] + x2[e] * cs[e];
-    ss += y1[e] * y1[e] + y2[e] * y2[e];
-    dot += y1[e] * g1[e] + y2[e] * g2[e];
-  }
-  ss = warp_sum(ss);
-  dot = warp_sum(dot);
-  const float r = rsqrtf(ss / D + kQkEps);
-  const float m = dot * r * r / D;     // mean(dxhat * xhat) * r, with xhat = u r
-  float o1[PER], o2[PER];
-#pragma unroll
-  for (int e = 0; e < PER; ++e) {
-    const float du1 = r * (g1[e] - y1[e] * m), du2 = r * (g2[e] - y2[e] * m);
-    o1[e] = du1 * cs[e] - du2 * sn[e];
-    o2[e] = du1 * sn[e] + du2 * cs[e];
-  }
-  if constexpr (PER == 2) {
-    *reinterpret_cast<__nv_bfloat162*>(out + 2 * lane) = __floats2bfloat162_rn(o1[0], o1[1]);
-    *reinterpret_cast<__nv_bfloat162*>(out + HALF + 2 * lane) = __floats2bfloat162_rn(o2[0], o2[1]);
-  } else {
-#pragma unroll
-    for (int e = 0; e < PER; ++e) {
-      const int i = lane * PER + e;
-      out[i] = __float2bfloat16(o1[e]);
-      out[HALF + i] = __float2bfloat16(o2[e]);
-    }
-  }
-}
-
-// head_dim 128 fast paths: eight lanes per head vector (16-byte accesses: elements [8 l, 8 l + 8) of the first half and
-// their rotate-half partners in the second half), four head vectors per warp, reductions over the 8-lane group.
+// D / 16 lanes per head vector (16-byte accesses: elements [8 l, 8 l + 8) of the first half and their rotate-half partners
+// in the second half), reductions over that group of lanes.
 __device__ __forceinline__ void ld8_bf16(const __nv_bfloat16* p, float* f) {
   const uint4 u = *reinterpret_cast<const uint4*>(p);
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
@@ -172,35 +46,40 @@ __device__ __forceinline__ void ld8_f32(const float* p, float* f) {
   const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
   f[0] = a.x; f[1] = a.y; f[2] = a.z; f[3] = a.w; f[4] = b.x; f[5] = b.y; f[6] = b.z; f[7] = b.w;
 }
-__device__ __forceinline__ float group8_sum(float v) {
-  v += __shfl_xor_sync(0xffffffffu, v, 1);
-  v += __shfl_xor_sync(0xffffffffu, v, 2);
-  v += __shfl_xor_sync(0xffffffffu, v, 4);
+template <int LANES>
+__device__ __forceinline__ float group_sum(float v) {
+#pragma unroll
+  for (int o = 1; o < LANES; o <<= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// Eight threads per (row, head); a thread takes its 16 elements of the query head and of the key head, which share the
+// D / 16 threads per (row, head); a thread takes its 16 elements of the query head and of the key head, which share the
 // rotation tables, so that 64 bytes of loads per thread are in flight (with 32 the kernel sat at 0.7 of the copy rate).
-__global__ void rope_qknorm_fwd128_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
-                                          const float* __restrict__ sinT, __nv_bfloat16* __restrict__ qk, long long M, int T, int H) {
-  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;     // (row, head)
-  const int l8 = threadIdx.x & 7;
+// `counter`: the work-item counter of the attention launch that follows on the stream, zeroed here (a memset of its own is
+// one more launch on calls whose kernels take a few microseconds).
+template <int D>
+__global__ void rope_qknorm_fwd_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT, const float* __restrict__ sinT,
+                                       __nv_bfloat16* __restrict__ qk, int* counter, long long M, int T, int H) {
+  constexpr int LANES = D / 16, HALF = D / 2;
+  if (counter && blockIdx.x == 0 && threadIdx.x == 0) *counter = 0;
+  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;     // (row, head)
+  const int l8 = threadIdx.x & (LANES - 1);
   const long long total = M * H;
   const bool live = item < total;
   const long long it = live ? item : total - 1;
   const int h = (int)(it % H);
   const long long row = it / H;
   const int t = (int)(row % T);
-  const long long A = (long long)H * 128;
-  const __nv_bfloat16* src = qkv + row * 3 * A + (long long)h * 128 + l8 * 8;
+  const long long A = (long long)H * D;
+  const __nv_bfloat16* src = qkv + row * 3 * A + (long long)h * D + l8 * 8;
   float x1[2][8], x2[2][8], cs[8], sn[8];
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     ld8_bf16(src + w * A, x1[w]);
-    ld8_bf16(src + w * A + 64, x2[w]);
+    ld8_bf16(src + w * A + HALF, x2[w]);
   }
-  ld8_f32(cosT + (long long)t * 64 + l8 * 8, cs);
-  ld8_f32(sinT + (long long)t * 64 + l8 * 8, sn);
+  ld8_f32(cosT + (long long)t * HALF + l8 * 8, cs);
+  ld8_f32(sinT + (long long)t * HALF + l8 * 8, sn);
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     float y1[8], y2[8];
@@ -211,14 +90,14 @@ __global__ void rope_qknorm_fwd128_kernel(const __nv_bfloat16* __restrict__ qkv,
       y2[e] = -x1[w][e] * sn[e] + x2[w][e] * cs[e];
       ss += y1[e] * y1[e] + y2[e] * y2[e];
     }
-    ss = group8_sum(ss);
-    const float r = rsqrtf(ss * (1.0f / 128.0f) + kQkEps);
+    ss = group_sum<LANES>(ss);
+    const float r = rsqrtf(ss * (1.0f / D) + kQkEps);
 #pragma unroll
     for (int e = 0; e < 8; ++e) { y1[e] *= r; y2[e] *= r; }
     if (live) {
-      __nv_bfloat16* dst = qk + row * 2 * A + w * A + (long long)h * 128 + l8 * 8;
+      __nv_bfloat16* dst = qk + row * 2 * A + w * A + (long long)h * D + l8 * 8;
       st8_bf16(dst, y1);
-      st8_bf16(dst + 64, y2);
+      st8_bf16(dst + HALF, y2);
     }
   }
 }
@@ -257,8 +136,8 @@ __global__ void rope_qknorm_bwd128_kernel(const __nv_bfloat16* __restrict__ qkv,
     ss += y1[e] * y1[e] + y2[e] * y2[e];
     dot += y1[e] * g1[e] + y2[e] * g2[e];
   }
-  ss = group8_sum(ss);
-  dot = group8_sum(dot);
+  ss = group_sum<8>(ss);
+  dot = group_sum<8>(dot);
   const float r = rsqrtf(ss * (1.0f / 128.0f) + kQkEps);
   const float m = dot * r * r * (1.0f / 128.0f);
   float o1[8], o2[8];
@@ -281,18 +160,20 @@ __global__ void rope_qknorm_bwd128_kernel(const __nv_bfloat16* __restrict__ qkv,
 
 // Same backward for bf16 dq-hat | dk-hat (the two-kernel attention backward writes them in bf16 and puts dV straight into
 // its third of dqkv): only the q and k thirds are produced here.
-__global__ void rope_qknorm_bwd128_bf16_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
+template <int D>
+__global__ void rope_qknorm_bwd_bf16_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
                                                const float* __restrict__ sinT, const __nv_bfloat16* __restrict__ dqk,
                                                __nv_bfloat16* __restrict__ dqkv, long long M, int T, int H) {
-  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 3;     // (row, head): query and key head
-  const int l8 = threadIdx.x & 7;
+  constexpr int LANES = D / 16, HALF = D / 2;
+  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;     // (row, head): query and key head
+  const int l8 = threadIdx.x & (LANES - 1);
   const long long total = M * H;
   const bool live = item < total;
   const long long it = live ? item : total - 1;
   const int h = (int)(it % H);
   const long long row = it / H;
-  const long long A = (long long)H * 128;
-  const long long col = (long long)h * 128 + l8 * 8;
+  const long long A = (long long)H * D;
+  const long long col = (long long)h * D + l8 * 8;
   const __nv_bfloat16* src = qkv + row * 3 * A + col;
   const __nv_bfloat16* g = dqk + row * 2 * A + col;
   const int t = (int)(row % T);
@@ -300,12 +181,12 @@ __global__ void rope_qknorm_bwd128_bf16_kernel(const __nv_bfloat16* __restrict__
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     ld8_bf16(src + w * A, x1[w]);
-    ld8_bf16(src + w * A + 64, x2[w]);
+    ld8_bf16(src + w * A + HALF, x2[w]);
     ld8_bf16(g + w * A, g1[w]);
-    ld8_bf16(g + w * A + 64, g2[w]);
+    ld8_bf16(g + w * A + HALF, g2[w]);
   }
-  ld8_f32(cosT + (long long)t * 64 + l8 * 8, cs);
-  ld8_f32(sinT + (long long)t * 64 + l8 * 8, sn);
+  ld8_f32(cosT + (long long)t * HALF + l8 * 8, cs);
+  ld8_f32(sinT + (long long)t * HALF + l8 * 8, sn);
 #pragma unroll
   for (int w = 0; w < 2; ++w) {
     float y1[8], y2[8];
@@ -317,10 +198,10 @@ __global__ void rope_qknorm_bwd128_bf16_kernel(const __nv_bfloat16* __restrict__
       ss += y1[e] * y1[e] + y2[e] * y2[e];
       dot += y1[e] * g1[w][e] + y2[e] * g2[w][e];
     }
-    ss = group8_sum(ss);
-    dot = group8_sum(dot);
-    const float r = rsqrtf(ss * (1.0f / 128.0f) + kQkEps);
-    const float m = dot * r * r * (1.0f / 128.0f);
+    ss = group_sum<LANES>(ss);
+    dot = group_sum<LANES>(dot);
+    const float r = rsqrtf(ss * (1.0f / D) + kQkEps);
+    const float m = dot * r * r * (1.0f / D);
     float o1[8], o2[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -331,13 +212,13 @@ __global__ void rope_qknorm_bwd128_bf16_kernel(const __nv_bfloat16* __restrict__
     if (live) {
       __nv_bfloat16* out = dqkv + row * 3 * A + w * A + col;
       st8_bf16(out, o1);
-      st8_bf16(out + 64, o2);
+      st8_bf16(out + HALF, o2);
     }
   }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
-// forward attention, head_dim 128
+// forward attention, head_dim 128 or 64
 // ---------------------------------------------------------------------------------------------------------------
 struct AttnParams {
   int B, T, H;
@@ -352,10 +233,8 @@ struct AttnParams {
   int* items;        // device counter the persistent CTAs draw their work items from (zero at launch)
 };
 
-constexpr int AT = 128;                    // tile edge (queries and keys)
-constexpr int AD = 128;                    // head dim
-constexpr uint32_t TILE_BYTES = AT * AD * 2;   // 32 KB: two 128-byte-swizzled atoms of [128 rows][64 cols]
-constexpr uint32_t ATOM_BYTES = TILE_BYTES / 2;
+constexpr int AT = 128;                         // tile edge (queries and keys)
+constexpr uint32_t ATOM_BYTES = AT * 64 * 2;    // 16 KB: one 128-byte-swizzled atom of [128 rows][64 cols]; a tile has D / 64
 
 __device__ __forceinline__ int attn_first_tile(const AttnParams& p, int b, int qt) {
   int lo = 0;
@@ -374,8 +253,6 @@ __device__ __forceinline__ int attn_first_tile(const AttnParams& p, int b, int q
 //   TMEM: S/P buffers at columns 0 and 128 (by running tile count), O buffers at 256 and 384 (by item parity).
 //   smem: Q x 2 (item parity), K x 2 and V x 3 stages (running tile count): a K stage is free again once its S tile is
 //   done, a V stage only after its O MMAs, so K and V rings of different depth keep the loads a full tile ahead.
-__device__ int g_fwd_items;      // item counter of the persistent forward (one launch at a time per device)
-
 struct FwdItem {
   int qt, h, b, kt0, n;
 };
@@ -396,8 +273,16 @@ constexpr uint32_t FWD_SLACK = 768;           // room for aligning the tiles to 
                                              // the scratch fill the rest of the 227 KB)
 constexpr int FWD_THREADS = 64 + 32 * FWD_SW;
 
+// D: head dim (64-wide heads on 128-wide tiles with zero halves did twice the MMAs and ten PyTorch passes of padding: a
+// forward and backward of 4 x 256 tokens, 4 heads took 314 us, 155 us natively).  T may have any value (padding the sequences
+// to whole tiles in PyTorch took 157 of the 271 us of 8 x 1777 tokens, 10 heads; 100 us without): the tensor maps are three-dimensional ([B, T, columns]), so the rows of a last tile
+// past the sequence's end arrive as zeros instead of the next sequence's values; their keys lie behind every real query and
+// are masked by causality, their queries are computed and not stored.
+template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
+  constexpr uint32_t TILE_BYTES = (D / 64) * ATOM_BYTES;
+  constexpr int DT = D / 4;                            // output columns a softmax thread drains
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -429,8 +314,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + kBars + 224);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int A = p.H * AD;
-  const int n_tiles = p.T / AT;
+  const int A = p.H * D;
+  const int n_tiles = (p.T + AT - 1) / AT;
   const int total = n_tiles * p.H * p.B;
 
   if (threadIdx.x == 0) {
@@ -482,33 +367,33 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       FwdItem im = fwd_item(p, w, n_tiles);
       im.kt0 = warp_uniform(im.kt0);
       im.n = im.qt - im.kt0 + 1;
-      const int qb = it & 1, row0 = im.b * p.T;
+      const int qb = it & 1;
       if (it >= 2 && !dead) dead = !mbar_wait(q_free(qb), (uint32_t)(((it - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
       if (elect_one() && !dead) {
         mbar_arrive_expect_tx(q_full(qb), TILE_BYTES);
-        tma_load_2d(sQ(qb), &tm_qk, q_full(qb), im.h * AD, row0 + im.qt * AT);
-        tma_load_2d(sQ(qb) + ATOM_BYTES, &tm_qk, q_full(qb), im.h * AD + 64, row0 + im.qt * AT);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qb) + c * ATOM_BYTES, &tm_qk, q_full(qb), im.h * D + c * 64, im.qt * AT, im.b);
       }
       for (int j = 0; j < im.n; ++j, ++g) {
         const int ks = g & 1, vs = g % 3;
-        const int r = row0 + (im.kt0 + j) * AT;
+        const int r = (im.kt0 + j) * AT;
         if (g >= 2 && !dead) dead = !mbar_wait(k_free(ks), (uint32_t)(((g - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(k_full(ks), TILE_BYTES);
-          tma_load_2d(sK(ks), &tm_qk, k_full(ks), A + im.h * AD, r);
-          tma_load_2d(sK(ks) + ATOM_BYTES, &tm_qk, k_full(ks), A + im.h * AD + 64, r);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sK(ks) + c * ATOM_BYTES, &tm_qk, k_full(ks), A + im.h * D + c * 64, r, im.b);
         }
         if (g >= 3 && !dead) dead = !mbar_wait(v_free(vs), (uint32_t)(((g - 3) / 3) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(v_full(vs), TILE_BYTES);
-          tma_load_2d(sV(vs), &tm_v, v_full(vs), 2 * A + im.h * AD, r);
-          tma_load_2d(sV(vs) + ATOM_BYTES, &tm_v, v_full(vs), 2 * A + im.h * AD + 64, r);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sV(vs) + c * ATOM_BYTES, &tm_v, v_full(vs), 2 * A + im.h * D + c * 64, r, im.b);
         }
       }
     }
   } else if (warp == 1) {
     const uint32_t idesc_s = umma_idesc_f16(128, 128, 1, 0, 0);   // Q (K-major) x K (K-major)
-    const uint32_t idesc_o = umma_idesc_f16(128, 128, 1, 0, 1);   // P (TMEM) x V (MN-major)
+    const uint32_t idesc_o = umma_idesc_f16(128, D, 1, 0, 1);   // P (TMEM) x V (MN-major)
     // the O += P V step of a tile is issued one tile late, behind the next tile's S, so the softmax of tile g runs
     // under the S MMAs of tile g+1.  P(g) sits in TMEM as packed bf16 pairs over the S(g) columns it was computed
     // from (each softmax warp packs its 32 columns into the first 16 of its own range).
@@ -551,7 +436,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
         const uint64_t qdesc0 = umma_smem_desc(sQ(qb), 0, 1024, kLayoutSw128), kdesc0 = umma_smem_desc(sK(sb), 0, 1024, kLayoutSw128);
         if (elect_one() && !dead) {
 #pragma unroll
-          for (int k = 0; k < 8; ++k) {
+          for (int k = 0; k < D / 16; ++k) {
             const uint64_t off = (uint64_t)(((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4);
             umma_f16(tS(sb), qdesc0 + off, kdesc0 + off, idesc_s, k ? 1u : 0u);
           }
@@ -586,20 +471,23 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       if (!__all_sync(0xffffffffu, got)) return false;
       tc_fence_after();
       {
-        uint32_t v[32];
+        uint32_t v[DT];
         __syncwarp();
-        BONES_TMEM_LD32(tO(ob) + lane_addr + (uint32_t)c0, v);
+        if constexpr (DT == 32) BONES_TMEM_LD32(tO(ob) + lane_addr + (uint32_t)(part * DT), v);
+        else BONES_TMEM_LD16(tO(ob) + lane_addr + (uint32_t)(part * DT), v);
         tmem_ld_wait();
-        uint4 u[4];
+        uint4 u[DT / 8];
 #pragma unroll
-        for (int gq = 0; gq < 4; ++gq) {
+        for (int gq = 0; gq < DT / 8; ++gq) {
           u[gq].x = pack_bf16(__uint_as_float(v[gq * 8 + 0]) * pend_inv, __uint_as_float(v[gq * 8 + 1]) * pend_inv);
           u[gq].y = pack_bf16(__uint_as_float(v[gq * 8 + 2]) * pend_inv, __uint_as_float(v[gq * 8 + 3]) * pend_inv);
           u[gq].z = pack_bf16(__uint_as_float(v[gq * 8 + 4]) * pend_inv, __uint_as_float(v[gq * 8 + 5]) * pend_inv);
           u[gq].w = pack_bf16(__uint_as_float(v[gq * 8 + 6]) * pend_inv, __uint_as_float(v[gq * 8 + 7]) * pend_inv);
         }
-        st_global_v8(pend_y, u[0], u[1]);                // one full 32-byte sector per store
-        st_global_v8(pend_y + 16, u[2], u[3]);
+        if (pend_y) {
+#pragma unroll
+          for (int gq = 0; gq < DT / 8; gq += 2) st_global_v8(pend_y + gq * 8, u[gq], u[gq + 1]);      // full 32-byte sectors
+        }
       }
       tc_fence_before();
       __syncwarp();
@@ -612,9 +500,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       const int w = ok ? item_take(ring_bars, ring_slots, it, abort_flag, p.err) : -1;
       if (w < 0) break;
       const FwdItem im = fwd_item(p, w, n_tiles);
-      const int qpos = im.qt * AT + r, row0 = im.b * p.T;
+      const int qpos = im.qt * AT + r;
+      const bool real = qpos < p.T;
       int lo = 0;
-      if (p.doc_start) lo = p.doc_start[(long long)im.b * p.T + qpos];
+      if (p.doc_start && real) lo = p.doc_start[(long long)im.b * p.T + qpos];
       float l = 0.f;
       for (int j = 0; j < im.n; ++j, ++g) {
         const int sb = g & 1;
@@ -660,11 +549,11 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       asm volatile("bar.sync 1, 512;" ::: "memory");
       l = (lsum[r] + lsum[AT + r]) + (lsum[2 * AT + r] + lsum[3 * AT + r]);      // the same order in all four threads
       asm volatile("bar.sync 1, 512;" ::: "memory");      // nobody rewrites the scratch before everybody has read it
-      if (part == 0) p.lse[((long long)im.b * p.H + im.h) * p.T + qpos] = logf(l) + p.shift_ln;
+      if (part == 0 && real) p.lse[((long long)im.b * p.H + im.h) * p.T + qpos] = logf(l) + p.shift_ln;
       pend = true;
       pend_it = it;
       pend_inv = 1.0f / l;
-      pend_y = p.y + ((long long)(row0 + qpos)) * A + (long long)im.h * AD + c0;
+      pend_y = real ? p.y + ((long long)im.b * p.T + qpos) * A + (long long)im.h * D + part * DT : nullptr;
     }
     if (ok && pend) drain();
   }
@@ -680,11 +569,35 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   }
 }
 
-static int tmap_rows_2d(CUtensorMap* out, const void* ptr, long long rows, long long cols) {
-  uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows};
-  uint64_t strides[1] = {(uint64_t)cols * 2};
-  uint32_t box[2] = {64, 128};
-  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+// [B, T, cols] bf16 rows, boxes of 64 columns x 128 rows of one sequence; rows past T read as zeros
+static int tmap_rows_3d(CUtensorMap* out, const void* ptr, int B, int T, long long cols) {
+  uint64_t dims[3] = {(uint64_t)cols, (uint64_t)T, (uint64_t)B};
+  uint64_t strides[2] = {(uint64_t)cols * 2, (uint64_t)cols * 2 * (uint64_t)T};
+  uint32_t box[3] = {64, 128, 1};
+  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <int D>
+static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tv, const AttnParams& p, int sms, cudaStream_t s) {
+  constexpr size_t smem = (size_t)(D / 64) * ATOM_BYTES * 7 + 256 + 2048 + FWD_SLACK;   // tiles, barriers, row-sum scratch, alignment slack
+  static bool attr_done = false;
+  if (!attr_done) {
+    BONES_CHECK(cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    attr_done = true;
+  }
+  const long long items = (long long)((p.T + AT - 1) / AT) * p.H * p.B;
+  const unsigned grid = (unsigned)(items < sms ? items : sms);       // persistent: one CTA per SM
+  attn_fwd_kernel<D><<<grid, FWD_THREADS, smem, s>>>(tq, tv, p);
+  return (int)cudaGetLastError();
+}
+
+template <int D>
+static int launch_rope_fwd(const void* qkv, const float* cosT, const float* sinT, void* qk, int* counter, long long M, int T, int H,
+                           cudaStream_t s) {
+  const long long threads = M * H * (D / 16);
+  rope_qknorm_fwd_kernel<D><<<(unsigned)((threads + 255) / 256), 256, 0, s>>>((const __nv_bfloat16*)qkv, cosT, sinT, (__nv_bfloat16*)qk,
+                                                                              counter, M, T, H);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace bones
@@ -692,84 +605,68 @@ static int tmap_rows_2d(CUtensorMap* out, const void* ptr, long long rows, long 
 extern "C" {
 using namespace bones;
 
-int bones_rope_qknorm_fwd(const void* qkv, const float* cosT, const float* sinT, void* qk, long long M, int T, int H, int D, void* stream) {
-  const long long warps = M * H * 2;
-  const unsigned grid = (unsigned)((warps + 7) / 8);
-  if (D == 128) {
-    const long long threads = M * H * 8;
-    rope_qknorm_fwd128_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)qkv, cosT, sinT,
-                                                                                                   (__nv_bfloat16*)qk, M, T, H);
-  }
-  else if (D == 64)
-    rope_qknorm_fwd_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)qkv, cosT, sinT, (__nv_bfloat16*)qk, M, T, H);
-  else
-    return -2;
-  return (int)cudaGetLastError();
+int bones_rope_qknorm_fwd(const void* qkv, const float* cosT, const float* sinT, void* qk, int* counter, long long M, int T, int H, int D,
+                          void* stream) {
+  if (D == 128) return launch_rope_fwd<128>(qkv, cosT, sinT, qk, counter, M, T, H, (cudaStream_t)stream);
+  if (D == 64) return launch_rope_fwd<64>(qkv, cosT, sinT, qk, counter, M, T, H, (cudaStream_t)stream);
+  return -2;
 }
 
+// fp32 dq-hat | dk-hat (the single-kernel backward), head_dim 128 only
 int bones_rope_qknorm_bwd(const void* qkv, const float* cosT, const float* sinT, const float* dqk, const void* dv, void* dqkv, long long M,
                           int T, int H, int D, void* stream) {
-  const long long warps = M * H * 3;
-  const unsigned grid = (unsigned)((warps + 7) / 8);
-  if (D == 128) {
-    const long long threads = M * 3 * H * 8;
-    rope_qknorm_bwd128_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-        (const __nv_bfloat16*)qkv, cosT, sinT, dqk, (const __nv_bfloat16*)dv, (__nv_bfloat16*)dqkv, M, T, H);
-  }
-  else if (D == 64)
-    rope_qknorm_bwd_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)qkv, cosT, sinT, dqk, (const __nv_bfloat16*)dv,
-                                                                    (__nv_bfloat16*)dqkv, M, T, H);
-  else
-    return -2;
+  if (D != 128) return -2;
+  const long long threads = M * 3 * H * 8;
+  rope_qknorm_bwd128_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
+      (const __nv_bfloat16*)qkv, cosT, sinT, dqk, (const __nv_bfloat16*)dv, (__nv_bfloat16*)dqkv, M, T, H);
   return (int)cudaGetLastError();
 }
 
-// dqk: bf16 [M, 2*H*128]; writes the q and k thirds of dqkv [M, 3*H*128] (head_dim 128 only)
+// dqk: bf16 [M, 2*H*D]; writes the q and k thirds of dqkv [M, 3*H*D]
 int bones_rope_qknorm_bwd_bf16(const void* qkv, const float* cosT, const float* sinT, const void* dqk, void* dqkv, long long M, int T, int H,
-                               void* stream) {
-  const long long threads = M * H * 8;
-  rope_qknorm_bwd128_bf16_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
-      (const __nv_bfloat16*)qkv, cosT, sinT, (const __nv_bfloat16*)dqk, (__nv_bfloat16*)dqkv, M, T, H);
+                               int D, void* stream) {
+  const long long threads = M * H * (D / 16);
+  const unsigned grid = (unsigned)((threads + 255) / 256);
+  const auto *x = (const __nv_bfloat16*)qkv, *g = (const __nv_bfloat16*)dqk;
+  if (D == 128) rope_qknorm_bwd_bf16_kernel<128><<<grid, 256, 0, (cudaStream_t)stream>>>(x, cosT, sinT, g, (__nv_bfloat16*)dqkv, M, T, H);
+  else if (D == 64) rope_qknorm_bwd_bf16_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>(x, cosT, sinT, g, (__nv_bfloat16*)dqkv, M, T, H);
+  else return -2;
   return (int)cudaGetLastError();
 }
 
-// qk: [B*T, 2*H*128] (rotated, normalised q and k); qkv: [B*T, 3*H*128] (values read in place); y: [B*T, H*128]; lse: [B,H,T]
-int bones_attn_fwd(const void* qk, const void* qkv, void* y, float* lse, const int* doc_start, int B, int T, int H, float scale,
-                   int window_tiles, void* stream) {
-  if (T % AT) return -2;
+// qk: [B*T, 2*H*D] (rotated, normalised q and k); qkv: [B*T, 3*H*D] (values read in place); y: [B*T, H*D]; lse: [B,H,T];
+// counter: one int that is zero when the kernel starts
+int bones_attn_fwd(const void* qk, const void* qkv, void* y, float* lse, const int* doc_start, int* counter, int B, int T, int H, int D,
+                   float scale, int window_tiles, void* stream) {
+  if (D != 128 && D != 64) return -2;
+  if ((uintptr_t)y & 31) return -3;
   CUtensorMap tq, tv;
-  const long long M = (long long)B * T, A = (long long)H * AD;
-  int rc = tmap_rows_2d(&tq, qk, M, 2 * A);
+  const long long A = (long long)H * D;
+  int rc = tmap_rows_3d(&tq, qk, B, T, 2 * A);
   if (rc) return rc;
-  rc = tmap_rows_2d(&tv, qkv, M, 3 * A);
+  rc = tmap_rows_3d(&tv, qkv, B, T, 3 * A);
   if (rc) return rc;
   AttnParams p;
   p.B = B; p.T = T; p.H = H;
   p.c1 = scale * 1.4426950408889634f;
-  p.c2 = scale * AD * 1.4426950408889634f;
-  p.shift_ln = scale * AD;
+  p.c2 = scale * D * 1.4426950408889634f;
+  p.shift_ln = scale * D;
   p.window_tiles = window_tiles;
   p.doc_start = doc_start;
   p.y = (__nv_bfloat16*)y;
   p.lse = lse;
   p.err = error_word();
-  constexpr size_t smem = (size_t)TILE_BYTES * 7 + 256 + 2048 + FWD_SLACK;   // tiles, barriers, row-sum scratch, alignment slack
-  static bool attr_done = false;
-  if (!attr_done) {
-    BONES_CHECK(cudaFuncSetAttribute(attn_fwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done = true;
-  }
+  p.items = counter;
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
   BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  const long long items = (long long)(T / AT) * H * B;
-  const unsigned grid = (unsigned)(items < sms ? items : sms);       // persistent: one CTA per SM
-  static int* counter[64] = {};
-  if (dev < 0 || dev >= 64) return -2;
-  if (!counter[dev]) BONES_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&counter[dev]), g_fwd_items));
-  BONES_CHECK(cudaMemsetAsync(counter[dev], 0, sizeof(int), (cudaStream_t)stream));
-  p.items = counter[dev];
-  attn_fwd_kernel<<<grid, FWD_THREADS, smem, (cudaStream_t)stream>>>(tq, tv, p);
-  return (int)cudaGetLastError();
+  return D == 128 ? launch_attn_fwd<128>(tq, tv, p, sms, (cudaStream_t)stream) : launch_attn_fwd<64>(tq, tv, p, sms, (cudaStream_t)stream);
+}
+
+// The whole forward: RoPE + QK-norm (which zeroes the counter), then attention.
+int bones_attention_fwd(const void* qkv, const float* cosT, const float* sinT, void* qk, void* y, float* lse, const int* doc_start,
+                        int* counter, int B, int T, int H, int D, float scale, int window_tiles, void* stream) {
+  const int rc = bones_rope_qknorm_fwd(qkv, cosT, sinT, qk, counter, (long long)B * T, T, H, D, stream);
+  return rc ? rc : bones_attn_fwd(qk, qkv, y, lse, doc_start, counter, B, T, H, D, scale, window_tiles, stream);
 }
 }  // extern "C"

@@ -1,4 +1,4 @@
-// Flash attention backward as two tcgen05 kernels (head_dim 128), the default backward of attention.cu's forward.
+// Flash attention backward as two tcgen05 kernels (head_dim 128 or 64), the default backward of attention.cu's forward.
 //
 //   dkv kernel   one CTA per 128-key tile walks the query tiles that see it, in transposed form so that keys are the
 //                TMEM lanes:  S^T = Kh Qh^T,  dP^T = V dO^T,  P^T = exp2(S^T c1 - lse2) masked,  dV += P^T dO,
@@ -18,8 +18,7 @@
 namespace bones {
 
 constexpr int ST = 128;
-constexpr uint32_t STILE = ST * 128 * 2;   // 32 KB: two 128-byte-swizzled atoms of [128 rows][64 cols]
-constexpr uint32_t SATOM = STILE / 2;
+constexpr uint32_t SATOM = ST * 64 * 2;    // 16 KB: one 128-byte-swizzled atom of [128 rows][64 cols]; a tile has D / 64
 constexpr float kLog2e = 1.4426950408889634f;
 
 // Cycle accounting of the dK / dV kernel's roles, compiled in only with -DBONES_ATTN_PROF (a measuring build; the regular
@@ -45,10 +44,11 @@ __device__ long long* g_attn_prof = nullptr;
 
 struct SplitParams {
   int B, T, H;
+  int Tp;                // T rounded up to whole tiles: row length of the statistics
   float c1, scale;
   int window_tiles;
   const int* doc_start;
-  const float2* stats;   // [B, H, T]: (-lse * log2(e), delta)
+  const float2* stats;   // [B, H, Tp]: (-lse * log2(e), delta); (-inf, 0) past T, so that the queries there have P = 0
   __nv_bfloat16* dqk;    // [B*T, 2A]: dq-hat | dk-hat
   __nv_bfloat16* dv;     // rows of dv_ld elements
   long long dv_ld;
@@ -97,50 +97,70 @@ __device__ __forceinline__ void store_packed32(uint32_t taddr, const float* v) {
   BONES_TMEM_ST16(taddr, pk);
   tmem_st_wait();
 }
-// 32 accumulator columns of this thread's row -> 32 bf16 in global memory (two 32-byte sectors)
-__device__ __forceinline__ void drain_row32(uint32_t taddr, __nv_bfloat16* dst) {
-  uint32_t v[32];
+// C accumulator columns of this thread's row -> C bf16 in global memory (32-byte sectors); dst null: nothing is stored
+template <int C>
+__device__ __forceinline__ void drain_row(uint32_t taddr, __nv_bfloat16* dst) {
+  uint32_t v[C];
   __syncwarp();
-  BONES_TMEM_LD32(taddr, v);
+  if constexpr (C == 32) BONES_TMEM_LD32(taddr, v);
+  else BONES_TMEM_LD16(taddr, v);
   tmem_ld_wait();
-  uint4 u[4];
+  if (!dst) return;
+  uint4 u[C / 8];
 #pragma unroll
-  for (int g = 0; g < 4; ++g) {
+  for (int g = 0; g < C / 8; ++g) {
     u[g].x = pack_bf16(__uint_as_float(v[g * 8 + 0]), __uint_as_float(v[g * 8 + 1]));
     u[g].y = pack_bf16(__uint_as_float(v[g * 8 + 2]), __uint_as_float(v[g * 8 + 3]));
     u[g].z = pack_bf16(__uint_as_float(v[g * 8 + 4]), __uint_as_float(v[g * 8 + 5]));
     u[g].w = pack_bf16(__uint_as_float(v[g * 8 + 6]), __uint_as_float(v[g * 8 + 7]));
   }
-  st_global_v8(dst, u[0], u[1]);
-  st_global_v8(dst + 16, u[2], u[3]);
+#pragma unroll
+  for (int g = 0; g < C / 8; g += 2) st_global_v8(dst + g * 8, u[g], u[g + 1]);
 }
 
-// stats[b,h,t] = (-lse * log2(e), sum_d dO * O); sixteen lanes per (row, head), 16 bytes of each operand per lane.
-// Items run in the order of the output, [b, h, t] with t fastest: a group still reads 256 contiguous bytes of each
+// stats[b,h,t] = (-lse * log2(e), sum_d dO * O); D / 8 lanes per (head, two positions), 16 bytes of each operand and
+// position per lane (64 bytes of loads in flight: 36.6 -> 30.8 us at 32768 rows of 10 heads, where the copy rate gives 26).
+// Items run in the order of the output, [b, h, t] with t fastest: a group still reads 2 D contiguous bytes of each
 // operand, and the statistics and the log-sum-exp values of neighbouring groups are neighbours in memory (with the
-// head fastest they were T elements apart: one 32-byte sector per 8-byte result).
+// head fastest they were T elements apart: one 32-byte sector per 8-byte result).  Positions T .. Tp - 1 get (-inf, 0).
+// The first thread zeroes the work-item counters of the two kernels that follow on the stream.
+template <int D>
 __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ dy, const __nv_bfloat16* __restrict__ y,
-                                      const float* __restrict__ lse, float2* __restrict__ stats, long long M, int T, int H) {
-  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 4;
-  const int l16 = threadIdx.x & 15;
-  const long long total = M * H;
-  const long long it = item < total ? item : total - 1;      // every lane takes part in the shuffles
-  const long long bh = it / T;
-  const int t = (int)(it - bh * T);
+                                      const float* __restrict__ lse, float2* __restrict__ stats, int* counters, int B, int T, int Tp, int H) {
+  constexpr int LANES = D / 8;
+  if (blockIdx.x == 0 && threadIdx.x < 2) counters[threadIdx.x] = 0;
+  const long long item = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+  const int lane = threadIdx.x & (LANES - 1);
+  const long long total = (long long)B * H * Tp / 2;
+  const long long it = (item < total ? item : total - 1) * 2;      // every lane takes part in the shuffles; Tp is even
+  const long long bh = it / Tp;
+  const int tp = (int)(it - bh * Tp);
   const long long b = bh / H;
   const int h = (int)(bh - b * H);
-  const long long off = ((b * T + t) * H + h) * 128 + l16 * 8;
-  const uint4 a = *reinterpret_cast<const uint4*>(dy + off), c = *reinterpret_cast<const uint4*>(y + off);
-  const uint32_t aw[4] = {a.x, a.y, a.z, a.w}, cw[4] = {c.x, c.y, c.z, c.w};
-  float s = 0.f;
+  uint4 u[2], v[2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const float2 fa = unpack_bf16(aw[i]), fc = unpack_bf16(cw[i]);
-    s += fa.x * fc.x + fa.y * fc.y;
+  for (int j = 0; j < 2; ++j) {
+    const long long off = ((b * T + min(tp + j, T - 1)) * H + h) * D + lane * 8;
+    u[j] = *reinterpret_cast<const uint4*>(dy + off);
+    v[j] = *reinterpret_cast<const uint4*>(y + off);
   }
+  float s[2];
 #pragma unroll
-  for (int o = 8; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-  if (l16 == 0 && item < total) stats[it] = make_float2(-lse[it] * kLog2e, s);
+  for (int j = 0; j < 2; ++j) {
+    const uint32_t aw[4] = {u[j].x, u[j].y, u[j].z, u[j].w}, cw[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+    s[j] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 fa = unpack_bf16(aw[i]), fc = unpack_bf16(cw[i]);
+      s[j] += fa.x * fc.x + fa.y * fc.y;
+    }
+#pragma unroll
+    for (int o = LANES / 2; o > 0; o >>= 1) s[j] += __shfl_xor_sync(0xffffffffu, s[j], o);
+  }
+  if (lane < 2 && item < total) {
+    const int t = tp + lane;
+    stats[it + lane] = t < T ? make_float2(-lse[bh * T + t] * kLog2e, lane ? s[1] : s[0]) : make_float2(__int_as_float(0xff800000), 0.f);
+  }
 }
 
 // ---------------------------------------------------------------------------------------------------------------
@@ -152,11 +172,9 @@ __global__ void attn_bwd_stats_kernel(const __nv_bfloat16* __restrict__ dy, cons
 //          single-buffered and reloaded as soon as the item's last S^T and dP^T MMAs have been issued, so the next
 //          item's first tiles are computed while the compute warps drain dK and dV.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr uint32_t DKV_STAT = STILE * 7;            // two stages of 128 x (float2 stats), travelling with dO
-constexpr uint32_t DKV_BARS = DKV_STAT + 2 * 1024;
+// shared-memory offsets, by the tile's D / 64 atoms: seven tiles, two stages of 128 x (float2 stats) travelling with dO, barriers
+__host__ __device__ constexpr uint32_t dkv_bars(int D) { return (uint32_t)(D / 64) * SATOM * 7 + 2 * 1024; }
 constexpr uint32_t DKV_SLACK = 512;                 // room for aligning the tiles to 1024 bytes
-
-__device__ int g_dkv_items;      // item counter of the persistent dK/dV kernel (one launch at a time per device)
 
 struct DkvItem {
   int kt, h, b, n;
@@ -176,9 +194,12 @@ __device__ __forceinline__ DkvItem dkv_item(const SplitParams& p, int w, int n_t
   return it;
 }
 
+template <int D>
 __global__ void __launch_bounds__(STHREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_v,
                     const __grid_constant__ CUtensorMap tm_dy, const SplitParams p) {
+  constexpr uint32_t STILE = (D / 64) * SATOM;
+  constexpr int DT = D / 4;                            // accumulator columns a compute thread drains
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -190,19 +211,19 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
   const uint32_t sK = base, sV = base + STILE;
   auto sQ = [&](int s) { return base + STILE * (2 + s); };       // three stages
   auto sdO = [&](int s) { return base + STILE * (5 + s); };      // two stages
-  const uint32_t bars = base + DKV_BARS;
+  const uint32_t bars = base + dkv_bars(D);
   enum { B_KV = 0, B_KVFREE, B_Q0, B_Q1, B_Q2, B_QFREE0, B_QFREE1, B_QFREE2, B_DO0, B_DO1, B_DOFREE0, B_DOFREE1, B_SFULL, B_DPFULL,
          B_PREADY, B_DSREADY, B_DONE, B_ACCFREE, B_COUNT };
   auto bar = [&](int i) { return bars + 8u * i; };
   const uint32_t tmem_slot = bars + 8u * B_COUNT;
-  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + DKV_BARS + 8 * B_COUNT);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + DKV_BARS + 8 * B_COUNT + 8);
+  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + dkv_bars(D) + 8 * B_COUNT);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + dkv_bars(D) + 8 * B_COUNT + 8);
   const uint32_t ring_bars = bars + 176u;
-  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + DKV_BARS + 208);
+  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + dkv_bars(D) + 208);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int A = p.H * 128;
-  const int n_tiles = p.T / ST;
+  const int A = p.H * D;
+  const int n_tiles = p.Tp / ST;
   const int total = n_tiles * p.H * p.B;
 
   if (threadIdx.x == 0) {
@@ -254,37 +275,36 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
       if (w < 0) break;
       DkvItem im = dkv_item(p, w, n_tiles);
       im.n = warp_uniform(im.n);
-      const int row0 = im.b * p.T;
       APROF_ADD(1);
       if (it >= 1 && !dead) dead = !mbar_wait(bar(B_KVFREE), (uint32_t)((it - 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
       APROF_ADD(0);
       if (elect_one() && !dead) {
         mbar_arrive_expect_tx(bar(B_KV), 2 * STILE);
-        tma_load_2d(sK, &tm_qk, bar(B_KV), A + im.h * 128, row0 + im.kt * ST);
-        tma_load_2d(sK + SATOM, &tm_qk, bar(B_KV), A + im.h * 128 + 64, row0 + im.kt * ST);
-        tma_load_2d(sV, &tm_v, bar(B_KV), 2 * A + im.h * 128, row0 + im.kt * ST);
-        tma_load_2d(sV + SATOM, &tm_v, bar(B_KV), 2 * A + im.h * 128 + 64, row0 + im.kt * ST);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sK + c * SATOM, &tm_qk, bar(B_KV), A + im.h * D + c * 64, im.kt * ST, im.b);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sV + c * SATOM, &tm_v, bar(B_KV), 2 * A + im.h * D + c * 64, im.kt * ST, im.b);
       }
-      const float2* stat_row = p.stats + ((long long)im.b * p.H + im.h) * p.T;
+      const float2* stat_row = p.stats + ((long long)im.b * p.H + im.h) * p.Tp;
       for (int i = 0; i < im.n; ++i, ++g) {
         const int qs = g % 3, ds = g & 1;
-        const int r = row0 + (im.kt + i) * ST;
+        const int r = (im.kt + i) * ST;
         APROF_ADD(1);
         if (g >= 3 && !dead) dead = !mbar_wait(bar(B_QFREE0 + qs), (uint32_t)(((g - 3) / 3) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         APROF_ADD(0);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(bar(B_Q0 + qs), STILE);
-          tma_load_2d(sQ(qs), &tm_qk, bar(B_Q0 + qs), im.h * 128, r);
-          tma_load_2d(sQ(qs) + SATOM, &tm_qk, bar(B_Q0 + qs), im.h * 128 + 64, r);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qs) + c * SATOM, &tm_qk, bar(B_Q0 + qs), im.h * D + c * 64, r, im.b);
         }
         APROF_ADD(1);
         if (g >= 2 && !dead) dead = !mbar_wait(bar(B_DOFREE0 + ds), (uint32_t)(((g - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         APROF_ADD(0);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(bar(B_DO0 + ds), STILE + 1024);
-          tma_load_2d(sdO(ds), &tm_dy, bar(B_DO0 + ds), im.h * 128, r);
-          tma_load_2d(sdO(ds) + SATOM, &tm_dy, bar(B_DO0 + ds), im.h * 128 + 64, r);
-          bulk_load(base + DKV_STAT + ds * 1024, stat_row + (im.kt + i) * ST, 1024, bar(B_DO0 + ds));
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sdO(ds) + c * SATOM, &tm_dy, bar(B_DO0 + ds), im.h * D + c * 64, r, im.b);
+          bulk_load(base + STILE * 7 + ds * 1024, stat_row + (im.kt + i) * ST, 1024, bar(B_DO0 + ds));
         }
       }
     }
@@ -292,7 +312,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
     if (lane == 0) { APROF_STORE(20, 0); APROF_STORE(21, 1); }
   } else if (warp == 1) {
     const uint32_t id_kk = umma_idesc_f16(128, 128, 1, 0, 0);
-    const uint32_t id_km = umma_idesc_f16(128, 128, 1, 0, 1);
+    const uint32_t id_km = umma_idesc_f16(128, D, 1, 0, 1);
     bool dead = false;
     APROF_DECL(8);
     auto issue_s = [&](int t) {                           // S^T(t) = Kh Qh(t)^T
@@ -302,7 +322,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
       tc_fence_after();
       if (elect_one() && !dead) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(tS, sdesc_k(sK, k), sdesc_k(sQ(t % 3), k), id_kk, k ? 1u : 0u);
+        for (int k = 0; k < D / 16; ++k) umma_f16(tS, sdesc_k(sK, k), sdesc_k(sQ(t % 3), k), id_kk, k ? 1u : 0u);
         tc_commit(bar(B_SFULL));
       }
     };
@@ -313,7 +333,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
       tc_fence_after();
       if (elect_one() && !dead) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(tdP, sdesc_k(sV, k), sdesc_k(sdO(t & 1), k), id_kk, k ? 1u : 0u);
+        for (int k = 0; k < D / 16; ++k) umma_f16(tdP, sdesc_k(sV, k), sdesc_k(sdO(t & 1), k), id_kk, k ? 1u : 0u);
         tc_commit(bar(B_DPFULL));
         if (last) tc_commit(bar(B_KVFREE));
       }
@@ -383,8 +403,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
       const int w = ok ? item_take(ring_bars, ring_slots, it, abort_flag, p.err) : -1;
       if (w < 0) break;
       const DkvItem im = dkv_item(p, w, n_tiles);
-      const int k0 = im.kt * ST, kpos = k0 + r, row0 = im.b * p.T;
-      int nx_lo_last = p.doc_start ? p.doc_start[(long long)im.b * p.T + im.kt * ST + ST - 1] : 0;
+      const int k0 = im.kt * ST, kpos = k0 + r;
+      const long long row0 = (long long)im.b * p.T;
+      int nx_lo_last = p.doc_start ? p.doc_start[row0 + min(k0 + ST, p.T) - 1] : 0;
       for (int i = 0; i < im.n; ++i, ++g) {
         const int s = g & 1;
         const uint32_t ph = (uint32_t)(g & 1);
@@ -392,12 +413,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
         bool got = mbar_wait(bar(B_DO0 + s), (uint32_t)((g >> 1) & 1), abort_flag, p.err, ERR_WAIT_FULL);   // this tile's statistics
         APROF_ADD(0);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
-        const float4* st4 = reinterpret_cast<const float4*>(gen + DKV_STAT + s * 1024) + c0 / 2;   // two queries per float4
+        const float4* st4 = reinterpret_cast<const float4*>(gen + STILE * 7 + s * 1024) + c0 / 2;   // two queries per float4
         // document starts of this tile's queries (global, cached): only the tile that straddles a document start past
         // this key tile needs them element by element, and its last query decides that
-        const int* slo = p.doc_start ? p.doc_start + (long long)im.b * p.T + (im.kt + i) * ST : nullptr;
+        const int q0 = (im.kt + i) * ST;
+        const int* slo = p.doc_start ? p.doc_start + row0 + q0 : nullptr;
         const bool need_doc = slo && nx_lo_last > k0;
-        if (slo && i + 1 < im.n) nx_lo_last = slo[2 * ST - 1];
+        if (slo && i + 1 < im.n) nx_lo_last = slo[min(2 * ST, p.T - q0) - 1];
         float pr[32];
         got = mbar_wait(bar(B_SFULL), ph, abort_flag, p.err, ERR_WAIT_TMEM_FULL);
         APROF_ADD(1);
@@ -421,9 +443,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
             if (r > c0 + j) pr[j] = 0.f;
         }
         if (need_doc) {                                  // a query sees only keys of its own document
+          if (q0 + ST <= p.T) {
 #pragma unroll
-          for (int j = 0; j < 32; ++j)
-            if (kpos < slo[c0 + j]) pr[j] = 0.f;
+            for (int j = 0; j < 32; ++j)
+              if (kpos < slo[c0 + j]) pr[j] = 0.f;
+          } else {                                       // last tile of a ragged sequence: P is already 0 past its end
+#pragma unroll
+            for (int j = 0; j < 32; ++j)
+              if (q0 + c0 + j < p.T && kpos < slo[c0 + j]) pr[j] = 0.f;
+          }
         }
         store_packed32(tS + lane_addr + (uint32_t)c0, pr);
         tc_fence_before();
@@ -457,8 +485,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
       APROF_ADD(5);
       if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       tc_fence_after();
-      drain_row32(tdK + lane_addr + (uint32_t)c0, p.dqk + ((long long)(row0 + kpos)) * 2 * A + A + (long long)im.h * 128 + c0);
-      drain_row32(tdV + lane_addr + (uint32_t)c0, p.dv + ((long long)(row0 + kpos)) * p.dv_ld + (long long)im.h * 128 + c0);
+      const long long hcol = (long long)im.h * D + part * DT;
+      drain_row<DT>(tdK + lane_addr + (uint32_t)(part * DT), kpos < p.T ? p.dqk + (row0 + kpos) * 2 * A + A + hcol : nullptr);
+      drain_row<DT>(tdV + lane_addr + (uint32_t)(part * DT), kpos < p.T ? p.dv + (row0 + kpos) * p.dv_ld + hcol : nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(B_ACCFREE));
@@ -495,9 +524,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
 //      buffers run on across items; Q and dO are single-buffered and reloaded as soon as the item's last S and dP MMAs
 //      have been issued, so the next item's first tiles are computed while the compute warps drain dQ.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr uint32_t DQ_BARS = STILE * 7;
-
-__device__ int g_dq_items;       // item counter of the persistent dQ kernel (one launch at a time per device)
+__host__ __device__ constexpr uint32_t dq_bars(int D) { return (uint32_t)(D / 64) * SATOM * 7; }
 
 struct DqItem {
   int qt, h, b, kt0, n;
@@ -513,9 +540,12 @@ __device__ __forceinline__ DqItem dq_item(const SplitParams& p, int w, int n_til
   return it;
 }
 
+template <int D>
 __global__ void __launch_bounds__(STHREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_v,
                    const __grid_constant__ CUtensorMap tm_dy, const SplitParams p) {
+  constexpr uint32_t STILE = (D / 64) * SATOM;
+  constexpr int DT = D / 4;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -523,19 +553,19 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
   const uint32_t sQ = base, sdO = base + STILE;
   auto sK = [&](int s) { return base + STILE * (2 + s); };      // three stages
   auto sV = [&](int s) { return base + STILE * (5 + s); };      // two stages
-  const uint32_t bars = base + DQ_BARS;
+  const uint32_t bars = base + dq_bars(D);
   enum { B_QDO = 0, B_QDOFREE, B_K0, B_K1, B_K2, B_KFREE0, B_KFREE1, B_KFREE2, B_V0, B_V1, B_VFREE0, B_VFREE1, B_SFULL, B_SFREE,
          B_DPFULL0, B_DPFULL1, B_DSREADY0, B_DSREADY1, B_DONE, B_DQFREE, B_COUNT };
   auto bar = [&](int i) { return bars + 8u * i; };
   const uint32_t tmem_slot = bars + 8u * B_COUNT;
-  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + DQ_BARS + 8 * B_COUNT);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + DQ_BARS + 8 * B_COUNT + 8);
+  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + dq_bars(D) + 8 * B_COUNT);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + dq_bars(D) + 8 * B_COUNT + 8);
   const uint32_t ring_bars = bars + 176u;
-  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + DQ_BARS + 208);
+  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + dq_bars(D) + 208);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int A = p.H * 128;
-  const int n_tiles = p.T / ST;
+  const int A = p.H * D;
+  const int n_tiles = p.Tp / ST;
   const int total = n_tiles * p.H * p.B;
 
   if (threadIdx.x == 0) {
@@ -587,35 +617,34 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
       DqItem im = dq_item(p, w, n_tiles);
       im.kt0 = warp_uniform(im.kt0);
       im.n = im.qt - im.kt0 + 1;
-      const int row0 = im.b * p.T, rq = row0 + im.qt * ST;
       if (it >= 1 && !dead) dead = !mbar_wait(bar(B_QDOFREE), (uint32_t)((it - 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
       if (elect_one() && !dead) {
         mbar_arrive_expect_tx(bar(B_QDO), 2 * STILE);
-        tma_load_2d(sQ, &tm_qk, bar(B_QDO), im.h * 128, rq);
-        tma_load_2d(sQ + SATOM, &tm_qk, bar(B_QDO), im.h * 128 + 64, rq);
-        tma_load_2d(sdO, &tm_dy, bar(B_QDO), im.h * 128, rq);
-        tma_load_2d(sdO + SATOM, &tm_dy, bar(B_QDO), im.h * 128 + 64, rq);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ + c * SATOM, &tm_qk, bar(B_QDO), im.h * D + c * 64, im.qt * ST, im.b);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sdO + c * SATOM, &tm_dy, bar(B_QDO), im.h * D + c * 64, im.qt * ST, im.b);
       }
       for (int j = 0; j < im.n; ++j, ++g) {
         const int ks = g % 3, vs = g & 1;
-        const int r = row0 + (im.kt0 + j) * ST;
+        const int r = (im.kt0 + j) * ST;
         if (g >= 3 && !dead) dead = !mbar_wait(bar(B_KFREE0 + ks), (uint32_t)(((g - 3) / 3) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(bar(B_K0 + ks), STILE);
-          tma_load_2d(sK(ks), &tm_qk, bar(B_K0 + ks), A + im.h * 128, r);
-          tma_load_2d(sK(ks) + SATOM, &tm_qk, bar(B_K0 + ks), A + im.h * 128 + 64, r);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sK(ks) + c * SATOM, &tm_qk, bar(B_K0 + ks), A + im.h * D + c * 64, r, im.b);
         }
         if (g >= 2 && !dead) dead = !mbar_wait(bar(B_VFREE0 + vs), (uint32_t)(((g - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(bar(B_V0 + vs), STILE);
-          tma_load_2d(sV(vs), &tm_v, bar(B_V0 + vs), 2 * A + im.h * 128, r);
-          tma_load_2d(sV(vs) + SATOM, &tm_v, bar(B_V0 + vs), 2 * A + im.h * 128 + 64, r);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sV(vs) + c * SATOM, &tm_v, bar(B_V0 + vs), 2 * A + im.h * D + c * 64, r, im.b);
         }
       }
     }
   } else if (warp == 1) {
     const uint32_t id_kk = umma_idesc_f16(128, 128, 1, 0, 0);
-    const uint32_t id_km = umma_idesc_f16(128, 128, 1, 0, 1);
+    const uint32_t id_km = umma_idesc_f16(128, D, 1, 0, 1);
     bool dead = false;
     // S(t) and dP(t) of running tile t; `last`: t is the last tile of its item, after which Q and dO may be reloaded
     auto issue_sdp = [&](int t, bool last) {
@@ -624,7 +653,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
       tc_fence_after();
       if (elect_one() && !dead) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(tS, sdesc_k(sQ, k), sdesc_k(sK(t % 3), k), id_kk, k ? 1u : 0u);
+        for (int k = 0; k < D / 16; ++k) umma_f16(tS, sdesc_k(sQ, k), sdesc_k(sK(t % 3), k), id_kk, k ? 1u : 0u);
         tc_commit(bar(B_SFULL));
       }
       if (!dead) dead = !mbar_wait(bar(B_V0 + (t & 1)), (uint32_t)((t >> 1) & 1), abort_flag, p.err, ERR_WAIT_FULL);
@@ -632,7 +661,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
       // dP(t) goes into the buffer whose packed dS(t-2) the dQ MMAs of tile t-2 (issued earlier, same pipe) have read
       if (elect_one() && !dead) {
 #pragma unroll
-        for (int k = 0; k < 8; ++k) umma_f16(tdP(t & 1), sdesc_k(sdO, k), sdesc_k(sV(t & 1), k), id_kk, k ? 1u : 0u);
+        for (int k = 0; k < D / 16; ++k) umma_f16(tdP(t & 1), sdesc_k(sdO, k), sdesc_k(sV(t & 1), k), id_kk, k ? 1u : 0u);
         tc_commit(bar(B_DPFULL0 + (t & 1)));
         tc_commit(bar(B_VFREE0 + (t & 1)));
         if (last) tc_commit(bar(B_QDOFREE));
@@ -675,10 +704,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
       const int w = ok ? item_take(ring_bars, ring_slots, it, abort_flag, p.err) : -1;
       if (w < 0) break;
       const DqItem im = dq_item(p, w, n_tiles);
-      const int qpos = im.qt * ST + r, row0 = im.b * p.T;
-      const float2 st = p.stats[((long long)im.b * p.H + im.h) * p.T + qpos];
+      const int qpos = im.qt * ST + r;
+      const long long row0 = (long long)im.b * p.T;
+      const float2 st = p.stats[((long long)im.b * p.H + im.h) * p.Tp + qpos];
       int lo = 0;
-      if (p.doc_start) lo = p.doc_start[(long long)im.b * p.T + qpos];
+      if (p.doc_start && qpos < p.T) lo = p.doc_start[row0 + qpos];
       for (int j = 0; j < im.n; ++j, ++g) {
         const int s = g & 1;
         bool got = mbar_wait(bar(B_SFULL), (uint32_t)(g & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
@@ -725,7 +755,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
       const bool got = mbar_wait(bar(B_DONE), (uint32_t)(it & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
       if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
       tc_fence_after();
-      drain_row32(tdQ + lane_addr + (uint32_t)c0, p.dqk + ((long long)(row0 + qpos)) * 2 * A + (long long)im.h * 128 + c0);
+      drain_row<DT>(tdQ + lane_addr + (uint32_t)(part * DT),
+                    qpos < p.T ? p.dqk + (row0 + qpos) * 2 * A + (long long)im.h * D + part * DT : nullptr);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(bar(B_DQFREE));
@@ -743,11 +774,32 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
   }
 }
 
-static int tmap_rows_2d_s(CUtensorMap* out, const void* ptr, long long rows, long long cols) {
-  uint64_t dims[2] = {(uint64_t)cols, (uint64_t)rows};
-  uint64_t strides[1] = {(uint64_t)cols * 2};
-  uint32_t box[2] = {64, 128};
-  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+// [B, T, cols] bf16 rows, boxes of 64 columns x 128 rows of one sequence; rows past T read as zeros
+static int tmap_rows_3d_s(CUtensorMap* out, const void* ptr, int B, int T, long long cols) {
+  uint64_t dims[3] = {(uint64_t)cols, (uint64_t)T, (uint64_t)B};
+  uint64_t strides[2] = {(uint64_t)cols * 2, (uint64_t)cols * 2 * (uint64_t)T};
+  uint32_t box[3] = {64, 128, 1};
+  return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+template <int D>
+static int launch_split(const CUtensorMap& tq, const CUtensorMap& tv, const CUtensorMap& td, SplitParams p, int* counters, int sms, cudaStream_t s) {
+  constexpr size_t smem_dkv = (size_t)dkv_bars(D) + 256 + DKV_SLACK;
+  constexpr size_t smem_dq = (size_t)dq_bars(D) + 256 + 1024;
+  static bool attr_done = false;
+  if (!attr_done) {
+    BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dkv));
+    BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq));
+    attr_done = true;
+  }
+  const long long items = (long long)(p.Tp / ST) * p.H * p.B;
+  const unsigned grid = (unsigned)(items < sms ? items : sms);          // persistent: one CTA per SM in both kernels
+  p.items = counters;
+  attn_bwd_dkv_kernel<D><<<grid, STHREADS, smem_dkv, s>>>(tq, tv, td, p);
+  BONES_CHECK(cudaGetLastError());
+  p.items = counters + 1;
+  attn_bwd_dq_kernel<D><<<grid, STHREADS, smem_dq, s>>>(tq, tv, td, p);
+  return (int)cudaGetLastError();
 }
 
 }  // namespace bones
@@ -755,32 +807,40 @@ static int tmap_rows_2d_s(CUtensorMap* out, const void* ptr, long long rows, lon
 extern "C" {
 using namespace bones;
 
-// stats: [B, H, T] float2 scratch filled by the pre-pass
-int bones_attn_bwd_stats(const void* dy, const void* y, const float* lse, void* stats, long long M, int T, int H, void* stream) {
-  const long long threads = M * H * 16;
-  attn_bwd_stats_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, (const __nv_bfloat16*)y,
-                                                                                       lse, (float2*)stats, M, T, H);
+int bones_rope_qknorm_bwd_bf16(const void* qkv, const float* cosT, const float* sinT, const void* dqk, void* dqkv, long long M, int T, int H,
+                               int D, void* stream);
+
+// stats: [B, H, Tp] float2 scratch (Tp: T rounded up to a multiple of 128); counters: two ints, zeroed here
+int bones_attn_bwd_stats(const void* dy, const void* y, const float* lse, void* stats, int* counters, int B, int T, int H, int D, void* stream) {
+  const int Tp = (T + ST - 1) / ST * ST;
+  const long long threads = (long long)B * H * Tp / 2 * (D / 8);
+  const unsigned grid = (unsigned)((threads + 255) / 256);
+  const auto *g = (const __nv_bfloat16*)dy, *o = (const __nv_bfloat16*)y;
+  if (D == 128) attn_bwd_stats_kernel<128><<<grid, 256, 0, (cudaStream_t)stream>>>(g, o, lse, (float2*)stats, counters, B, T, Tp, H);
+  else if (D == 64) attn_bwd_stats_kernel<64><<<grid, 256, 0, (cudaStream_t)stream>>>(g, o, lse, (float2*)stats, counters, B, T, Tp, H);
+  else return -2;
   return (int)cudaGetLastError();
 }
 
-// qk: [B*T, 2A] rotated, normalised q | k;  qkv: [B*T, 3A] (values read in place);  dy: [B*T, A];  stats from the pre-pass.
-// Outputs (bf16, every element overwritten): dqk [B*T, 2A];  dv rows of dv_ld elements (e.g. the last third of dqkv).
-int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const void* stats, void* dqk, void* dv, long long dv_ld,
-                         const int* doc_start, int B, int T, int H, float scale, int window_tiles, void* stream) {
-  if (T % ST) return -2;
+// qk: [B*T, 2A] rotated, normalised q | k;  qkv: [B*T, 3A] (values read in place);  dy: [B*T, A];  stats and counters from the
+// pre-pass.  Outputs (bf16, every element overwritten): dqk [B*T, 2A];  dv rows of dv_ld elements (e.g. the last third of dqkv).
+int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const void* stats, int* counters, void* dqk, void* dv,
+                         long long dv_ld, const int* doc_start, int B, int T, int H, int D, float scale, int window_tiles, void* stream) {
+  if (D != 128 && D != 64) return -2;
   if ((dv_ld % 16) || ((uintptr_t)dv & 31) || ((uintptr_t)dqk & 31) || ((uintptr_t)stats & 15) ||
       (doc_start && ((uintptr_t)doc_start & 15)))
     return -3;
-  const long long M = (long long)B * T, A = (long long)H * 128;
+  const long long A = (long long)H * D;
   CUtensorMap tq, tv, td;
-  int rc = tmap_rows_2d_s(&tq, qk, M, 2 * A);
+  int rc = tmap_rows_3d_s(&tq, qk, B, T, 2 * A);
   if (rc) return rc;
-  rc = tmap_rows_2d_s(&tv, qkv, M, 3 * A);
+  rc = tmap_rows_3d_s(&tv, qkv, B, T, 3 * A);
   if (rc) return rc;
-  rc = tmap_rows_2d_s(&td, dy, M, A);
+  rc = tmap_rows_3d_s(&td, dy, B, T, A);
   if (rc) return rc;
   SplitParams p;
   p.B = B; p.T = T; p.H = H;
+  p.Tp = (T + ST - 1) / ST * ST;
   p.c1 = scale * kLog2e;
   p.scale = scale;
   p.window_tiles = window_tiles;
@@ -790,33 +850,23 @@ int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const 
   p.dv = (__nv_bfloat16*)dv;
   p.dv_ld = dv_ld;
   p.err = error_word();
-  constexpr size_t smem_dkv = (size_t)DKV_BARS + 256 + DKV_SLACK;
-  constexpr size_t smem_dq = (size_t)DQ_BARS + 256 + 1024;
-  static bool attr_done = false;
-  if (!attr_done) {
-    BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dkv));
-    BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dq_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq));
-    attr_done = true;
-  }
-  cudaStream_t s = (cudaStream_t)stream;
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
   BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  if (dev < 0 || dev >= 64) return -2;
-  const long long items = (long long)(T / ST) * H * B;
-  const unsigned grid = (unsigned)(items < sms ? items : sms);          // persistent: one CTA per SM in both kernels
-  static int* counter_dkv[64] = {};
-  static int* counter_dq[64] = {};
-  if (!counter_dkv[dev]) BONES_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&counter_dkv[dev]), g_dkv_items));
-  if (!counter_dq[dev]) BONES_CHECK(cudaGetSymbolAddress(reinterpret_cast<void**>(&counter_dq[dev]), g_dq_items));
-  BONES_CHECK(cudaMemsetAsync(counter_dkv[dev], 0, sizeof(int), s));
-  BONES_CHECK(cudaMemsetAsync(counter_dq[dev], 0, sizeof(int), s));
-  p.items = counter_dkv[dev];
-  attn_bwd_dkv_kernel<<<grid, STHREADS, smem_dkv, s>>>(tq, tv, td, p);
-  BONES_CHECK(cudaGetLastError());
-  p.items = counter_dq[dev];
-  attn_bwd_dq_kernel<<<grid, STHREADS, smem_dq, s>>>(tq, tv, td, p);
-  return (int)cudaGetLastError();
+  return D == 128 ? launch_split<128>(tq, tv, td, p, counters, sms, (cudaStream_t)stream)
+                  : launch_split<64>(tq, tv, td, p, counters, sms, (cudaStream_t)stream);
+}
+
+// The whole backward: statistics (which zeroes the counters), dK / dV and dQ, RoPE / QK-norm backward into dqkv [B*T, 3A].
+int bones_attention_bwd(const void* dy, const void* qkv, const void* qk, const void* y, const float* lse, const float* cosT, const float* sinT,
+                        const int* doc_start, void* stats, int* counters, void* dqk, void* dqkv, int B, int T, int H, int D, float scale,
+                        int window_tiles, void* stream) {
+  const long long A = (long long)H * D;
+  int rc = bones_attn_bwd_stats(dy, y, lse, stats, counters, B, T, H, D, stream);
+  if (rc) return rc;
+  rc = bones_attn_bwd_split(qk, qkv, dy, stats, counters, dqk, (__nv_bfloat16*)dqkv + 2 * A, 3 * A, doc_start, B, T, H, D, scale, window_tiles, stream);
+  if (rc) return rc;
+  return bones_rope_qknorm_bwd_bf16(qkv, cosT, sinT, dqk, dqkv, (long long)B * T, T, H, D, stream);
 }
 
 #ifdef BONES_ATTN_PROF

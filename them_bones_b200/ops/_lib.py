@@ -51,11 +51,11 @@ def stream():
 _I, _L, _F = ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 
 
-LAUNCHES = [0]        # native kernel launches issued by this process (each entry point launches one kernel)
+LAUNCHES = [0]        # native kernel launches issued by this process (`launches`: an entry point with more than one kernel)
 
 
-def call(name: str, *args):
-    LAUNCHES[0] += 1
+def call(name: str, *args, launches: int = 1):
+    LAUNCHES[0] += launches
     rc = getattr(load(), name)(*args)
     if rc != 0:
         raise RuntimeError(f"{name} failed with code {rc}")

@@ -14,20 +14,27 @@ _I, _L, _F = ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 _IMPL = os.environ.get("BONES_ATTN_BWD", "split")
 
 
+def length_multiple(head_dim: int) -> int:
+    """The sequence length has to be a multiple of this: the split kernels take any length, the fused one whole tiles."""
+    return 128 if _IMPL == "fused" and head_dim == 128 else 1
+
+
 def backward(dy, qkv2, qk, y, lse, cos, sin, ds, b, t, n_head, head_dim, scale, window):
     m, a = b * t, n_head * head_dim
     dev = dy.device
     dy2 = (dy if dy.is_contiguous() else dy.contiguous()).view(m, a)
     dqkv = torch.empty(m, 3 * a, dtype=torch.bfloat16, device=dev)
-    if _IMPL != "fused" and head_dim == 128:
-        stats = torch.empty(b, n_head, t, 2, dtype=torch.float32, device=dev)
-        L.call("bones_attn_bwd_stats", L.ptr(dy2), L.ptr(y), L.ptr(lse), L.ptr(stats), _L(m), _I(t), _I(n_head), L.stream())
+    if _IMPL != "fused" or head_dim != 128:
+        if t % 128 and dy2.data_ptr() % 16:
+            dy2 = dy2.clone()
+        # statistics of whole 128-query tiles, and behind them the two kernels' work-item counters
+        n = b * n_head * (-(-t // 128) * 128) * 2
+        stats = torch.empty(n + 2, dtype=torch.float32, device=dev)
         dqk = torch.empty(m, 2 * a, dtype=torch.bfloat16, device=dev)
-        dv = dqkv[:, 2 * a:]                                   # the kernel writes dV in place, rows 3a apart
-        L.call("bones_attn_bwd_split", L.ptr(qk), L.ptr(qkv2), L.ptr(dy2), L.ptr(stats), L.ptr(dqk), L.ptr(dv), _L(3 * a), L.ptr(ds),
-               _I(b), _I(t), _I(n_head), _F(scale), _I(window // 128), L.stream())
-        L.call("bones_rope_qknorm_bwd_bf16", L.ptr(qkv2), L.ptr(cos), L.ptr(sin), L.ptr(dqk), L.ptr(dqkv), _L(m), _I(t), _I(n_head),
-               L.stream())
+        # dV goes straight into its third of dqkv, rows 3a apart
+        L.call("bones_attention_bwd", L.ptr(dy2), L.ptr(qkv2), L.ptr(qk), L.ptr(y), L.ptr(lse), L.ptr(cos), L.ptr(sin), L.ptr(ds), L.ptr(stats),
+               ctypes.c_void_p(stats.data_ptr() + 4 * n), L.ptr(dqk), L.ptr(dqkv), _I(b), _I(t), _I(n_head), _I(head_dim), _F(scale),
+               _I(window // 128), L.stream(), launches=4)
         return dqkv
     delta = torch.empty(b, n_head, t, dtype=torch.float32, device=dev)
     L.call("bones_attn_delta", L.ptr(dy2), L.ptr(y), L.ptr(delta), _L(m), _I(t), _I(n_head), L.stream())

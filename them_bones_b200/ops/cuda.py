@@ -355,12 +355,14 @@ def attention(qkv, cos, sin, n_head, head_dim, scale, doc_start, window):
     (``csrc/attention.cu``, ``csrc/attention_bwd_split.cu``).  A shape the kernels do not cover raises: the SDPA route
     exists only as the explicit baseline (``BONES_KERNELS=ref``), never as a silent fallback (reference: a kernel
     route that does not apply on the device raises, round2/source/train.py:4882-4887)."""
+    from . import attention_bwd as AB
     from . import attention_native as AN
     t = qkv.shape[1]
-    pad = -t % 128
+    pad = -t % AB.length_multiple(head_dim)
     if pad:
-        # the kernels work on 128-token tiles: a ragged length (scoring, cache-free decoding) is zero-padded at the end,
-        # which causal masking keeps away from the real positions, and the padding rows are dropped again
+        # the single-kernel backward (`BONES_ATTN_BWD=fused`) works on whole 128-token tiles: the sequence is zero-padded at
+        # the end, which causal masking keeps away from the real positions, and the padding rows are dropped again.  The
+        # default kernels take any length (rows past the end are zeros of the tensor maps, and are not stored).
         qkv = F.pad(qkv, (0, 0, 0, pad))
         cos, sin = F.pad(cos, (0, 0, 0, pad)), F.pad(sin, (0, 0, 0, pad))
         if doc_start is not None:

@@ -117,13 +117,18 @@ def roles(a):
         qk = AN.rope_qknorm(qkv, cos, sin, t, h, d)
         y, lse = AN.attn_forward(qk, qkv, None, b, t, h, scale, 0)
         dy = torch.randn(m, ad, device="cuda", dtype=bf)
-        stats = torch.empty(b, h, t, 2, dtype=torch.float32, device="cuda")
+        stats = torch.empty(b, h, -(-t // 128) * 128, 2, dtype=torch.float32, device="cuda")
+        counters = torch.zeros(2, dtype=torch.int32, device="cuda")
         dqk = torch.empty(m, 2 * ad, dtype=bf, device="cuda")
         dqkv = torch.empty(m, 3 * ad, dtype=bf, device="cuda")
         dv = dqkv[:, 2 * ad:]
-        L.call("bones_attn_bwd_stats", L.ptr(dy), L.ptr(y), L.ptr(lse), L.ptr(stats), LL(m), I(t), I(h), L.stream())
-        fn = lambda: L.call("bones_attn_bwd_split", L.ptr(qk), L.ptr(qkv), L.ptr(dy), L.ptr(stats), L.ptr(dqk), L.ptr(dv), LL(3 * ad),  # noqa: E731
-                            L.ptr(None), I(b), I(t), I(h), F(scale), I(0), L.stream())
+        L.call("bones_attn_bwd_stats", L.ptr(dy), L.ptr(y), L.ptr(lse), L.ptr(stats), L.ptr(counters), I(b), I(t), I(h), I(d), L.stream())
+
+        def fn():
+            counters.zero_()
+            L.call("bones_attn_bwd_split", L.ptr(qk), L.ptr(qkv), L.ptr(dy), L.ptr(stats), L.ptr(counters), L.ptr(dqk), L.ptr(dv), LL(3 * ad),
+                   L.ptr(None), I(b), I(t), I(h), I(d), F(scale), I(0), L.stream())
+
         ms = timeit(fn, a.iters, a.warmup, not a.no_flush)
         lib.bones_attn_set_prof(ctypes.c_void_p(prof.data_ptr()))
         fn()
