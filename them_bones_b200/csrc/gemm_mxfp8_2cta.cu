@@ -841,7 +841,8 @@ __device__ __forceinline__ size_t q_sf_base32(uint32_t r0, uint32_t kb, uint32_t
 template <bool kRow, bool kCol, int kHalves, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32, 1)
 mx_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t* __restrict__ qr, uint8_t* __restrict__ sfr, int group_r,
-                     uint8_t* __restrict__ qc, uint8_t* __restrict__ sfc, int group_c, long long R, long long C, uint32_t n_tiles, int* err) {
+                     uint8_t* __restrict__ qc, uint8_t* __restrict__ sfc, int group_c, long long R, long long C, uint32_t rows_per,
+                     size_t sfr_per, size_t sfc_per, uint32_t n_tiles, int* err) {
   using G = QdGeom<kHalves, kWarps>;
   constexpr int kCols = 64 * kHalves, kPitch = 2 * kCols;        // columns of a tile; bytes of a tile row in shared memory
   extern __shared__ __align__(128) uint8_t qd_smem[];
@@ -858,7 +859,7 @@ mx_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
   __syncthreads();
   const uint32_t tiles_c = (uint32_t)(C / kCols);
   const uint32_t stride = gridDim.x * kWarps;
-  const uint32_t kb_c = (uint32_t)((C + 127) >> 7), kb_r = (uint32_t)((R + 127) >> 7);
+  const uint32_t kb_c = (uint32_t)((C + 127) >> 7), kb_r = (rows_per + 127u) >> 7;
   // the rows of tile `tile` into stage s: every lane copies one row
   auto issue = [&](uint32_t tile, int s) {
     const uint32_t tr = tile / tiles_c, tc = tile - tr * tiles_c;
@@ -882,6 +883,8 @@ mx_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
     const uint32_t tr = tile / tiles_c, tc = tile - tr * tiles_c;
     const long long row0 = (long long)tr * 32;
     const int rows_here = (int)min((long long)32, R - row0);
+    // its matrix of the batch, and its first row in that matrix
+    const uint32_t bm = (uint32_t)row0 / rows_per, lrow0 = (uint32_t)row0 - bm * rows_per;
     // the tile's place in its 128-column K block of the row copy: first chunk and K block
     const uint32_t kblock = kHalves == 2 ? tc : (tc >> 1);
     const int chunk0 = kHalves == 2 ? 0 : (int)(tc & 1u) * 2;
@@ -939,8 +942,8 @@ mx_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
         const uint32_t inv_lo = q_scale_bf16(pair & 0xffffu, b_lo), inv_hi = q_scale_bf16(pair >> 16, b_hi);
         const uint32_t my_inv2 = (inv_lo & 0xffffu) | (inv_hi & 0xffff0000u);
         // the transposed operand's "rows" are the columns; its K block is the 128-row block of row0
-        uint8_t* sp = sfc + q_sf_base32(tc * (uint32_t)kCols + (uint32_t)c * 32u, (uint32_t)(row0 >> 7), kb_r, group_c) +
-                      (size_t)(((piece & 3) * 8 + 2 * rsub) * 16 + (int)((row0 & 127) >> 5));
+        uint8_t* sp = sfc + bm * sfc_per + q_sf_base32(tc * (uint32_t)kCols + (uint32_t)c * 32u, lrow0 >> 7, kb_r, group_c) +
+                      (size_t)(((piece & 3) * 8 + 2 * rsub) * 16 + (int)((lrow0 & 127u) >> 5));
         sp[0] = (uint8_t)b_lo;
         sp[16] = (uint8_t)b_hi;
         uint32_t inv2[4];
@@ -957,7 +960,7 @@ mx_quant_dual_kernel(const __nv_bfloat16* __restrict__ x, long long ldx, uint8_t
     if (kRow) {
       // pieces 0 and 4 of a row hold the scale bytes of the tile's even and odd chunks; a whole K block's four bytes
       // leave as one 32-bit store, half a block's two as one 16-bit store
-      uint8_t* rp = sfr + q_sf_base32((uint32_t)row0, kblock, kb_c, group_r) + (size_t)(rsub * 16 + chunk0);
+      uint8_t* rp = sfr + bm * sfr_per + q_sf_base32(lrow0, kblock, kb_c, group_r) + (size_t)(rsub * 16 + chunk0);
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
         const uint32_t v = rowsf[i] | __shfl_xor_sync(0xffffffffu, rowsf[i], 4);
@@ -1028,8 +1031,16 @@ long long bones_mx2_sf_bytes(long long rows, long long K, int group) {
 // x bf16 [R, C] -> optional row-quantised copy (qr, sfr: blocks along C, scale tiles of `group_r` rows) and optional
 // column-quantised copy (qc, sfc: blocks along R; its scale chunks describe an operand with rows = C, K = R, tiles of
 // `group_c` rows).  C a multiple of 128; a last, partial block of rows is quantised as a block of its own.
+// batch > 1: x is a stack of `batch` such matrices of R rows (a multiple of 32: a 32-row tile lies in one matrix), outputs
+// stacked likewise.  One launch for the 16 experts of an MoE layer instead of one per expert and direction: 49 us for both
+// copies of 40960 x 1280 where 1 + 16 launches took 149 us.
 int bones_mx2_quant(const void* x, long long ldx, void* qr, void* sfr, int group_r, void* qc, void* sfc, int group_c, long long R, long long C,
-                    void* stream) {
+                    int batch, void* stream) {
+  if (batch < 1 || (batch > 1 && (R % 32))) return -2;
+  const long long rows_per = R;
+  const size_t sfr_per = (size_t)bones_mx2_sf_bytes(rows_per, C, group_r > 0 ? group_r : 128);
+  const size_t sfc_per = (size_t)bones_mx2_sf_bytes(C, rows_per, group_c > 0 ? group_c : 128);
+  R *= batch;
   if ((C % 128) || (ldx % 8) || ((uintptr_t)x & 15)) return -2;
   if ((qr && ((group_r % 32) || ((uintptr_t)sfr & 3))) || (qc && (group_c % 32)) || R >= (1LL << 31) || C >= (1LL << 31)) return -2;
   if (R == 0 || (!qr && !qc)) return 0;
@@ -1053,7 +1064,8 @@ int bones_mx2_quant(const void* x, long long ldx, void* qr, void* sfr, int group
   }
 #define BONES_QUANT_LAUNCH(ROW, COL)                                                                                          \
   mx_quant_dual_kernel<ROW, COL, kHalves, kWarps><<<grid, kWarps * 32, G::kSmemBytes, (cudaStream_t)stream>>>(                 \
-      (const __nv_bfloat16*)x, ldx, (uint8_t*)qr, (uint8_t*)sfr, group_r, (uint8_t*)qc, (uint8_t*)sfc, group_c, R, C, (uint32_t)tiles, err)
+      (const __nv_bfloat16*)x, ldx, (uint8_t*)qr, (uint8_t*)sfr, group_r, (uint8_t*)qc, (uint8_t*)sfc, group_c, R, C, (uint32_t)rows_per, \
+      sfr_per, sfc_per, (uint32_t)tiles, err)
   if (qr && qc) BONES_QUANT_LAUNCH(true, true);
   else if (qr) BONES_QUANT_LAUNCH(true, false);
   else if (qc) BONES_QUANT_LAUNCH(false, true);

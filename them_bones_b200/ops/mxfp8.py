@@ -61,25 +61,24 @@ def _sf_buf(rows: int, k: int, group: int, dev, lead=()):
     return mk(*lead, sf2_bytes(rows, k, group), dtype=torch.uint8, device=dev)
 
 
-def quant2(x2: torch.Tensor, *, row: bool = True, col: bool = False, group_r: int = 128, group_c: int = 128, out=None):
+def quant2(x2: torch.Tensor, *, row: bool = True, col: bool = False, group_r: int = 128, group_c: int = 128):
     """bf16 ``[R, C]`` -> ``(q_row, sf_row, q_col, sf_col)``: E4M3 copies quantised in 1 x 32 blocks along C (``row``) and
     along R (``col``), each with UE8M0 scale chunks laid out for an operand whose tiles are ``group`` rows.  The column
     copy's chunks describe the transposed operand (rows = C, contraction = R) that a weight-gradient GEMM reads.
-    ``out``: the same four tensors preallocated (slices of a batch)."""
-    r, c = x2.shape
+    ``x2`` may be a contiguous stack ``[E, R, C]`` (R a multiple of 32), quantised matrix by matrix in the same launch; the four
+    results then carry the leading axis."""
+    lead = tuple(x2.shape[:-2])
+    r, c = x2.shape[-2:]
     dev = x2.device
     qr = sfr = qc = sfc = None
-    if out is not None:
-        qr, sfr, qc, sfc = out
-    else:
-        if row:
-            qr = torch.empty(r, c, dtype=torch.uint8, device=dev)
-            sfr = _sf_buf(r, c, group_r, dev)
-        if col:
-            qc = torch.empty(r, c, dtype=torch.uint8, device=dev)
-            sfc = _sf_buf(c, r, group_c, dev)
-    L.call("bones_mx2_quant", L.ptr(x2), _L(x2.stride(0)), L.ptr(qr), L.ptr(sfr), _I(group_r), L.ptr(qc), L.ptr(sfc), _I(group_c),
-           _L(r), _L(c), L.stream())
+    if row:
+        qr = torch.empty(*lead, r, c, dtype=torch.uint8, device=dev)
+        sfr = _sf_buf(r, c, group_r, dev, lead)
+    if col:
+        qc = torch.empty(*lead, r, c, dtype=torch.uint8, device=dev)
+        sfc = _sf_buf(c, r, group_c, dev, lead)
+    L.call("bones_mx2_quant", L.ptr(x2), _L(x2.stride(-2)), L.ptr(qr), L.ptr(sfr), _I(group_r), L.ptr(qc), L.ptr(sfc), _I(group_c),
+           _L(r), _L(c), _I(lead[0] if lead else 1), L.stream())
     COUNTS["mx_quant"] += 1
     return qr, sfr, qc, sfc
 
@@ -90,11 +89,8 @@ def weight_q2_batched(w3: torch.Tensor, transposed: bool, bn: int):
     ent = _CACHE.get(key)
     if ent is None or ent[0] != _EPOCH[0] or ent[1] != w3._version:
         src = w3.detach().transpose(1, 2).contiguous() if transposed else w3.detach()
-        e, rows, k = src.shape
-        q = torch.empty(e, rows, k, dtype=torch.uint8, device=w3.device)
-        sf = torch.zeros(e, sf2_bytes(rows, k, bn), dtype=torch.uint8, device=w3.device)
-        for j in range(e):
-            quant2(src[j], group_r=bn, out=(q[j], sf[j], None, None))
+        src = src if src.is_contiguous() else src.contiguous()
+        q, sf, _, _ = quant2(src, group_r=bn)
         ent = (_EPOCH[0], w3._version, q, sf)
         _CACHE[key] = ent
     return ent[2], ent[3]
@@ -317,15 +313,10 @@ class _MxExpertsFn(torch.autograd.Function):
         e, f, d = w_fc.shape
         x3 = C._c(xs).view(e, -1, d)
         rows = x3.shape[1]
-        dev = xs.device
-        xq, xsf, _, _ = quant2(x3.view(-1, d))                              # rows % 128 == 0: batches are whole chunk runs
-        xq_c = torch.empty(e, rows, d, dtype=torch.uint8, device=dev)
-        xsf_c = torch.zeros(e, sf2_bytes(d, rows, BN_WGRAD), dtype=torch.uint8, device=dev)
-        for j in range(e):
-            quant2(x3[j], row=False, col=True, group_c=BN_WGRAD, out=(None, None, xq_c[j], xsf_c[j]))
+        xq, xsf, xq_c, xsf_c = quant2(x3, col=True, group_c=BN_WGRAD)
         bn1, bn2 = bn_for(d, True), bn_for(f)
         wq, wsf = weight_q2_batched(w_fc, False, bn1)
-        h, hq, hsf, hq_c, hsf_c = gemm2(xq.view(e, rows, d), xsf, wq, wsf, rows, f, d, epi=GE_RELU2, want_q=True, want_t=True,
+        h, hq, hsf, hq_c, hsf_c = gemm2(xq, xsf, wq, wsf, rows, f, d, epi=GE_RELU2, want_q=True, want_t=True,
                                         dt_group=BN_WGRAD, bn=bn1, batch=e)
         pq, psf = weight_q2_batched(w_proj, False, bn2)
         y = gemm2(hq, hsf, pq, psf, rows, d, f, bn=bn2, batch=e)[0]
@@ -341,14 +332,10 @@ class _MxExpertsFn(torch.autograd.Function):
         rows = h.shape[1]
         dev = dy.device
         dy3 = C._c(dy).view(e, rows, d)
-        dyq, dysf, _, _ = quant2(dy3.view(-1, d))
-        dyq_c = torch.empty(e, rows, d, dtype=torch.uint8, device=dev)
-        dysf_c = torch.zeros(e, sf2_bytes(d, rows, 128), dtype=torch.uint8, device=dev)
-        for j in range(e):
-            quant2(dy3[j], row=False, col=True, group_c=128, out=(None, None, dyq_c[j], dysf_c[j]))
+        dyq, dysf, dyq_c, dysf_c = quant2(dy3, col=True, group_c=128)
         bn1, bn2 = bn_for(d, True), bn_for(f)
         ptq, ptsf = weight_q2_batched(w_proj, True, bn1)                   # [e, f, d]: dh = dy @ w_proj
-        _, dpq, dpsf, dpq_c, dpsf_c = gemm2(dyq.view(e, rows, d), dysf, ptq, ptsf, rows, f, d, epi=GE_MUL_2SQRT, r=h, want_d=False,
+        _, dpq, dpsf, dpq_c, dpsf_c = gemm2(dyq, dysf, ptq, ptsf, rows, f, d, epi=GE_MUL_2SQRT, r=h, want_d=False,
                                              want_q=True, want_t=True, dt_group=128, bn=bn1, batch=e)
         ftq, ftsf = weight_q2_batched(w_fc, True, bn2)                     # [e, d, f]: dx = dpre @ w_fc
         dx = gemm2(dpq, dpsf, ftq, ftsf, rows, d, f, bn=bn2, batch=e)[0]
@@ -358,7 +345,7 @@ class _MxExpertsFn(torch.autograd.Function):
             ret = None
             if g is None:
                 g = ret = torch.zeros(w.shape, dtype=torch.float32, device=dev)
-            gemm2(a, asf, b, bsf, w.shape[1], w.shape[2], rows, a_major=1, b_major=1, epi=GE_ACC_F32, out=g, bn=BN_WGRAD, batch=e)
+            gemm2(a, asf, b, bsf, n_out, n_in, rows, a_major=1, b_major=1, epi=GE_ACC_F32, out=g, bn=BN_WGRAD, batch=e)
             outs.append(ret.to(w.dtype) if ret is not None else None)
         return dx.view(dy.shape), outs[0], outs[1]
 
