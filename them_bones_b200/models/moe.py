@@ -20,7 +20,6 @@ import torch.nn.functional as F
 
 from .. import ops
 from ..config import GPTConfig
-from ..ref import functional as RF
 
 
 def moe_seed(*parts) -> int:
@@ -109,8 +108,7 @@ class MoeMLP(nn.Module):
         b, t, d = xn.shape
         n = b * t
         h = xn.reshape(n, d)
-        logits = ops.router_logits(h, self.router)
-        p, idx, gates = RF.moe_route(logits, self.topk)
+        idx, gates, aux, stats = ops.moe_router(h, self.router, self.topk, self.aux_w, self.z_w, want_aux=moe_aux is not None)
         # a sequence of t tokens cannot send more than t of them to one expert: the same routing with a smaller slot
         # buffer for short inputs (a decode step is one token per sequence)
         cap = min(self.cap, t)
@@ -126,7 +124,6 @@ class MoeMLP(nn.Module):
         if residual is not None:
             out = out + residual
         if moe_aux is not None:
-            aux, lb, z, f = RF.moe_aux_terms(p, logits, idx, self.n_exp, self.topk, self.aux_w, self.z_w)
             kept = (slot < self.n_exp * b * cap).float().mean()
-            moe_aux.append((aux, torch.cat([torch.stack([kept, lb.detach(), z.detach()]), f.detach()])))
+            moe_aux.append((aux, torch.cat([kept.view(1), stats])))
         return out

@@ -262,6 +262,19 @@ def router_logits(h, router):
     return F.linear(h.float(), router.float())
 
 
+def moe_router(h, router, topk, aux_w=0.0, z_w=0.0, want_aux=True):
+    """Router of an MoE block: ``(idx [n, k], gates [n, k], aux, stats)`` with the auxiliary loss ``aux_w * lb + z_w * z`` and
+    its parts ``stats = [lb, z, f_0 ..]`` (both None unless ``want_aux``).  Natively one kernel each way around the logits GEMM."""
+    if native(h) and _cuda().moe_router_ok(h, router, topk):
+        return _cuda().moe_router(h, router, topk, aux_w, z_w, want_aux)
+    logits = router_logits(h, router)
+    p, idx, gates = RF.moe_route(logits, topk)
+    if not want_aux:
+        return idx, gates, None, None
+    aux, lb, z, f = RF.moe_aux_terms(p, logits, idx, router.shape[0], topk, aux_w, z_w)
+    return idx, gates, aux, torch.cat([torch.stack([lb.detach(), z.detach()]), f.detach()])
+
+
 def moe_slots(idx, b, t, n_exp, cap):
     """Causal per-sequence capacity slotting: ``(slot [n, k], token_of_slot [E*b*cap])``."""
     if native(idx):

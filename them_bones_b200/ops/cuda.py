@@ -619,6 +619,61 @@ def router_logits(h, router):
     return _RouterFn.apply(_c(h), router)
 
 
+class _MoeRouterFn(torch.autograd.Function):
+    """The whole router: logits on the padded tensor-core GEMM (as in ``_RouterFn``), then one kernel for soft-max, top-k choice,
+    gates and the statistics of the auxiliary loss; backward one kernel that writes the padded bf16 logit gradient both
+    gradient GEMMs read (``csrc/router.cu``)."""
+
+    @staticmethod
+    def forward(ctx, h, router, topk, aux_w, z_w, want_aux):
+        e, c = router.shape
+        n, dev = h.shape[0], h.device
+        rp = torch.zeros(128, c, dtype=BF16, device=dev)
+        rp[:e].copy_(router.detach())
+        logits = mm_nt(h, rp, epi=L.EPI_F32, out_dtype=torch.float32)
+        idx = torch.empty(n, topk, dtype=torch.int64, device=dev)
+        gates = torch.empty(n, topk, dtype=torch.float32, device=dev)
+        aux = torch.empty((), dtype=torch.float32, device=dev) if want_aux else None
+        stats = torch.empty(2 + e, dtype=torch.float32, device=dev) if want_aux else None
+        part = torch.empty(-(-n // 128) * (2 * e + 1), dtype=torch.float32, device=dev) if want_aux else None
+        L.call("bones_moe_route_fwd", L.ptr(logits), _L(128), _L(n), _I(e), _I(topk), L.ptr(idx), L.ptr(gates), L.ptr(part), _F(aux_w), _F(z_w),
+               L.ptr(aux), L.ptr(stats), L.stream(), launches=2 if want_aux else 1)
+        ctx.save_for_backward(h, rp, logits, idx, stats)
+        ctx.meta, ctx.rdtype = (e, topk, aux_w, z_w), router.dtype
+        ctx.set_materialize_grads(False)
+        ctx.mark_non_differentiable(*([idx, stats] if want_aux else [idx]))
+        COUNTS["moe_router"] += 1
+        return idx, gates, aux, stats
+
+    @staticmethod
+    def backward(ctx, _didx, dgates, daux, _dstats):
+        h, rp, logits, idx, stats = ctx.saved_tensors
+        e, topk, aux_w, z_w = ctx.meta
+        n, c = h.shape
+        dlp = torch.empty(n, 128, dtype=BF16, device=h.device)
+        dgates = _c(dgates.float()) if dgates is not None else None
+        daux = _c(daux.float()) if daux is not None else None
+        f = ctypes.c_void_p(stats.data_ptr() + 8) if stats is not None else L.ptr(None)
+        L.call("bones_moe_route_bwd", L.ptr(logits), _L(128), _L(n), _I(e), _I(topk), L.ptr(idx), L.ptr(dgates), L.ptr(daux), f, _F(aux_w), _F(z_w),
+               L.ptr(dlp), L.stream())
+        dh = mm_nn(dlp, rp) if ctx.needs_input_grad[0] else None
+        dr = None
+        if ctx.needs_input_grad[1]:
+            dr32 = torch.zeros(128, c, dtype=torch.float32, device=h.device)
+            mm_tn_acc(dlp, h, dr32)
+            dr = dr32[:e].to(ctx.rdtype)
+        return dh, dr, None, None, None, None
+
+
+def moe_router_ok(h, router, topk):
+    """The fused router covers bf16 activations, up to 64 experts and the GEMM's 16-byte rows."""
+    return h.dtype == BF16 and router.shape[0] <= 64 and h.shape[1] % 8 == 0 and topk in (1, 2) and h.shape[0] > 0
+
+
+def moe_router(h, router, topk, aux_w, z_w, want_aux):
+    return _MoeRouterFn.apply(_c(h), router, topk, float(aux_w), float(z_w), want_aux)
+
+
 def moe_slots(idx, b, t, n_exp, cap):
     """Native capacity slotting: ``idx [b*t, k]`` int64 -> ``(slot [b*t, k], tok [E*b*cap])``."""
     n, k = idx.shape
@@ -728,7 +783,6 @@ class _ExpertsFn(torch.autograd.Function):
             ret = None
             if g is None:
                 g = ret = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
-            n_out, n_in = w.shape[1], w.shape[2]
             L.gemm(a, b, g, m=n_out, n=n_in, k=rows, lda=n_out, ldb=n_in, ldd=n_in, a_major=1, b_major=1,
                    epi=L.EPI_ACC_F32, batch=e, stride_a=rows * n_out, stride_b=rows * n_in, stride_d=n_out * n_in)
             outs.append(ret.to(w.dtype) if ret is not None else None)
