@@ -342,6 +342,11 @@ class _MxExpertsFn(torch.autograd.Function):
         outs = []
         for w, a, asf, b, bsf in ((ctx.ws[0], dpq_c, dpsf_c, xq_c, xsf_c), (ctx.ws[1], dyq_c, dysf_c, hq_c, hsf_c)):
             g = getattr(w, "main_grad", None)
+            n_out, n_in = w.shape[1], w.shape[2]
+            if g is None and w.dtype == torch.bfloat16 and e * -(-n_out // 256) * -(-n_in // 256) >= C.WGRAD_WHOLE_TILES:
+                # enough output tiles that the contraction is not split: the bf16 gradient leaves the GEMM as it is
+                outs.append(gemm2(a, asf, b, bsf, n_out, n_in, rows, a_major=1, b_major=1, bn=BN_WGRAD, batch=e)[0])
+                continue
             ret = None
             if g is None:
                 g = ret = torch.zeros(w.shape, dtype=torch.float32, device=dev)
