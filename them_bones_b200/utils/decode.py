@@ -16,6 +16,8 @@ from .. import ops
 from ..models.moe import MoeMLP
 from ..ref import functional as RF
 
+_I = ctypes.c_int
+
 
 def L_check():
     from ..ops import _lib as L
@@ -158,13 +160,76 @@ class NativeDecoder:
         # adds in a fixed order (no atomics: a step is reproducible bit for bit).
         self.split = b <= 128 and cfg.n_embd % 256 == 0 and a % 256 == 0
         self.dense = [not isinstance(blk.mlp, MoeMLP) for blk in model.transformer.h]
-        if self.split:
+        self.fused = self._fused_ok()
+        if self.fused:
+            c, f32, bf = cfg.n_embd, torch.float32, torch.bfloat16
+            self.wqkv = [torch.cat([blk.attn.c_q.weight, blk.attn.c_k.weight, blk.attn.c_v.weight]) for blk in model.transformer.h]
+            self.x0, self.xa, self.xb = (torch.empty(b, c, dtype=bf, device=dev) for _ in range(3))
+            self.qkv = torch.empty(b, 3 * a, dtype=bf, device=dev)
+            self.h = torch.empty(b, cfg.mlp_ratio * c, dtype=bf, device=dev)
+            self.ssq_a, self.ssq_b = (torch.empty(c // 128, b, dtype=f32, device=dev) for _ in range(2))
+            self.ticket = torch.zeros(1, dtype=torch.int32, device=dev)
+            self.last_logits = torch.empty(b, model.lm_head.weight.shape[0], dtype=bf, device=dev)
+        elif self.split:
             self.wqkv = [torch.cat([blk.attn.c_q.weight, blk.attn.c_k.weight, blk.attn.c_v.weight]).contiguous()
                          for blk in model.transformer.h]
             ws = self.wqkv + [blk.attn.c_proj.weight for blk in model.transformer.h]
             ws += [w for blk, dense in zip(model.transformer.h, self.dense) if dense for w in (blk.mlp.c_fc.weight, blk.mlp.c_proj.weight)]
             self.split = all(w.shape[1] % 256 == 0 for w in ws)
             self.part = torch.empty(max(b * w.shape[0] * (w.shape[1] // 256) for w in ws), dtype=torch.float32, device=dev)
+
+    def _fused_ok(self) -> bool:
+        """Whether the step runs on the kernels of ``csrc/decode_gemm.cu``: a plain dense decoder with at most 128 sequences."""
+        model, cfg = self.model, self.model.config
+        ws = [w for blk, dense in zip(model.transformer.h, self.dense) if dense
+              for w in (blk.attn.c_q.weight, blk.attn.c_k.weight, blk.attn.c_v.weight, blk.attn.c_proj.weight, blk.mlp.c_fc.weight, blk.mlp.c_proj.weight)]
+        ws += [model.lm_head.weight, model.transformer.wte.weight]
+        scalars = [v for blk in model.transformer.h for v in (blk.resid_lambda, blk.x0_lambda)]
+        return (self.tok.shape[0] <= 128 and all(self.dense) and model.tables is None and model.value_embeds is None and not model.n_skip
+                and len(model.transformer.h) > 0 and cfg.n_embd % 128 == 0
+                and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.shape[0] % 128 == 0 and w.shape[1] % 64 == 0 for w in ws)
+                and all(v.dtype == torch.float32 for v in scalars) and model.cos.dtype == torch.float32 and model.sin.dtype == torch.float32)
+
+    def _proj(self, x, w, out, epi, ssq=None, n_ssq=0, res=None, mix=None, ssq_out=None):
+        """One projection of the fused step (``bones_decode_gemm``).  The contraction is split over a cluster until the CTAs
+        cover the SMs: a tile is 128 output columns, so 1280 columns are 10 tiles and 8 CTAs share each."""
+        from ..ops import _lib as L
+        b, (n, k) = x.shape[0], w.shape
+        splits, most = 1, 4 if b <= 16 else 8
+        while splits < most and n // 128 * splits * 2 <= 160 and splits * 2 <= k // 64:
+            splits *= 2
+        x0, ma, mb = (self.x0, mix[0], mix[1]) if mix is not None else (None, None, None)
+        L.call("bones_decode_gemm", L.ptr(x), L.ptr(w), L.ptr(out), _I(b), _I(n), _I(k), _I(splits), _I(epi), L.ptr(ssq), _I(n_ssq), L.ptr(res),
+               L.ptr(x0), L.ptr(ma), L.ptr(mb), L.ptr(ssq_out), ctypes.c_float(self.model.config.softcap), _I(1),
+               L.stream())
+
+    def _step_fused(self):
+        """Five kernels a layer (qkv, attention, out, c_fc, c_proj), one before the first and two after the last; the norms,
+        the residual mix, ReLU^2 and the soft-cap are in the projections' epilogues."""
+        from ..ops import _lib as L
+        model, cache, cfg = self.model, self.cache, self.model.config
+        tok, pos, b, c = self.tok, self.pos, self.tok.shape[0], cfg.n_embd
+        tmax, tiles = cache.k.shape[2], c // 128
+        ds = cache.doc_start if cfg.doc_mask else None
+        hs = model.transformer.h
+        w = model.transformer.wte.weight
+        L.call("bones_decode_begin", L.ptr(tok), L.ptr(pos), L.ptr(ds), ctypes.c_longlong(cfg.bos_id), L.ptr(w), ctypes.c_longlong(w.shape[0]), _I(c),
+               L.ptr(hs[0].resid_lambda), L.ptr(hs[0].x0_lambda), L.ptr(self.x0), L.ptr(self.xa), L.ptr(self.ssq_a), _I(b), L.stream())
+        n_ssq = 1
+        for i, blk in enumerate(hs):
+            at = blk.attn
+            self._proj(self.xa, self.wqkv[i], self.qkv, 0, ssq=self.ssq_a, n_ssq=n_ssq)
+            L.call("bones_decode_attn_step", L.ptr(self.qkv), L.ptr(model.cos), L.ptr(model.sin), L.ptr(cache.k[i]), L.ptr(cache.v[i]), L.ptr(pos), L.ptr(ds),
+                   L.ptr(self.y), _I(b), _I(at.n_head), _I(tmax), ctypes.c_float(at.scale), _I(at.window // 128), L.stream())
+            self._proj(self.y, at.c_proj.weight, self.xb, 2, res=self.xa, ssq_out=self.ssq_b)
+            self._proj(self.xb, blk.mlp.c_fc.weight, self.h, 1, ssq=self.ssq_b, n_ssq=tiles)
+            nxt = hs[i + 1] if i + 1 < len(hs) else None
+            mix = (nxt.resid_lambda, nxt.x0_lambda) if nxt is not None else None
+            self._proj(self.h, blk.mlp.c_proj.weight, self.xa, 2, res=self.xb, mix=mix, ssq_out=self.ssq_a)
+            n_ssq = tiles
+        self._proj(self.xa, model.lm_head.weight, self.last_logits, 3, ssq=self.ssq_a, n_ssq=n_ssq)
+        L.call("bones_decode_end", L.ptr(self.last_logits), ctypes.c_longlong(self.last_logits.shape[1]), _I(cfg.vocab_size), L.ptr(pos),
+               L.ptr(self.prompt_len), L.ptr(self.out), _I(self.out.shape[1]), L.ptr(tok), L.ptr(self.ticket), _I(b), L.stream())
 
     def _lin(self, x, w, mode=0, residual=None):
         """``x [b, k] @ w[n, k]^T`` as ``k / 256`` batched partial products into fp32 slices, then their ordered sum as
@@ -184,6 +249,8 @@ class NativeDecoder:
     def _step(self):
         from ..ops import _lib as L
         from ..ops import cuda as C
+        if self.fused:
+            return self._step_fused()
         model, cache, cfg = self.model, self.cache, self.model.config
         tok, pos = self.tok, self.pos
         b, tmax = tok.shape[0], cache.k.shape[2]
