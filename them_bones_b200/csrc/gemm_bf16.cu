@@ -71,7 +71,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   constexpr uint32_t A_BYTES = BM * BK * 2;
   constexpr uint32_t B_BYTES = BN * BK * 2;
   constexpr uint32_t STAGE_BYTES = A_BYTES + B_BYTES;
-  constexpr uint32_t TMEM_COLS = 2 * BN;   // 256 or 512: power of two
+  constexpr uint32_t TMEM_COLS = BN <= 128 ? 256 : 512;   // two accumulators, rounded up to a power of two
 
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -288,9 +288,32 @@ static int operand_tmap(CUtensorMap* out, const void* ptr, int major, long long 
   return make_tmap(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, ptr, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B);
 }
 
+// Tile width of a single-CTA GEMM whose contraction is not split: the narrowest that needs no more waves of tiles than the
+// widest.  A K block takes about 0.3 us in any width (its loads, not its MMAs: 1000 x 1280 x 5120 takes 31.1, 29.6, 28.4 us in
+// tiles of 256, 192, 128 columns), so fewer waves come first, and within them a narrower tile's shorter prologue and epilogue
+// (300 x 1280 x 1280: 11.8 us in 256, 9.8 in 96; 1000 x 5120 x 1280: two waves of 160 in 18.8, three of 128 in 24.3).
+// A B operand stored along N comes in 64-column swizzle atoms.
+static int pick_bn(long long tiles_m_batch, int N, int b_major, int sms, long long* waves_out) {
+  static const int any[] = {256, 224, 192, 160, 128, 96}, atoms[] = {256, 192, 128};
+  const int* c = b_major ? atoms : any;
+  const int n = b_major ? 3 : 6;
+  long long least = -1;
+  int bn = 256;
+  for (int i = 0; i < n; ++i) {
+    const long long waves = (tiles_m_batch * ((N + c[i] - 1) / c[i]) + sms - 1) / sms;
+    if (least < 0 || waves <= least) { least = waves; bn = c[i]; }
+  }
+  if (waves_out) *waves_out = least;
+  return bn;
+}
+
 }  // namespace bones
 
 extern "C" {
+
+int bones_gemm_bf16_pair(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int batch, long long lda,
+                         long long ldb, long long ldd, long long ldr, long long strideA, long long strideB, long long strideD,
+                         long long strideR, int a_major, int b_major, int epi, float alpha, float beta, int splits, int atomic, void* stream);
 
 // Returns 0 on success, a CUDA error code (> 0) or a negative descriptor-encoding error.
 int bones_gemm_bf16(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int batch, long long lda,
@@ -301,7 +324,10 @@ int bones_gemm_bf16(const void* A, const void* B, void* D, const void* R, int M,
   if ((lda % 8) || (ldb % 8) || ((uintptr_t)A & 15) || ((uintptr_t)B & 15) || ((uintptr_t)D & 15)) return -2;
   const bool f32out = epi == EPI_ACC_F32 || epi == EPI_F32 || epi == EPI_F32_RES;
   if (ldd % (f32out ? 4 : 8)) return -3;
-  int bn = force_bn ? force_bn : (N > 128 ? 256 : 128);
+  int dev = 0, sms = 0;
+  BONES_CHECK(cudaGetDevice(&dev));
+  BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  int bn = force_bn ? force_bn : N <= 128 ? 128 : epi == EPI_ACC_F32 ? 256 : pick_bn((long long)((M + BM - 1) / BM) * batch, N, b_major, sms, nullptr);
   GemmParams p;
   p.M = M; p.N = N; p.K = K; p.batch = batch;
   p.a_major = a_major; p.b_major = b_major; p.epi = epi;
@@ -320,8 +346,42 @@ int bones_gemm_bf16(const void* A, const void* B, void* D, const void* R, int M,
   rc = operand_tmap(&tb, B, b_major, N, K, ldb, strideB, batch, bn);
   if (rc) return rc;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
-  if (bn == 256) return launch_gemm<256, 4>(ta, tb, p, s);
-  return launch_gemm<128, 6>(ta, tb, p, s);
+  switch (bn) {
+    case 256: return launch_gemm<256, 4>(ta, tb, p, s);
+    case 224: return launch_gemm<224, 4>(ta, tb, p, s);
+    case 192: return launch_gemm<192, 5>(ta, tb, p, s);
+    case 160: return launch_gemm<160, 5>(ta, tb, p, s);
+    case 128: return launch_gemm<128, 6>(ta, tb, p, s);
+    case 96: return launch_gemm<96, 7>(ta, tb, p, s);
+  }
+  return -2;
+}
+
+// Chooses between this kernel and the CTA pairs (gemm_bf16_2cta.cu: 256 x 256 tiles, one third less L2 traffic per flop).
+// fp32 accumulation splits its contraction, so there few output tiles still fill the pairs when K is long (weight gradients).
+// Otherwise single CTAs take what they finish in one wave (300 x 1280 x 1280: 9.8 us against 11.7 on pairs), the pairs the rest
+// (2000 x 5120 x 1280: 25.5 us against 27.1).
+int bones_gemm_bf16_auto(const void* A, const void* B, void* D, const void* R, int M, int N, int K, int batch, long long lda,
+                         long long ldb, long long ldd, long long ldr, long long strideA, long long strideB, long long strideD,
+                         long long strideR, int a_major, int b_major, int epi, float alpha, float beta, int splits, int atomic, void* stream) {
+  using namespace bones;
+  if (M <= 0 || N <= 0 || K <= 0 || batch <= 0) return 0;
+  const long long tiles = (long long)((M + 255) / 256) * ((N + 255) / 256) * batch;
+  bool pair = M >= 256 && N >= 256;
+  if (pair && epi == EPI_ACC_F32) {
+    pair = tiles >= 37 || K >= 8192 * 37 / tiles;
+  } else if (pair) {
+    int dev = 0, sms = 0;
+    BONES_CHECK(cudaGetDevice(&dev));
+    BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    long long waves = 0;
+    pick_bn((long long)((M + BM - 1) / BM) * batch, N, b_major, sms, &waves);
+    pair = waves > 1;
+  }
+  return pair ? bones_gemm_bf16_pair(A, B, D, R, M, N, K, batch, lda, ldb, ldd, ldr, strideA, strideB, strideD, strideR, a_major, b_major, epi,
+                                     alpha, beta, splits, atomic, stream)
+              : bones_gemm_bf16(A, B, D, R, M, N, K, batch, lda, ldb, ldd, ldr, strideA, strideB, strideD, strideR, a_major, b_major, epi, alpha,
+                                beta, 0, splits, atomic, stream);
 }
 
 }  // extern "C"

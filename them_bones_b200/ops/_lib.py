@@ -22,13 +22,28 @@ def lib_path() -> str:
     return _PATH
 
 
+_P, _I, _L, _F = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+_GEMM = [_P] * 4 + [_I] * 4 + [_L] * 8 + [_I] * 3 + [_F] * 2
+# Entry points called with plain Python numbers (converted by ctypes itself: building two dozen argument objects in Python was
+# a third of a GEMM's host time).  Everything else passes ctypes objects.
+SIGNATURES = {
+    "bones_gemm_bf16": _GEMM + [_I] * 3 + [_P],                     # ..., force_bn, splits, atomic, stream
+    "bones_gemm_bf16_pair": _GEMM + [_I] * 2 + [_P],
+    "bones_gemm_bf16_auto": _GEMM + [_I] * 2 + [_P],
+    "bones_gemm_mxfp8_pair": [_P] * 8 + [_I] + [_P] * 2 + [_I] * 5 + [_L] * 8 + [_I] * 3 + [_F] * 2 + [_I] * 3 + [_P],
+}
+
+
 def load():
     global _LIB
     if _LIB is None:
         if not os.path.exists(_PATH):
             raise RuntimeError(f"native library missing: {_PATH}; run `python -m them_bones_b200.csrc.build` "
                                "(or __graft_entry__.build()) first")
-        _LIB = ctypes.CDLL(_PATH)
+        lib = ctypes.CDLL(_PATH)
+        for name, types in SIGNATURES.items():
+            getattr(lib, name).argtypes = types
+        _LIB = lib
     return _LIB
 
 
@@ -45,10 +60,8 @@ def ptr(t):
 
 
 def stream():
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
-
-
-_I, _L, _F = ctypes.c_int, ctypes.c_longlong, ctypes.c_float
+    """The current stream's handle, without building a ``torch.cuda.Stream`` object (4 us of a 10 us launch)."""
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
 
 
 LAUNCHES = [0]        # native kernel launches issued by this process (`launches`: an entry point with more than one kernel)
@@ -56,7 +69,7 @@ LAUNCHES = [0]        # native kernel launches issued by this process (`launches
 
 def call(name: str, *args, launches: int = 1):
     LAUNCHES[0] += launches
-    rc = getattr(load(), name)(*args)
+    rc = getattr(_LIB or load(), name)(*args)
     if rc != 0:
         raise RuntimeError(f"{name} failed with code {rc}")
 
@@ -96,23 +109,19 @@ PAIR_MODE = os.environ.get("BONES_GEMM_PAIR", "auto")      # auto | 0 | 1
 
 def gemm(a, b, d, *, m, n, k, lda, ldb, ldd, a_major=0, b_major=0, epi=EPI_BF16, r=None, ldr=0, alpha=1.0, beta=1.0,
          batch=1, stride_a=0, stride_b=0, stride_d=0, stride_r=0, force_bn=0, splits=0, pair=None, d_ptr=None, atomic=False):
-    """``d = epilogue(alpha * a @ b^T, r)``; see csrc/gemm_bf16.cu for operand layouts.  Large problems run on CTA
-    pairs (csrc/gemm_bf16_2cta.cu: 256 x 256 tiles, one third less L2 traffic per flop); small ones on single CTAs."""
+    """``d = epilogue(alpha * a @ b^T, r)``; see csrc/gemm_bf16.cu for operand layouts.  ``pair=None``: CTA
+    pairs (csrc/gemm_bf16_2cta.cu) or single CTAs by the rule of ``bones_gemm_bf16_auto``."""
+    auto = pair is None and PAIR_MODE == "auto" and force_bn == 0
     if pair is None:
-        if PAIR_MODE == "auto":
-            tiles = -(-m // 256) * -(-n // 256) * batch
-            # few output tiles still fill the pairs when a long K is split (weight gradients)
-            pair = force_bn == 0 and m >= 256 and n >= 256 and (tiles >= 37 or (epi == EPI_ACC_F32 and k >= 8192 * 37 // tiles))
-        else:
-            pair = PAIR_MODE == "1" and force_bn == 0
+        pair = PAIR_MODE == "1" and force_bn == 0
     # d_ptr: raw device address used instead of ``d`` (e.g. the same buffer in another GPU's memory); atomic: fp32
     # accumulation by vector atomics even without split-K, for outputs several GPUs add into at once
-    dp = ptr(d) if d_ptr is None else ctypes.c_void_p(int(d_ptr))
-    if pair:
-        call("bones_gemm_bf16_pair", ptr(a), ptr(b), dp, ptr(r), _I(m), _I(n), _I(k), _I(batch), _L(lda), _L(ldb),
-             _L(ldd), _L(ldr), _L(stride_a), _L(stride_b), _L(stride_d), _L(stride_r), _I(a_major), _I(b_major), _I(epi),
-             _F(alpha), _F(beta), _I(splits), _I(int(atomic)), stream())
+    dp = d.data_ptr() if d_ptr is None else int(d_ptr)
+    rp = r.data_ptr() if r is not None else 0
+    st = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    if auto or pair:
+        call("bones_gemm_bf16_auto" if auto else "bones_gemm_bf16_pair", a.data_ptr(), b.data_ptr(), dp, rp, m, n, k, batch, lda, ldb, ldd, ldr,
+             stride_a, stride_b, stride_d, stride_r, a_major, b_major, epi, alpha, beta, splits, int(atomic), st)
         return
-    call("bones_gemm_bf16", ptr(a), ptr(b), dp, ptr(r), _I(m), _I(n), _I(k), _I(batch), _L(lda), _L(ldb), _L(ldd),
-         _L(ldr), _L(stride_a), _L(stride_b), _L(stride_d), _L(stride_r), _I(a_major), _I(b_major), _I(epi), _F(alpha),
-         _F(beta), _I(force_bn), _I(splits), _I(int(atomic)), stream())
+    call("bones_gemm_bf16", a.data_ptr(), b.data_ptr(), dp, rp, m, n, k, batch, lda, ldb, ldd, ldr, stride_a, stride_b, stride_d, stride_r, a_major,
+         b_major, epi, alpha, beta, force_bn, splits, int(atomic), st)

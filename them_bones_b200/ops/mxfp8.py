@@ -134,10 +134,9 @@ def gemm2(aq, sfa, bq, sfb, m, n, k, *, a_major=0, b_major=0, epi=GE_BF16, r=Non
     ldd = d.stride(-2) if d is not None else 0
     sr = r.stride(0) if (r is not None and batch > 1) else 0
     ldr = r.stride(-2) if r is not None else 0
-    L.call("bones_gemm_mxfp8_pair", L.ptr(aq), L.ptr(sfa), L.ptr(bq), L.ptr(sfb), L.ptr(d), L.ptr(r), L.ptr(dq), L.ptr(dsf),
-           _I(dq_group), L.ptr(dt), L.ptr(dtsf), _I(dt_group), _I(m), _I(n), _I(k), _I(batch), _L(lda), _L(ldb), _L(ldd), _L(ldr),
-           _L(sa), _L(sb), _L(sd), _L(sr), _I(a_major), _I(b_major), _I(epi), _F(alpha), _F(beta), _I(bn), _I(splits), _I(0),
-           L.stream())
+    dp = [0 if t is None else t.data_ptr() for t in (aq, sfa, bq, sfb, d, r, dq, dsf, dt, dtsf)]
+    L.call("bones_gemm_mxfp8_pair", *dp[:8], dq_group, *dp[8:], dt_group, m, n, k, batch, lda, ldb, ldd, ldr, sa, sb, sd, sr, a_major, b_major, epi,
+           alpha, beta, bn, splits, 0, torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
     COUNTS["mx_gemm"] += 1
     return d, dq, dsf, dt, dtsf
 
