@@ -39,6 +39,12 @@ struct Gemm2Params {
   int splits;
   int atomic;          // E2_ACC_F32: always add with atomics (other GPUs add into the same buffer at the same time)
   int wide;            // rows are 32-byte aligned: use 256-bit global accesses in the epilogue
+  // logits with statistics (template flag LSE): D = bf16(beta tanh(alpha acc)) (D null: not stored), for each row the sum of
+  // exp(z - beta) over this half tile's columns below `vocab`, and the target's logit
+  float* part;         // [2 tiles_n, M]
+  int vocab;
+  const long long* targets;
+  float* z_target;     // [M] or null
 };
 
 constexpr int PM = 256;      // pair tile M (128 per CTA)
@@ -49,6 +55,7 @@ constexpr uint32_t PA_BYTES = 128 * PK * 2;
 constexpr uint32_t PB_BYTES = 128 * PK * 2;
 constexpr uint32_t PSTAGE_BYTES = PA_BYTES + PB_BYTES;
 constexpr int kGroupM2 = 8;
+constexpr size_t kPairSmem = (size_t)PSTAGES * PSTAGE_BYTES + 8 * (2 * PSTAGES + 4) + 16 + 1024;
 
 __device__ __forceinline__ void decode_tile2(int tile, int tiles_m, int tiles_n, int& b, int& mb, int& nb) {
   const int per_batch = tiles_m * tiles_n;
@@ -106,6 +113,53 @@ __device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
                : "memory");
 }
 
+// 32 accumulator columns of one row as soft-capped logits; returns the row's sum of exp(z - beta) over them.  The values that are
+// summed are the bf16 ones that are stored, so the statistics belong to the logits that the gradient pass reads.
+__device__ __forceinline__ float logits_chunk(const uint32_t (&r)[32], float alpha, float beta, __nv_bfloat16* D, bool wide, int col0, int vocab,
+                                              long long tgt, float* z_target) {
+  uint32_t w[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    w[j] = pack_bf16(beta * tanh_approx(__uint_as_float(r[2 * j]) * alpha), beta * tanh_approx(__uint_as_float(r[2 * j + 1]) * alpha));
+  float s = 0.f;
+  const float k2 = beta * 1.4426950408889634f;
+  auto ex = [&](float z) {
+    float e;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(fmaf(z, 1.4426950408889634f, -k2)));
+    return e;
+  };
+  if (col0 + 32 <= vocab) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) s += ex(__uint_as_float(w[j] << 16)) + ex(__uint_as_float(w[j] & 0xffff0000u));
+  } else {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (col0 + 2 * j < vocab) s += ex(__uint_as_float(w[j] << 16));
+      if (col0 + 2 * j + 1 < vocab) s += ex(__uint_as_float(w[j] & 0xffff0000u));
+    }
+  }
+  if (z_target && tgt >= col0 && tgt < min(col0 + 32, vocab)) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      if (tgt == col0 + 2 * j) *z_target = __uint_as_float(w[j] << 16);
+      if (tgt == col0 + 2 * j + 1) *z_target = __uint_as_float(w[j] & 0xffff0000u);
+    }
+  }
+  if (D) {
+    const uint4 u[4] = {make_uint4(w[0], w[1], w[2], w[3]), make_uint4(w[4], w[5], w[6], w[7]), make_uint4(w[8], w[9], w[10], w[11]),
+                        make_uint4(w[12], w[13], w[14], w[15])};
+    if (wide) {
+      st_global_v8(D, u[0], u[1]);
+      st_global_v8(D + 16, u[2], u[3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(D + j * 8) = u[j];
+    }
+  }
+  return s;
+}
+
+template <bool LSE>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(320, 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const Gemm2Params p) {
   extern __shared__ uint8_t smem_raw[];
@@ -259,6 +313,28 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_co
       const bool got = mbar_wait(tfull(acc), acc_phase, abort_flag, p.err, ERR_WAIT_TMEM_FULL);
       if (!__all_sync(0xffffffffu, got)) break;
       tc_fence_after();
+      if constexpr (LSE) {
+        float lsum = 0.f;
+        const long long tgt = row_ok && p.z_target ? p.targets[row] : -1;
+#pragma unroll 1
+        for (int cc = 0; cc < 4; ++cc) {
+          const int c = half * 4 + cc, col0 = nb * PN + c * 32;
+          uint32_t r[32];
+          __syncwarp();
+          BONES_TMEM_LD32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * PN + c * 32), r);
+          tmem_ld_wait();
+          if (row_ok && col0 < p.N)
+            lsum += logits_chunk(r, p.alpha, p.beta, p.D ? reinterpret_cast<__nv_bfloat16*>(p.D) + drow + col0 : nullptr, p.wide != 0, col0, p.vocab, tgt,
+                                 p.z_target ? p.z_target + row : nullptr);
+        }
+        if (row_ok) p.part[(long long)(nb * 2 + half) * p.M + row] = lsum;
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(tempty(acc), 0);
+        acc ^= 1;
+        if (acc == 0) acc_phase ^= 1u;
+        continue;
+      }
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc) {
         const int c = half * 4 + cc;
@@ -343,10 +419,9 @@ int bones_gemm_bf16_pair(const void* A, const void* B, void* D, const void* R, i
   if (rc) return rc;
   rc = operand_tmap2(&tb, B, b_major, N, K, ldb, strideB, batch);
   if (rc) return rc;
-  constexpr size_t smem = (size_t)PSTAGES * PSTAGE_BYTES + 8 * (2 * PSTAGES + 4) + 16 + 1024;
   static bool attr_done = false;
   if (!attr_done) {
-    BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
     attr_done = true;
   }
   int dev = 0, sms = 0;
@@ -373,7 +448,46 @@ int bones_gemm_bf16_pair(const void* A, const void* B, void* D, const void* R, i
   if (p.splits > KB) p.splits = KB;          // every split owns at least one K block (its last block signals the epilogue)
   const int total = base_tiles * p.splits;
   const int clusters = total < pairs ? total : pairs;
-  gemm_bf16_pair_kernel<<<2 * clusters, 320, smem, reinterpret_cast<cudaStream_t>(stream)>>>(ta, tb, p);
+  gemm_bf16_pair_kernel<false><<<2 * clusters, 320, kPairSmem, reinterpret_cast<cudaStream_t>(stream)>>>(ta, tb, p);
+  return (int)cudaGetLastError();
+}
+
+// Soft-capped logits z = cap tanh(x w^T / cap) of x [M, K] and w [N, K] (rows of ldx, ldw elements) into D [M, ldd] (null: they
+// are not stored), with what a cross-entropy needs of them: part [2 ceil(N / 256), M], the sums of exp(z - cap) over the columns
+// below `vocab` by half tile, and z_target [M] (null: not wanted), the logit of each row's target (untouched where the target is
+// outside 0 .. vocab - 1).  N a multiple of 32.
+int bones_logits_stats(const void* x, const void* w, void* D, int M, int N, int K, long long ldx, long long ldw, long long ldd, float cap, int vocab,
+                       float* part, const long long* targets, float* z_target, void* stream) {
+  using namespace bones;
+  if (M <= 0) return 0;
+  if (N <= 0 || K <= 0 || (N % 32) || (ldx % 8) || (ldw % 8) || ((uintptr_t)x & 15) || ((uintptr_t)w & 15) || !part) return -2;
+  if (D && ((ldd % 8) || ((uintptr_t)D & 15))) return -3;
+  if (z_target && !targets) return -2;
+  Gemm2Params p = {};
+  p.M = M; p.N = N; p.K = K; p.batch = 1;
+  p.alpha = 1.0f / cap; p.beta = cap;
+  p.D = D; p.ldd = ldd; p.R = D; p.ldr = ldd;
+  p.err = error_word();
+  p.wide = D && (ldd % 16 == 0) && (((uintptr_t)D & 31) == 0);
+  p.tiles_m = (M + PM - 1) / PM;
+  p.tiles_n = (N + PN - 1) / PN;
+  p.splits = 1;
+  p.part = part; p.vocab = vocab; p.targets = targets; p.z_target = z_target;
+  CUtensorMap ta, tb;
+  int rc = operand_tmap2(&ta, x, 0, M, K, ldx, 0, 1);
+  if (rc) return rc;
+  rc = operand_tmap2(&tb, w, 0, N, K, ldw, 0, 1);
+  if (rc) return rc;
+  static bool attr_done = false;
+  if (!attr_done) {
+    BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+    attr_done = true;
+  }
+  int dev = 0, sms = 0;
+  BONES_CHECK(cudaGetDevice(&dev));
+  BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int tiles = p.tiles_m * p.tiles_n, clusters = tiles < sms / 2 ? tiles : sms / 2;
+  gemm_bf16_pair_kernel<true><<<2 * clusters, 320, kPairSmem, reinterpret_cast<cudaStream_t>(stream)>>>(ta, tb, p);
   return (int)cudaGetLastError();
 }
 

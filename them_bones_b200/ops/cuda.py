@@ -390,6 +390,36 @@ def attention(qkv, cos, sin, n_head, head_dim, scale, doc_start, window):
 LOSS_ROWS = max(128, int(os.environ.get("BONES_LOSS_ROWS", 4096)))       # rows per logits block
 
 
+def _logits_stats_ok(x2, w, vocab) -> bool:
+    """What the logits GEMM with row statistics covers: bf16, whole 32-column chunks, aligned operands."""
+    return (x2.dtype == BF16 and w.dtype == BF16 and w.dim() == 2 and w.stride(1) == 1 and w.shape[0] % 32 == 0 and vocab % 8 == 0 and x2.shape[1] % 8 == 0
+            and w.stride(0) % 8 == 0 and w.data_ptr() % 16 == 0 and x2.data_ptr() % 16 == 0 and LOSS_ROWS <= 65535)
+
+
+def _logits_stats(x2, w, out, vocab, cap, part, targets, z_target):
+    """Soft-capped logits into ``out`` (None: not stored) and their rows' partial sums of exponentials into ``part``."""
+    L.call("bones_logits_stats", L.ptr(x2), L.ptr(w), L.ptr(out), _I(x2.shape[0]), _I(w.shape[0]), _I(x2.shape[1]), _L(x2.stride(0)), _L(w.stride(0)),
+           _L(out.stride(0) if out is not None else 0), _F(cap), _I(vocab), L.ptr(part), L.ptr(targets), L.ptr(z_target), L.stream())
+    COUNTS["gemm"] += 1
+
+
+def _mm_tn_write(dy, x, grad):
+    """``grad [N,K] (fp32) = dy[M,N]^T @ x[M,K]``: the first accumulation into a buffer that holds nothing yet"""
+    m, n = dy.shape
+    k = x.shape[1]
+    L.gemm(dy, x, grad, m=n, n=k, k=m, lda=dy.stride(0), ldb=x.stride(0), ldd=grad.stride(0), a_major=1, b_major=1, epi=L.EPI_F32)
+    COUNTS["gemm"] += 1
+
+
+def _scale_cast(g32, scale, dtype):
+    """``g32`` rounded to ``dtype``, times ``scale`` (a device scalar), rounded again."""
+    if dtype != BF16 or g32.numel() % 8:
+        return g32.to(dtype) * scale.to(dtype)
+    out = torch.empty(g32.shape, dtype=dtype, device=g32.device)
+    L.call("bones_scale_cast", L.ptr(g32), L.ptr(_c(scale.float())), L.ptr(out), _L(g32.numel()), L.stream())
+    return out
+
+
 class _LmHeadLossFn(torch.autograd.Function):
     """Chunked head: for each block of rows the logits GEMM, the softcap cross-entropy (which overwrites the logits
     with their gradient), the dX GEMM and the dW GEMM (accumulating into the head's gradient slab) run back to back, so
@@ -411,9 +441,11 @@ class _LmHeadLossFn(torch.autograd.Function):
         rw = _c(row_weights).view(-1).float() if row_weights is not None else None
         vp = w.shape[0]
         grad_w = getattr(w, "main_grad", None)
-        own_gw = None
+        own_gw, fresh = None, False
         if want_grad and grad_w is None:
-            own_gw = grad_w = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+            # with so many output tiles the contraction is not split: the first block can write instead of accumulate
+            fresh = m > 0 and -(-vp // 256) * -(-w.shape[1] // 256) >= WGRAD_WHOLE_TILES
+            own_gw = grad_w = (torch.empty if fresh else torch.zeros)(w.shape, dtype=torch.float32, device=w.device)
         buf = torch.empty(min(LOSS_ROWS, m), vp, dtype=BF16, device=x.device)
         aux = [(_c(t).view(-1).to(torch.int64), _c(wk).view(-1).float()) for t, wk in (aux or [])][:2]
         nll_aux = torch.zeros(m, dtype=torch.float32, device=x.device) if aux else None
@@ -424,20 +456,37 @@ class _LmHeadLossFn(torch.autograd.Function):
                 out += [L.ptr(aux[k][0][r0:r1]), L.ptr(aux[k][1][r0:r1])] if k < len(aux) else [L.ptr(None), L.ptr(None)]
             return out + [L.ptr(nll_aux[r0:r1] if aux else None)]
 
+        # the logits GEMM leaves the rows' sums of exponentials, so the loss kernels pass over the logits once; label smoothing
+        # needs their plain sum too and takes the two-pass kernel
+        stats = _logits_stats_ok(x2, w, vocab) and label_smoothing == 0.0 and want_grad
+        if stats:
+            rows, dev = buf.shape[0], x.device
+            part = torch.empty(-(-vp // 256) * 2, rows, dtype=torch.float32, device=dev)
+            info = torch.empty(rows, 4, dtype=torch.float32, device=dev)
         for r0 in range(0, m, LOSS_ROWS):
             r1 = min(m, r0 + LOSS_ROWS)
             lg = buf[:r1 - r0]
             # the logits GEMM soft-caps in its epilogue (cap * tanh(. / cap)); the loss kernel then only exponentiates
-            mm_nt(x2[r0:r1], w, out=lg, epi=L.EPI_SOFTCAP, alpha=1.0 / cap, beta=cap)
-            L.call("bones_softcap_ce", L.ptr(lg), _L(vp), L.ptr(tg[r0:r1]), _I(vocab), _F(cap), L.ptr(nll[r0:r1]),
-                   L.ptr(lg if want_grad else None), L.ptr(rw[r0:r1] if rw is not None else None), L.ptr(n_valid),
-                   _F(1.0 / loss_div), _I(r1 - r0), _I(1), *aux_ptrs(r0, r1), _F(label_smoothing), L.stream())
+            if stats:
+                ap = aux_ptrs(r0, r1)
+                _logits_stats(x2[r0:r1], w, lg, vocab, cap, part, None, None)
+                L.call("bones_ce_finish", L.ptr(part), _I(part.shape[0]), _I(r1 - r0), L.ptr(lg), _L(vp), L.ptr(None), L.ptr(tg[r0:r1]), _I(vocab),
+                       _F(cap), L.ptr(nll[r0:r1]), L.ptr(info), L.ptr(rw[r0:r1] if rw is not None else None), L.ptr(n_valid), _F(1.0 / loss_div), *ap,
+                       L.stream())
+                L.call("bones_ce_grad", L.ptr(lg), _L(vp), L.ptr(info), L.ptr(tg[r0:r1]), ap[0], ap[2], _I(vocab), _F(cap), _I(r1 - r0), L.stream())
+            else:
+                mm_nt(x2[r0:r1], w, out=lg, epi=L.EPI_SOFTCAP, alpha=1.0 / cap, beta=cap)
+                L.call("bones_softcap_ce", L.ptr(lg), _L(vp), L.ptr(tg[r0:r1]), _I(vocab), _F(cap), L.ptr(nll[r0:r1]),
+                       L.ptr(lg if want_grad else None), L.ptr(rw[r0:r1] if rw is not None else None), L.ptr(n_valid),
+                       _F(1.0 / loss_div), _I(r1 - r0), _I(1), *aux_ptrs(r0, r1), _F(label_smoothing), L.stream())
             if want_grad:
                 mm_nn_acc(lg, w, dx32[r0:r1])
-                mm_tn_acc(lg, x2[r0:r1], grad_w)
+                if fresh and r0 == 0:
+                    _mm_tn_write(lg, x2[r0:r1], grad_w)
+                else:
+                    mm_tn_acc(lg, x2[r0:r1], grad_w)
         COUNTS["lmhead_loss"] += 1
-        dx = dx32.to(x2.dtype) if want_grad else None
-        ctx.dx, ctx.shp, ctx.own_gw, ctx.wdtype = dx, shp, own_gw, w.dtype
+        ctx.dx, ctx.shp, ctx.own_gw, ctx.xdtype, ctx.wdtype = dx32, shp, own_gw, x2.dtype, w.dtype
         if rw is not None:
             loss = (nll * rw).sum()
         else:
@@ -449,12 +498,31 @@ class _LmHeadLossFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dloss, _dnll):
-        dx = ctx.dx.view(ctx.shp) * dloss.to(ctx.dx.dtype)
-        gw = ctx.own_gw.to(ctx.wdtype) * dloss.to(ctx.wdtype) if ctx.own_gw is not None else None
+        dx = _scale_cast(ctx.dx, dloss, ctx.xdtype).view(ctx.shp)
+        gw = _scale_cast(ctx.own_gw, dloss, ctx.wdtype) if ctx.own_gw is not None else None
         return dx, gw, None, None, None, None, None, None, None, None
 
 
+@torch.no_grad()
+def _lmhead_nll(x, w, targets, vocab, cap):
+    """Per-row negative log-likelihoods (0 where the target is masked); the logits never leave the GEMM."""
+    x2 = _c(x).view(-1, x.shape[-1])
+    m = x2.shape[0]
+    tg = _c(targets).view(-1).to(torch.int64)
+    nll, z = torch.empty(m, dtype=torch.float32, device=x.device), torch.empty(m, dtype=torch.float32, device=x.device)
+    part = torch.empty(-(-w.shape[0] // 256) * 2, m, dtype=torch.float32, device=x.device)
+    null = L.ptr(None)
+    _logits_stats(x2, w, None, vocab, cap, part, tg, z)
+    L.call("bones_ce_finish", L.ptr(part), _I(part.shape[0]), _I(m), null, _L(0), L.ptr(z), L.ptr(tg), _I(vocab), _F(cap), L.ptr(nll), null, null, null,
+           _F(1.0), null, null, null, null, null, L.stream())
+    COUNTS["lmhead_loss"] += 1
+    return nll
+
+
 def lmhead_loss(x, w, targets, vocab, cap, reduction="mean", row_weights=None, loss_div=1.0, aux=None, label_smoothing=0.0):
+    if reduction != "mean" and not aux and label_smoothing == 0.0 and 0 < x.numel() and _logits_stats_ok(_c(x).view(-1, x.shape[-1]), w, vocab):
+        nll = _lmhead_nll(x, w, targets, vocab, cap)
+        return nll.sum() if reduction == "sum" else nll.view(targets.shape)
     want_grad = torch.is_grad_enabled() and (x.requires_grad or w.requires_grad) and reduction == "mean"
     loss, nll = _LmHeadLossFn.apply(x, w, targets, vocab, cap, float(loss_div), row_weights, want_grad, aux,
                                     float(label_smoothing))
