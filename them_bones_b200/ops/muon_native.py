@@ -8,6 +8,8 @@ launches per iteration with the ``alpha*acc + beta*R`` epilogue doing the polyno
 """
 from __future__ import annotations
 
+import ctypes
+
 import torch
 
 from ..ref.functional import POLAR_EXPRESS_COEFFS
@@ -24,6 +26,20 @@ def newton_schulz(x: torch.Tensor, steps: int = 5) -> torch.Tensor:
         return ns_ref(x, steps)
     tall = r > c
     n = c if tall else r
+    if r % 16 == 0 and c % 16 == 0 and x.data_ptr() % 32 == 0 and 0 < steps <= 8 and k and (k >= 4 or n <= 256):
+        # the whole iteration as one kernel over an ordered list of tiles (csrc/newton_schulz.cu), where there are matrices enough to
+        # run side by side or so little work that launches are what it costs: 5 x 5120 x 1280 751 -> 657 us, 10 x 1280 x 1280
+        # 660 -> 524, 20 x 1280 x 1280 1025 -> 841, 4 x 1280 x 1280 327 -> 312, 3 x 1024 x 256 232 -> 183.  One to three large
+        # matrices have nobody to hide a product's end behind (2 x 5120 x 1280: 405 us in launches, 536 in one kernel).
+        co = POLAR_EXPRESS_COEFFS[:steps]
+        bufs = [torch.empty_like(x), torch.empty_like(x) if len(co) > 1 else x]
+        gb = torch.empty(2, k, n, n, dtype=torch.bfloat16, device=x.device)
+        scratch = torch.empty(1 + 3 * len(co) * k, dtype=torch.int32, device=x.device)
+        flat = (ctypes.c_float * (3 * len(co)))(*[v for t in co for v in t])
+        L.call("bones_newton_schulz", L.ptr(x), L.ptr(bufs[0]), L.ptr(bufs[1]), L.ptr(gb[0]), L.ptr(gb[1]), ctypes.c_int(k), ctypes.c_int(r),
+               ctypes.c_int(c), ctypes.c_int(len(co)), flat, L.ptr(scratch), L.stream())
+        COUNTS["ns_gemm"] += 3 * len(co)
+        return bufs[0] if len(co) % 2 else bufs[1]
     g = torch.empty(k, n, n, dtype=torch.bfloat16, device=x.device)
     b = torch.empty_like(g)
     cur, nxt = x, torch.empty_like(x)
@@ -53,7 +69,6 @@ def muon_finish(g, w, second, *, beta2, lr, wd):
     owner's fp32 master ``w [k, r, c]`` (reference: round2/source/train.py:11890-11905).  Two native passes over the
     stack (``csrc/muon.cu``: line statistics, update); the arithmetic on the ``k * r`` or ``k * c`` line values between
     them is PyTorch."""
-    import ctypes
     k, r, c = g.shape
     lr_eff = lr * max(1.0, r / c) ** 0.5
     by_row = r >= c
