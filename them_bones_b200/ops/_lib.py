@@ -30,6 +30,9 @@ SIGNATURES = {
     "bones_gemm_bf16": _GEMM + [_I] * 3 + [_P],                     # ..., force_bn, splits, atomic, stream
     "bones_gemm_bf16_pair": _GEMM + [_I] * 2 + [_P],
     "bones_gemm_bf16_auto": _GEMM + [_I] * 2 + [_P],
+    "bones_attention_fwd": [_P] * 8 + [_I] * 4 + [_F, _I, _P],
+    "bones_attention_bwd": [_P] * 12 + [_I] * 4 + [_F, _I, _P],
+    "bones_mx2_quant": [_P, _L, _P, _P, _I, _P, _P, _I, _L, _L, _I, _P],
     "bones_gemm_mxfp8_pair": [_P] * 8 + [_I] + [_P] * 2 + [_I] * 5 + [_L] * 8 + [_I] * 3 + [_F] * 2 + [_I] * 3 + [_P],
 }
 
@@ -55,13 +58,18 @@ def available() -> bool:
         return False
 
 
+def raw_stream() -> int:
+    """The current stream's handle as a number, for the entry points of ``SIGNATURES``."""
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+
+
 def ptr(t):
     return ctypes.c_void_p(0 if t is None else t.data_ptr())
 
 
 def stream():
     """The current stream's handle, without building a ``torch.cuda.Stream`` object (4 us of a 10 us launch)."""
-    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+    return ctypes.c_void_p(raw_stream())
 
 
 LAUNCHES = [0]        # native kernel launches issued by this process (`launches`: an entry point with more than one kernel)
@@ -118,7 +126,7 @@ def gemm(a, b, d, *, m, n, k, lda, ldb, ldd, a_major=0, b_major=0, epi=EPI_BF16,
     # accumulation by vector atomics even without split-K, for outputs several GPUs add into at once
     dp = d.data_ptr() if d_ptr is None else int(d_ptr)
     rp = r.data_ptr() if r is not None else 0
-    st = torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
+    st = raw_stream()
     if auto or pair:
         call("bones_gemm_bf16_auto" if auto else "bones_gemm_bf16_pair", a.data_ptr(), b.data_ptr(), dp, rp, m, n, k, batch, lda, ldb, ldd, ldr,
              stride_a, stride_b, stride_d, stride_r, a_major, b_major, epi, alpha, beta, splits, int(atomic), st)

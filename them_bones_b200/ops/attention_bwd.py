@@ -32,9 +32,9 @@ def backward(dy, qkv2, qk, y, lse, cos, sin, ds, b, t, n_head, head_dim, scale, 
         stats = torch.empty(n + 2, dtype=torch.float32, device=dev)
         dqk = torch.empty(m, 2 * a, dtype=torch.bfloat16, device=dev)
         # dV goes straight into its third of dqkv, rows 3a apart
-        L.call("bones_attention_bwd", L.ptr(dy2), L.ptr(qkv2), L.ptr(qk), L.ptr(y), L.ptr(lse), L.ptr(cos), L.ptr(sin), L.ptr(ds), L.ptr(stats),
-               ctypes.c_void_p(stats.data_ptr() + 4 * n), L.ptr(dqk), L.ptr(dqkv), _I(b), _I(t), _I(n_head), _I(head_dim), _F(scale),
-               _I(window // 128), L.stream(), launches=4)
+        L.call("bones_attention_bwd", dy2.data_ptr(), qkv2.data_ptr(), qk.data_ptr(), y.data_ptr(), lse.data_ptr(), cos.data_ptr(), sin.data_ptr(),
+               0 if ds is None else ds.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * n, dqk.data_ptr(), dqkv.data_ptr(), b, t, n_head, head_dim,
+               scale, window // 128, L.raw_stream(), launches=4)
         return dqkv
     delta = torch.empty(b, n_head, t, dtype=torch.float32, device=dev)
     L.call("bones_attn_delta", L.ptr(dy2), L.ptr(y), L.ptr(delta), _L(m), _I(t), _I(n_head), L.stream())

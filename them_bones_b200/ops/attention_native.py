@@ -41,7 +41,7 @@ def _lse_buffer(b, t, n_head, dev):
     """The log-sum-exp rows ``[b, n_head, t]`` and, behind them, the int the forward kernel draws its work items from."""
     n = b * n_head * t
     buf = torch.empty(n + 1, dtype=torch.float32, device=dev)
-    return buf, ctypes.c_void_p(buf.data_ptr() + 4 * n)
+    return buf, buf.data_ptr() + 4 * n
 
 
 def rope_qknorm(qkv2, cos, sin, t, n_head, head_dim):
@@ -82,8 +82,8 @@ class _AttnFn(torch.autograd.Function):
         qk = torch.empty(b * t, 2 * a, dtype=qkv2.dtype, device=dev)
         y = torch.empty(b, t, a, dtype=qkv2.dtype, device=dev)
         lse, counter = _lse_buffer(b, t, n_head, dev)
-        L.call("bones_attention_fwd", L.ptr(qkv2), L.ptr(cos), L.ptr(sin), L.ptr(qk), L.ptr(y), L.ptr(lse), L.ptr(ds), counter, _I(b), _I(t),
-               _I(n_head), _I(head_dim), _F(scale), _I(window // 128), L.stream(), launches=2)
+        L.call("bones_attention_fwd", qkv2.data_ptr(), cos.data_ptr(), sin.data_ptr(), qk.data_ptr(), y.data_ptr(), lse.data_ptr(),
+               0 if ds is None else ds.data_ptr(), counter, b, t, n_head, head_dim, scale, window // 128, L.raw_stream(), launches=2)
         ctx.save_for_backward(qkv2, qk, y, lse, cos, sin, ds)
         ctx.meta = (b, t, n_head, head_dim, scale, window)
         return y

@@ -77,8 +77,8 @@ def quant2(x2: torch.Tensor, *, row: bool = True, col: bool = False, group_r: in
     if col:
         qc = torch.empty(*lead, r, c, dtype=torch.uint8, device=dev)
         sfc = _sf_buf(c, r, group_c, dev, lead)
-    L.call("bones_mx2_quant", L.ptr(x2), _L(x2.stride(-2)), L.ptr(qr), L.ptr(sfr), _I(group_r), L.ptr(qc), L.ptr(sfc), _I(group_c),
-           _L(r), _L(c), _I(lead[0] if lead else 1), L.stream())
+    qp = [0 if t is None else t.data_ptr() for t in (qr, sfr, qc, sfc)]
+    L.call("bones_mx2_quant", x2.data_ptr(), x2.stride(-2), qp[0], qp[1], group_r, qp[2], qp[3], group_c, r, c, lead[0] if lead else 1, L.raw_stream())
     COUNTS["mx_quant"] += 1
     return qr, sfr, qc, sfc
 
@@ -136,7 +136,7 @@ def gemm2(aq, sfa, bq, sfb, m, n, k, *, a_major=0, b_major=0, epi=GE_BF16, r=Non
     ldr = r.stride(-2) if r is not None else 0
     dp = [0 if t is None else t.data_ptr() for t in (aq, sfa, bq, sfb, d, r, dq, dsf, dt, dtsf)]
     L.call("bones_gemm_mxfp8_pair", *dp[:8], dq_group, *dp[8:], dt_group, m, n, k, batch, lda, ldb, ldd, ldr, sa, sb, sd, sr, a_major, b_major, epi,
-           alpha, beta, bn, splits, 0, torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice()))
+           alpha, beta, bn, splits, 0, L.raw_stream())
     COUNTS["mx_gemm"] += 1
     return d, dq, dsf, dt, dtsf
 
