@@ -1,0 +1,33 @@
+"""The MoE combine and its gradient by slot, against the PyTorch statement: dropped assignments, empty slots, residual."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n,k,e,cap,c,with_res,with_tok", [(1, 1, 2, 1, 8, False, True), (65, 2, 4, 20, 264, True, True), (300, 2, 16, 30, 1280, True, False),
+                                                           (128, 3, 5, 128, 512, False, True)])
+def test_combine_matches_statement(n, k, e, cap, c, with_res, with_tok):
+    from them_bones_b200 import ops
+    from them_bones_b200.ref import functional as RF
+    g = torch.Generator(device="cuda").manual_seed(n)
+    idx = torch.rand(n, e, generator=g, device="cuda").topk(k, dim=1).indices
+    slot, tok = RF.moe_slots(idx, 1, n, e, cap)
+    rnd = lambda *s: torch.randn(*s, generator=g, device="cuda").bfloat16()  # noqa: E731
+    ys, res, dout = rnd(e * cap, c), rnd(n, c), rnd(n, c)
+    gates = torch.rand(n, k, generator=g, device="cuda")
+    ys.requires_grad_(True), gates.requires_grad_(True), res.requires_grad_(True)
+    out = ops.moe_combine(ys, slot, gates, res if with_res else None, tok if with_tok else None)
+    ins = [ys, gates] + ([res] if with_res else [])
+    got = torch.autograd.grad(out, ins, dout)
+    y64, g64 = ys.detach().double().requires_grad_(True), gates.detach().double().requires_grad_(True)
+    yp = torch.cat([y64, y64.new_zeros(1, c)])
+    want = (g64[..., None] * yp[slot]).sum(1)
+    dy, dg = torch.autograd.grad(want, [y64, g64], dout.double())
+    want = want.detach() + (res.detach().double() if with_res else 0)
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm().clamp_min(1e-30))  # noqa: E731
+    assert rel(out, want) < 6e-3               # one or two bf16 roundings
+    assert rel(got[0], dy) < 4e-3 and rel(got[1], dg) < 1e-5
+    assert bool((got[0][tok == n] == 0).all()) and bool((got[1][slot == e * cap] == 0).all())
+    if with_res:
+        assert torch.equal(got[2], dout)

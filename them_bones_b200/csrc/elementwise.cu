@@ -354,28 +354,52 @@ __global__ void scatter_add_rows_kernel(const __nv_bfloat16* dy, const IdxT* idx
 }
 
 // out[n] = sum_k gates[n,k] * ys[slot[n,k]]   (slot == S: dropped)
-__global__ void moe_combine_kernel(const __nv_bfloat16* ys, const long long* slot, const float* gates, __nv_bfloat16* out, int n, int C,
-                                   int topk, long long S) {
+// gates null: all one.  residual: added to the combined row after its rounding, as a separate addition would.  A token's slots and
+// gates are read once and four column groups are in flight together (16384 x 1280 from two slots each, forward with the residual
+// and the dispatch gradient: 54 us; 60 and 20 for the addition before).
+template <int K>
+__global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const long long* __restrict__ slot, const float* __restrict__ gates,
+                                   const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out, int n, int C, int topk, long long S) {
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= n) return;
+  const __nv_bfloat16* src[K];
+  float g[K];
+#pragma unroll
+  for (int k = 0; k < K; ++k) {                // K: topk rounded up to 1, 2 or 8
+    const long long s = k < topk ? slot[(size_t)row * topk + k] : -1;
+    const bool live = s >= 0 && s < S;
+    src[k] = live ? ys + (size_t)s * C : nullptr;
+    g[k] = live ? (gates ? gates[(size_t)row * topk + k] : 1.0f) : 0.f;
+  }
+#pragma unroll 4
   for (int c = lane * 8; c < C; c += 256) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int k = 0; k < topk; ++k) {
-      const long long s = slot[(size_t)row * topk + k];
-      if (s < 0 || s >= S) continue;
-      const float g = gates[(size_t)row * topk + k];
-      const uint4 u = *reinterpret_cast<const uint4*>(ys + (size_t)s * C + c);
+#pragma unroll
+    for (int k = 0; k < K; ++k) {
+      if (!src[k]) continue;
+      const uint4 u = *reinterpret_cast<const uint4*>(src[k] + c);
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const float2 f = unpack_bf16(w[t]);
-        acc[2 * t] += g * f.x;
-        acc[2 * t + 1] += g * f.y;
+        acc[2 * t] += g[k] * f.x;
+        acc[2 * t + 1] += g[k] * f.y;
       }
     }
     uint4 o;
     o.x = pack_bf16(acc[0], acc[1]); o.y = pack_bf16(acc[2], acc[3]);
     o.z = pack_bf16(acc[4], acc[5]); o.w = pack_bf16(acc[6], acc[7]);
+    if (residual) {
+      const uint4 r = *reinterpret_cast<const uint4*>(residual + (size_t)row * C + c);
+      const uint32_t a4[4] = {o.x, o.y, o.z, o.w}, r4[4] = {r.x, r.y, r.z, r.w};
+      uint32_t q[4];
+#pragma unroll
+      for (int t = 0; t < 4; ++t) {
+        const float2 f = unpack_bf16(a4[t]), h = unpack_bf16(r4[t]);
+        q[t] = pack_bf16(f.x + h.x, f.y + h.y);
+      }
+      o = make_uint4(q[0], q[1], q[2], q[3]);
+    }
     *reinterpret_cast<uint4*>(out + (size_t)row * C + c) = o;
   }
 }
@@ -437,35 +461,44 @@ __global__ void moe_slots_kernel(const long long* __restrict__ idx, long long* _
   }
 }
 
-// Backward of the gate-weighted combine: dys[slot[n,k]] = gates[n,k] * dout[n] (slots are unique; empty slots stay at
-// the zero the caller wrote) and dgates[n,k] = <ys[slot[n,k]], dout[n]>.  One warp per token.
+// Backward of the gate-weighted combine, by slot: dys[s] = gates[n,k] * dout[n] for the assignment (n, k) whose slot is s
+// (token_of_slot[s] = n; zero rows for empty slots) and dgates[n,k] = <ys[s], dout[n]> (a dropped assignment's stays as the caller
+// wrote it: zero).  One warp per slot: every row of dys is written once, without a zero fill before (105 MB, 16 us, for 40960
+// slots of 1280).
 __global__ void moe_combine_bwd_kernel(const __nv_bfloat16* __restrict__ ys, const long long* __restrict__ slot, const float* __restrict__ gates,
-                                       const __nv_bfloat16* __restrict__ dout, __nv_bfloat16* __restrict__ dys, float* __restrict__ dgates,
-                                       int n, int C, int topk, long long S) {
-  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
-  if (row >= n) return;
-  for (int kk = 0; kk < topk; ++kk) {
-    const long long s = slot[(size_t)row * topk + kk];
-    float acc = 0.f;
-    if (s >= 0 && s < S) {
-      const float g = gates[(size_t)row * topk + kk];
-      for (int c = lane * 8; c < C; c += 256) {
-        const uint4 uy = *reinterpret_cast<const uint4*>(ys + (size_t)s * C + c);
-        const uint4 ud = *reinterpret_cast<const uint4*>(dout + (size_t)row * C + c);
-        const uint32_t wy[4] = {uy.x, uy.y, uy.z, uy.w}, wd[4] = {ud.x, ud.y, ud.z, ud.w};
-        uint32_t o[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const float2 fy = unpack_bf16(wy[i]), fd = unpack_bf16(wd[i]);
-          acc += fy.x * fd.x + fy.y * fd.y;
-          o[i] = pack_bf16(g * fd.x, g * fd.y);
-        }
-        *reinterpret_cast<uint4*>(dys + (size_t)s * C + c) = make_uint4(o[0], o[1], o[2], o[3]);
-      }
-    }
-    acc = warp_sum(acc);
-    if (lane == 0) dgates[(size_t)row * topk + kk] = acc;
+                                       const long long* __restrict__ token_of_slot, const __nv_bfloat16* __restrict__ dout,
+                                       __nv_bfloat16* __restrict__ dys, float* __restrict__ dgates, int n, int C, int topk, long long S) {
+  const long long s = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const int lane = threadIdx.x & 31;
+  if (s >= S) return;
+  const long long tok = token_of_slot[s];
+  int kk = -1;
+  if (tok >= 0 && tok < n)
+    for (int k = 0; k < topk; ++k)
+      if (slot[tok * topk + k] == s) kk = k;
+  __nv_bfloat16* dst = dys + (size_t)s * C;
+  if (kk < 0) {
+    for (int c = lane * 8; c < C; c += 256) *reinterpret_cast<uint4*>(dst + c) = make_uint4(0u, 0u, 0u, 0u);
+    return;
   }
+  const float g = gates[tok * topk + kk];
+  float acc = 0.f;
+#pragma unroll 4
+  for (int c = lane * 8; c < C; c += 256) {
+    const uint4 uy = *reinterpret_cast<const uint4*>(ys + (size_t)s * C + c);
+    const uint4 ud = *reinterpret_cast<const uint4*>(dout + (size_t)tok * C + c);
+    const uint32_t wy[4] = {uy.x, uy.y, uy.z, uy.w}, wd[4] = {ud.x, ud.y, ud.z, ud.w};
+    uint32_t o[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 fy = unpack_bf16(wy[i]), fd = unpack_bf16(wd[i]);
+      acc += fy.x * fd.x + fy.y * fd.y;
+      o[i] = pack_bf16(g * fd.x, g * fd.y);
+    }
+    *reinterpret_cast<uint4*>(dst + c) = make_uint4(o[0], o[1], o[2], o[3]);
+  }
+  acc = warp_sum(acc);
+  if (lane == 0) dgates[tok * topk + kk] = acc;
 }
 
 // Up to two auxiliary targets per row (multi-token prediction: the tokens two and three positions ahead) share the
@@ -937,9 +970,18 @@ int bones_scatter_add_rows(const void* dy, const void* idx, int idx_is_64, float
     scatter_add_rows_kernel<int><<<ROW_GRID(n), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)dy, (const int*)idx, grad, n, C, n_rows);
   return (int)cudaGetLastError();
 }
-int bones_moe_combine(const void* ys, const long long* slot, const float* gates, void* out, int n, int C, int topk, long long S, void* stream) {
-  if (C % 8) return -2;
-  moe_combine_kernel<<<ROW_GRID(n), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)ys, slot, gates, (__nv_bfloat16*)out, n, C, topk, S);
+// gates, residual: null for all ones, none.  ys, out and residual 16-byte aligned
+int bones_moe_combine(const void* ys, const long long* slot, const float* gates, const void* residual, void* out, int n, int C, int topk, long long S,
+                      void* stream) {
+  if ((C % 8) || topk < 1 || topk > 8) return -2;
+  if (n <= 0) return 0;
+#define BONES_COMBINE(K)                                                                                                                  \
+  moe_combine_kernel<K><<<ROW_GRID(n), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)ys, slot, gates, (const __nv_bfloat16*)residual, \
+                                                                  (__nv_bfloat16*)out, n, C, topk, S)
+  if (topk == 1) BONES_COMBINE(1);
+  else if (topk == 2) BONES_COMBINE(2);
+  else BONES_COMBINE(8);
+#undef BONES_COMBINE
   return (int)cudaGetLastError();
 }
 int bones_moe_slots(const long long* idx, long long* slot, long long* tok, int b, int t, int k, int n_exp, int cap, void* stream) {
@@ -947,10 +989,12 @@ int bones_moe_slots(const long long* idx, long long* slot, long long* tok, int b
   moe_slots_kernel<<<b, kSlotThreads, 0, (cudaStream_t)stream>>>(idx, slot, tok, b, t, k, n_exp, cap);
   return (int)cudaGetLastError();
 }
-int bones_moe_combine_bwd(const void* ys, const long long* slot, const float* gates, const void* dout, void* dys, float* dgates, int n, int C,
-                          int topk, long long S, void* stream) {
+// dys [S, C] is written whole; dgates [n, topk] zero before the call
+int bones_moe_combine_bwd(const void* ys, const long long* slot, const float* gates, const long long* token_of_slot, const void* dout, void* dys,
+                          float* dgates, int n, int C, int topk, long long S, void* stream) {
   if (C % 8) return -2;
-  moe_combine_bwd_kernel<<<ROW_GRID(n), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)ys, slot, gates, (const __nv_bfloat16*)dout,
+  if (S <= 0) return 0;
+  moe_combine_bwd_kernel<<<ROW_GRID(S), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)ys, slot, gates, token_of_slot, (const __nv_bfloat16*)dout,
                                                                  (__nv_bfloat16*)dys, dgates, n, C, topk, S);
   return (int)cudaGetLastError();
 }

@@ -117,11 +117,12 @@ class MoeMLP(nn.Module):
         xs = ops.moe_dispatch_exchange(h, tok, self.ep_group, self.ep_world, self.n_exp, slot, key=self.layer)
         ys = ops.moe_experts(xs, self.w_fc, self.w_proj, self.precision)   # rows grouped by local expert
         ys = ops.moe_exchange(ys, self.ep_group, self.ep_world, self.n_exp, forward=False, key=self.layer)
-        out = ops.moe_combine(ys, slot, gates)                            # [n, d]
+        fold = residual is not None and self.shared is None               # the residual joins in the combine kernel
+        out = ops.moe_combine(ys, slot, gates, residual.reshape(n, d) if fold else None, tok)      # [n, d]
         if self.shared is not None:
             out = out + ops.mlp(h, self.shared.c_fc.weight, self.shared.c_proj.weight, precision=self.precision)
         out = out.view(b, t, d)
-        if residual is not None:
+        if residual is not None and not fold:
             out = out + residual
         if moe_aux is not None:
             kept = (slot < self.n_exp * b * cap).float().mean()

@@ -290,15 +290,16 @@ def moe_dispatch(h, tok, slot=None):
     return hp.index_select(0, tok)
 
 
-def moe_combine(ys, slot, gates):
-    """``out[n] = sum_k gates[n,k] * ys[slot[n,k]]`` with dropped assignments (slot == S) contributing zero."""
+def moe_combine(ys, slot, gates, residual=None, tok=None):
+    """``out[n] = sum_k gates[n,k] * ys[slot[n,k]] (+ residual[n])`` with dropped assignments (slot == S) contributing zero.
+    ``tok``: the token in each slot (``moe_slots``), which the native backward otherwise derives from ``slot``."""
     if native(ys):
-        return _cuda().moe_combine(ys, slot, gates)
+        return _cuda().moe_combine(ys, slot, gates, residual, tok)
     yp = torch.cat([ys, ys.new_zeros(1, ys.shape[1])])
     out = 0
     for k in range(slot.shape[1]):
         out = out + gates[:, k:k + 1].to(ys.dtype) * yp.index_select(0, slot[:, k])
-    return out
+    return out if residual is None else out + residual
 
 
 def moe_dispatch_exchange(h, tok, group, world, n_exp, slot=None, key=None):

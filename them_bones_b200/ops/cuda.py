@@ -779,9 +779,8 @@ class _DispatchFn(torch.autograd.Function):
         tok, slot = ctx.saved_tensors
         dxs = _c(dxs)
         if ctx.has_slot:
-            ones = torch.ones(slot.shape, dtype=torch.float32, device=dxs.device)
             dh = torch.empty(ctx.n, dxs.shape[1], dtype=dxs.dtype, device=dxs.device)
-            L.call("bones_moe_combine", L.ptr(dxs), L.ptr(slot), L.ptr(ones), L.ptr(dh), _I(ctx.n), _I(dxs.shape[1]),
+            L.call("bones_moe_combine", L.ptr(dxs), L.ptr(slot), L.ptr(None), L.ptr(None), L.ptr(dh), _I(ctx.n), _I(dxs.shape[1]),
                    _I(slot.shape[1]), _L(dxs.shape[0]), L.stream())
             return dh, None, None
         g = torch.zeros(ctx.n, dxs.shape[1], dtype=torch.float32, device=dxs.device)
@@ -796,29 +795,37 @@ def moe_dispatch(h, tok, slot=None):
 
 class _CombineFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, ys, slot, gates):
+    def forward(ctx, ys, slot, gates, residual, tok):
         n, k = slot.shape
         out = torch.empty(n, ys.shape[1], dtype=ys.dtype, device=ys.device)
         g32 = _c(gates.float())
-        L.call("bones_moe_combine", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(out), _I(n), _I(ys.shape[1]), _I(k),
+        L.call("bones_moe_combine", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(residual), L.ptr(out), _I(n), _I(ys.shape[1]), _I(k),
                _L(ys.shape[0]), L.stream())
-        ctx.save_for_backward(ys, slot, g32)
+        ctx.save_for_backward(ys, slot, g32, tok)
+        ctx.has_res = residual is not None
         COUNTS["moe_combine"] += 1
         return out
 
     @staticmethod
     def backward(ctx, dout):
-        ys, slot, g32 = ctx.saved_tensors
+        ys, slot, g32, tok = ctx.saved_tensors
         dout = _c(dout)
-        dys = torch.zeros_like(ys)
-        dg = torch.empty_like(g32)
-        L.call("bones_moe_combine_bwd", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(dout), L.ptr(dys), L.ptr(dg), _I(slot.shape[0]),
+        if tok is None:              # the token in each slot, where the caller did not have it
+            n_slots = ys.shape[0]
+            s = torch.where((slot < 0) | (slot > n_slots), n_slots, slot).view(-1)
+            tok = torch.full((n_slots + 1,), slot.shape[0], dtype=torch.int64, device=ys.device)
+            tok.scatter_(0, s, torch.arange(slot.shape[0], device=ys.device).repeat_interleave(slot.shape[1]))
+        dys = torch.empty_like(ys)
+        dg = torch.zeros_like(g32)
+        L.call("bones_moe_combine_bwd", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(tok), L.ptr(dout), L.ptr(dys), L.ptr(dg), _I(slot.shape[0]),
                _I(ys.shape[1]), _I(slot.shape[1]), _L(ys.shape[0]), L.stream())
-        return dys, None, dg
+        return dys, None, dg, (dout if ctx.has_res else None), None
 
 
-def moe_combine(ys, slot, gates):
-    return _CombineFn.apply(_c(ys), _c(slot), gates)
+def moe_combine(ys, slot, gates, residual=None, tok=None):
+    if residual is not None and (residual.dtype != ys.dtype or residual.data_ptr() % 16):
+        return _CombineFn.apply(_c(ys), _c(slot), gates, None, tok) + residual
+    return _CombineFn.apply(_c(ys), _c(slot), gates, _c(residual) if residual is not None else None, tok)
 
 
 class _ExpertsFn(torch.autograd.Function):

@@ -437,10 +437,8 @@ class _PeerDispatch(torch.autograd.Function):
         ex, world, m, d = ctx.ex, ctx.world, ctx.m, g.shape[-1]
         dxs = ex._blocks(g.reshape(-1, d), world, m, 1, "gdisp")            # gradients of my slots, [E * rows, d]
         if ctx.has_slot:            # every token sums its (at most k) slots: the combine kernel with unit gates
-            from ..ops import cuda as C
-            ones = torch.ones(slot.shape, dtype=torch.float32, device=g.device)
             dh = torch.empty(ctx.n, d, dtype=g.dtype, device=g.device)
-            L.call("bones_moe_combine", L.ptr(dxs), L.ptr(slot), L.ptr(ones), L.ptr(dh), _I(ctx.n), _I(d), _I(slot.shape[1]),
+            L.call("bones_moe_combine", L.ptr(dxs), L.ptr(slot), L.ptr(None), L.ptr(None), L.ptr(dh), _I(ctx.n), _I(d), _I(slot.shape[1]),
                    _L(dxs.shape[0]), L.stream())
             return dh, None, None, None, None, None, None
         dh = torch.zeros(ctx.n + 1, d, dtype=torch.float32, device=g.device)
