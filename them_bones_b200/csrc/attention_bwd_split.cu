@@ -50,6 +50,8 @@ struct SplitParams {
   const int* doc_start;
   const float2* stats;   // [B, H, Tp]: (-lse * log2(e), delta); (-inf, 0) past T, so that the queries there have P = 0
   __nv_bfloat16* dqk;    // [B*T, 2A]: dq-hat | dk-hat
+  __nv_bfloat16* ds;     // dS^T of every tile pair, [slot][16 strips of 8 queries][128 keys][8], for the dQ kernel that reads it; or null
+  int slots;             // tile pairs of a (sequence, head) in that buffer
   __nv_bfloat16* dv;     // rows of dv_ld elements
   long long dv_ld;
   int* err;
@@ -58,9 +60,18 @@ struct SplitParams {
 
 __device__ __forceinline__ int split_first_tile(const SplitParams& p, int b, int qt) {
   int lo = 0;
-  if (p.doc_start) lo = p.doc_start[(long long)b * p.T + qt * ST] / ST;
+  if (p.doc_start) lo = min(max(p.doc_start[(long long)b * p.T + qt * ST] / ST, 0), qt);
   if (p.window_tiles > 0) lo = max(lo, qt - p.window_tiles + 1);
   return lo;
+}
+// Where the tile pair (query tile qt, key tile kt) of a (sequence, head) stands in the buffer of dS^T: the query tiles one after
+// another, each with the key tiles that causality and the band allow (those of earlier documents are neither written nor read).
+__host__ __device__ __forceinline__ int ds_before(int qt, int w) {        // slots of the query tiles before qt; w: window_tiles
+  return w <= 0 || qt <= w ? qt * (qt + 1) / 2 : w * (w + 1) / 2 + (qt - w) * w;
+}
+__device__ __forceinline__ long long ds_slot(const SplitParams& p, int b, int h, int qt, int kt) {
+  const int first = p.window_tiles > 0 ? max(0, qt - p.window_tiles + 1) : 0;
+  return ((long long)b * p.H + h) * p.slots + ds_before(qt, p.window_tiles) + kt - first;
 }
 // Descriptors are the tile's base descriptor plus a compile-time step in the address field (16-byte units; shared-memory
 // addresses stay below 2^18, so the field never carries): one 64-bit add per operand and MMA in the issuing loop instead
@@ -185,12 +196,18 @@ __device__ __forceinline__ DkvItem dkv_item(const SplitParams& p, int w, int n_t
   it.kt = w % n_tiles;                                // longest walks (small kt) of a (head, batch) first
   it.h = grp % p.H;
   it.b = grp / p.H;
-  int n = 0;
-  for (int qt = it.kt; qt < n_tiles; ++qt) {          // the query tiles that see this key tile
-    if (split_first_tile(p, it.b, qt) > it.kt) break;
-    ++n;
+  // Up to the last query tile that sees this key tile: every pair that a dQ item reads (it takes all key tiles from its first one
+  // on) is walked here, whatever the document starts are.  The lanes of the (whole) warp look at 32 tiles at a time.
+  const int cap = p.window_tiles > 0 ? min(n_tiles - it.kt, p.window_tiles) : n_tiles - it.kt;
+  it.n = cap;
+  if (p.doc_start) {
+    it.n = 1;                                         // a key tile is always seen by its own query tile
+    for (int c = 1; c < cap; c += 32) {
+      const int i = c + (int)(threadIdx.x & 31);
+      const uint32_t sees = __ballot_sync(0xffffffffu, i < cap && split_first_tile(p, it.b, it.kt + i) <= it.kt);
+      if (sees) it.n = c + 32 - __clz(sees);
+    }
   }
-  it.n = n;                                           // >= 1: a key tile is always seen by its own query tile
   return it;
 }
 
@@ -474,10 +491,21 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_cons
             pr[2 * j + 1] *= (__uint_as_float(v0[2 * j + 1]) - a.w) * p.scale;
           }
         }
-        store_packed32(tdP + lane_addr + (uint32_t)c0, pr);
+        uint32_t pk[16];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) pk[j] = pack_bf16(pr[2 * j], pr[2 * j + 1]);
+        BONES_TMEM_ST16(tdP + lane_addr + (uint32_t)c0, pk);
+        tmem_st_wait();
         tc_fence_before();
         __syncwarp();
         if (lane == 0) mbar_arrive(bar(B_DSREADY));
+        // behind the hand-over: four strips of 8 queries, where the 32 key rows of a warp are neighbours (512 B contiguous a
+        // store; as rows of 128 queries, 32 lines a store, this cost 44 us of 287)
+        if (p.ds) {
+          uint4* dst = reinterpret_cast<uint4*>(p.ds + ds_slot(p, im.b, im.h, im.kt + i, im.kt) * 16384) + part * 4 * 128 + r;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) dst[j * 128] = make_uint4(pk[4 * j], pk[4 * j + 1], pk[4 * j + 2], pk[4 * j + 3]);
+        }
         APROF_ADD(4);
       }
       if (!ok) break;
@@ -774,6 +802,168 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_const
   }
 }
 
+// ---------------------------------------------------------------------------------------------------------------
+// dQ from stored dS: dQ = sum over key tiles of dS Kh, with dS^T as the dK / dV kernel left it (bf16, what its own MMAs consumed).
+// The kernel above computes S, the exponentials and dP a second time for this; a tile pair costs it 3 300 clocks, most of them
+// exponentials and TMEM traffic, where the dQ MMAs themselves take 512.  Reading 32 KB of dS^T per tile pair instead is bound by
+// memory.  16 x 2048 tokens, 10 heads (0.71 GB of dS): dQ 198 -> 101 us, 7.1 TB/s, for 288 -> 297 us of the dK / dV kernel that
+// stores it.
+// A tile's strips of 8 queries x 128 keys are the unswizzled MN-major operand layout as they stand (8 keys of a strip are one
+// 128-byte core matrix), so a tile arrives as one 32 KB bulk copy; Kh is an MN-major operand in the usual swizzled atoms.  (Rows of
+// 128 queries would load as swizzled boxes in 101 us, but cost the dK / dV kernel 44 us of scattered stores; strips of 16 with
+// copying warps that swizzle took 121.)  Warp 0: item draws and loads, warp 1: MMAs, eight epilogue warps; two accumulators, so an
+// item's drain hides behind the next one's MMAs.
+// ---------------------------------------------------------------------------------------------------------------
+constexpr int DQG_SA = 4, DQG_SB = 3, DQG_EW = 8, DQG_THREADS = 64 + 32 * DQG_EW;
+constexpr int DQG_NBARS = 2 * DQG_SA + 2 * DQG_SB + 12;
+__host__ __device__ constexpr uint32_t dqg_bars(int D) { return DQG_SA * 2 * SATOM + DQG_SB * (uint32_t)(D / 64) * SATOM; }
+
+template <int D>
+__global__ void __launch_bounds__(DQG_THREADS, 1)
+attn_bwd_dq_gemm_kernel(const __grid_constant__ CUtensorMap tm_qk, const SplitParams p) {
+  constexpr uint32_t KT = (D / 64) * SATOM, BARS = dqg_bars(D);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t raw = smem_u32(smem_raw), base = (raw + 1023u) & ~1023u;
+  uint8_t* gen = smem_raw + (base - raw);
+  auto sA = [&](int s) { return base + (uint32_t)s * 2 * SATOM; };
+  auto sB = [&](int s) { return base + DQG_SA * 2 * SATOM + (uint32_t)s * KT; };
+  const uint32_t bars = base + BARS;
+  auto a_full = [&](int s) { return bars + 8u * s; };
+  auto a_free = [&](int s) { return bars + 8u * (DQG_SA + s); };
+  auto b_full = [&](int s) { return bars + 8u * (2 * DQG_SA + s); };
+  auto b_free = [&](int s) { return bars + 8u * (2 * DQG_SA + DQG_SB + s); };
+  auto tfull = [&](int a) { return bars + 8u * (2 * DQG_SA + 2 * DQG_SB + a); };
+  auto tempty = [&](int a) { return bars + 8u * (2 * DQG_SA + 2 * DQG_SB + 2 + a); };
+  const uint32_t ring_bars = bars + 8u * (2 * DQG_SA + 2 * DQG_SB + 4), ring_free = ring_bars + 32u;
+  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + BARS + 8 * DQG_NBARS);
+  const uint32_t tmem_slot = bars + 8u * (DQG_NBARS + 2);
+  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + BARS + 8 * (DQG_NBARS + 2));
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + BARS + 8 * (DQG_NBARS + 2) + 8);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int A = p.H * D, n_tiles = p.Tp / ST, total = n_tiles * p.H * p.B;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < DQG_SA; ++s) {
+      mbar_init(a_full(s), 1);
+      mbar_init(a_free(s), 1);
+    }
+    for (int s = 0; s < DQG_SB; ++s) {
+      mbar_init(b_full(s), 1);
+      mbar_init(b_free(s), 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      mbar_init(tfull(a), 1);
+      mbar_init(tempty(a), DQG_EW);
+    }
+    for (int s = 0; s < 4; ++s) {
+      mbar_init(ring_bars + 8u * s, 1);
+      mbar_init(ring_free + 8u * s, DQG_EW + 1);
+    }
+    *abort_flag = 0;
+    fence_barrier_init();
+    tma_prefetch_desc(&tm_qk);
+  }
+  __syncthreads();
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 256);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = *tmem_slot_g;
+  auto take = [&](int it) {                    // a consumer takes item `it` and gives its ring slot back
+    const int w = warp_uniform(item_take(ring_bars, ring_slots, it, abort_flag, p.err));
+    if (lane == 0) mbar_arrive(ring_free + 8u * (it & 3));
+    return w;
+  };
+  if (warp == 0) {
+    int g = 0;
+    bool dead = false;
+    for (int it = 0;; ++it) {
+      if (it >= 4 && !dead) dead = !mbar_wait(ring_free + 8u * (it & 3), (uint32_t)(((it >> 2) - 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
+      int w = -1;
+      if (lane == 0 && !dead) w = item_publish(ring_bars, ring_slots, it, p.items, total);
+      w = warp_uniform(w);
+      if (w < 0) break;
+      DqItem im = dq_item(p, w, n_tiles);
+      im.kt0 = warp_uniform(im.kt0);
+      im.n = im.qt - im.kt0 + 1;
+      const __nv_bfloat16* ds = p.ds + ds_slot(p, im.b, im.h, im.qt, im.kt0) * 16384;
+      for (int j = 0; j < im.n; ++j, ++g) {
+        const int as = g % DQG_SA, s = g % DQG_SB;
+        if (g >= DQG_SA && !dead) dead = !mbar_wait(a_free(as), (uint32_t)((g / DQG_SA - 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
+        if (elect_one() && !dead) {
+          mbar_arrive_expect_tx(a_full(as), 2 * SATOM);
+          bulk_load(sA(as), ds + (long long)j * 16384, 2 * SATOM, a_full(as));
+        }
+        if (g >= DQG_SB && !dead) dead = !mbar_wait(b_free(s), (uint32_t)((g / DQG_SB - 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
+        if (elect_one() && !dead) {
+          mbar_arrive_expect_tx(b_full(s), KT);
+#pragma unroll
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sB(s) + c * SATOM, &tm_qk, b_full(s), A + im.h * D + c * 64, (im.kt0 + j) * ST, im.b);
+        }
+      }
+    }
+  } else if (warp == 1) {
+    const uint32_t idesc = umma_idesc_f16(128, D, 1, 1, 1);
+    int g = 0;
+    bool dead = false;
+    for (int it = 0;; ++it) {
+      const int w = dead ? -1 : take(it);
+      if (w < 0) break;
+      DqItem im = dq_item(p, w, n_tiles);
+      im.kt0 = warp_uniform(im.kt0);
+      im.n = im.qt - im.kt0 + 1;
+      const int acc = it & 1;
+      if (it >= 2 && !dead) dead = !mbar_wait(tempty(acc), (uint32_t)(((it - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
+      for (int j = 0; j < im.n; ++j, ++g) {
+        const int as = g % DQG_SA, bs = g % DQG_SB;
+        if (!dead) dead = !mbar_wait(b_full(bs), (uint32_t)((g / DQG_SB) & 1), abort_flag, p.err, ERR_WAIT_FULL);
+        if (!dead) dead = !mbar_wait(a_full(as), (uint32_t)((g / DQG_SA) & 1), abort_flag, p.err, ERR_WAIT_FULL);
+        tc_fence_after();
+        if (elect_one() && !dead) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)              // 16 keys a step: two core matrices of a strip
+            umma_f16(tmem + acc * 128, umma_smem_desc(sA(as), 128, 2048, kLayoutNone) + (uint64_t)((k * 256) >> 4), sdesc_mn(sB(bs), k), idesc,
+                     (j | k) ? 1u : 0u);
+          tc_commit(a_free(as));
+          tc_commit(b_free(bs));
+          if (j == im.n - 1) tc_commit(tfull(acc));
+        }
+      }
+    }
+  } else {
+    const int q = warp & 3, half = (warp - 2) >> 2;
+    for (int it = 0;; ++it) {
+      const int w = take(it);
+      if (w < 0) break;
+      const DqItem im = dq_item(p, w, n_tiles);
+      const int acc = it & 1, qpos = im.qt * ST + q * 32 + lane;
+      const bool got = mbar_wait(tfull(acc), (uint32_t)((it >> 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
+      if (!__all_sync(0xffffffffu, got)) break;
+      tc_fence_after();
+      __nv_bfloat16* dst = qpos < p.T ? p.dqk + ((long long)im.b * p.T + qpos) * 2 * A + (long long)im.h * D : nullptr;
+#pragma unroll
+      for (int c = 0; c < D / 2; c += 32) {
+        const int col = half * (D / 2) + c;
+        drain_row<32>(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * 128 + col), dst ? dst + col : nullptr);
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(tempty(acc));
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 200; ++i) __nanosleep(1000);
+  }
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem, 256);
+  }
+}
+
 // [B, T, cols] bf16 rows, boxes of 64 columns x 128 rows of one sequence; rows past T read as zeros
 static int tmap_rows_3d_s(CUtensorMap* out, const void* ptr, int B, int T, long long cols) {
   uint64_t dims[3] = {(uint64_t)cols, (uint64_t)T, (uint64_t)B};
@@ -798,7 +988,17 @@ static int launch_split(const CUtensorMap& tq, const CUtensorMap& tv, const CUte
   attn_bwd_dkv_kernel<D><<<grid, STHREADS, smem_dkv, s>>>(tq, tv, td, p);
   BONES_CHECK(cudaGetLastError());
   p.items = counters + 1;
-  attn_bwd_dq_kernel<D><<<grid, STHREADS, smem_dq, s>>>(tq, tv, td, p);
+  if (p.ds) {
+    constexpr size_t smem_g = (size_t)dqg_bars(D) + 8 * (DQG_NBARS + 2) + 16 + 1024;
+    static bool g_done = false;
+    if (!g_done) {
+      BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dq_gemm_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g));
+      g_done = true;
+    }
+    attn_bwd_dq_gemm_kernel<D><<<grid, DQG_THREADS, smem_g, s>>>(tq, p);
+  } else {
+    attn_bwd_dq_kernel<D><<<grid, STHREADS, smem_dq, s>>>(tq, tv, td, p);
+  }
   return (int)cudaGetLastError();
 }
 
@@ -824,8 +1024,9 @@ int bones_attn_bwd_stats(const void* dy, const void* y, const float* lse, void* 
 
 // qk: [B*T, 2A] rotated, normalised q | k;  qkv: [B*T, 3A] (values read in place);  dy: [B*T, A];  stats and counters from the
 // pre-pass.  Outputs (bf16, every element overwritten): dqk [B*T, 2A];  dv rows of dv_ld elements (e.g. the last third of dqkv).
+// ds: scratch, 32 KB for each of the B * H * ds_before(tiles, window_tiles) tile pairs, 32-byte aligned; or null: dQ computes S and dP again.
 int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const void* stats, int* counters, void* dqk, void* dv,
-                         long long dv_ld, const int* doc_start, int B, int T, int H, int D, float scale, int window_tiles, void* stream) {
+                         long long dv_ld, void* ds, const int* doc_start, int B, int T, int H, int D, float scale, int window_tiles, void* stream) {
   if (D != 128 && D != 64) return -2;
   if ((dv_ld % 16) || ((uintptr_t)dv & 31) || ((uintptr_t)dqk & 31) || ((uintptr_t)stats & 15) ||
       (doc_start && ((uintptr_t)doc_start & 15)))
@@ -849,6 +1050,9 @@ int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const 
   p.dqk = (__nv_bfloat16*)dqk;
   p.dv = (__nv_bfloat16*)dv;
   p.dv_ld = dv_ld;
+  p.ds = (__nv_bfloat16*)ds;
+  p.slots = ds_before(p.Tp / ST, window_tiles);
+  if (ds && (((uintptr_t)ds & 31) || (long long)B * H * p.slots >= (1LL << 31))) return -3;
   p.err = error_word();
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
@@ -859,12 +1063,12 @@ int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const 
 
 // The whole backward: statistics (which zeroes the counters), dK / dV and dQ, RoPE / QK-norm backward into dqkv [B*T, 3A].
 int bones_attention_bwd(const void* dy, const void* qkv, const void* qk, const void* y, const float* lse, const float* cosT, const float* sinT,
-                        const int* doc_start, void* stats, int* counters, void* dqk, void* dqkv, int B, int T, int H, int D, float scale,
+                        const int* doc_start, void* stats, int* counters, void* ds, void* dqk, void* dqkv, int B, int T, int H, int D, float scale,
                         int window_tiles, void* stream) {
   const long long A = (long long)H * D;
   int rc = bones_attn_bwd_stats(dy, y, lse, stats, counters, B, T, H, D, stream);
   if (rc) return rc;
-  rc = bones_attn_bwd_split(qk, qkv, dy, stats, counters, dqk, (__nv_bfloat16*)dqkv + 2 * A, 3 * A, doc_start, B, T, H, D, scale, window_tiles, stream);
+  rc = bones_attn_bwd_split(qk, qkv, dy, stats, counters, dqk, (__nv_bfloat16*)dqkv + 2 * A, 3 * A, ds, doc_start, B, T, H, D, scale, window_tiles, stream);
   if (rc) return rc;
   return bones_rope_qknorm_bwd_bf16(qkv, cosT, sinT, dqk, dqkv, (long long)B * T, T, H, D, stream);
 }

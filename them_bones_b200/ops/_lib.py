@@ -31,7 +31,7 @@ SIGNATURES = {
     "bones_gemm_bf16_pair": _GEMM + [_I] * 2 + [_P],
     "bones_gemm_bf16_auto": _GEMM + [_I] * 2 + [_P],
     "bones_attention_fwd": [_P] * 8 + [_I] * 4 + [_F, _I, _P],
-    "bones_attention_bwd": [_P] * 12 + [_I] * 4 + [_F, _I, _P],
+    "bones_attention_bwd": [_P] * 13 + [_I] * 4 + [_F, _I, _P],
     "bones_mx2_quant": [_P, _L, _P, _P, _I, _P, _P, _I, _L, _L, _I, _P],
     "bones_gemm_mxfp8_pair": [_P] * 8 + [_I] + [_P] * 2 + [_I] * 5 + [_L] * 8 + [_I] * 3 + [_F] * 2 + [_I] * 3 + [_P],
 }

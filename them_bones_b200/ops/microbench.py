@@ -127,7 +127,7 @@ def roles(a):
         def fn():
             counters.zero_()
             L.call("bones_attn_bwd_split", L.ptr(qk), L.ptr(qkv), L.ptr(dy), L.ptr(stats), L.ptr(counters), L.ptr(dqk), L.ptr(dv), LL(3 * ad),
-                   L.ptr(None), I(b), I(t), I(h), I(d), F(scale), I(0), L.stream())
+                   L.ptr(None), L.ptr(None), I(b), I(t), I(h), I(d), F(scale), I(0), L.stream())
 
         ms = timeit(fn, a.iters, a.warmup, not a.no_flush)
         lib.bones_attn_set_prof(ctypes.c_void_p(prof.data_ptr()))
