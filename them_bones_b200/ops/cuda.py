@@ -471,8 +471,8 @@ class _LmHeadLossFn(torch.autograd.Function):
                 ap = aux_ptrs(r0, r1)
                 _logits_stats(x2[r0:r1], w, lg, vocab, cap, part, None, None)
                 L.call("bones_ce_finish", L.ptr(part), _I(part.shape[0]), _I(r1 - r0), L.ptr(lg), _L(vp), L.ptr(None), L.ptr(tg[r0:r1]), _I(vocab),
-                       _F(cap), L.ptr(nll[r0:r1]), L.ptr(info), L.ptr(rw[r0:r1] if rw is not None else None), L.ptr(n_valid), _F(1.0 / loss_div), *ap,
-                       L.stream())
+                       _F(cap), L.ptr(nll[r0:r1]), L.ptr(info), L.ptr(rw[r0:r1] if rw is not None else None), L.ptr(n_valid), _F(1.0 / loss_div),
+                       *aux_ptrs(r0, r1), L.stream())
                 L.call("bones_ce_grad", L.ptr(lg), _L(vp), L.ptr(info), L.ptr(tg[r0:r1]), ap[0], ap[2], _I(vocab), _F(cap), _I(r1 - r0), L.stream())
             else:
                 mm_nt(x2[r0:r1], w, out=lg, epi=L.EPI_SOFTCAP, alpha=1.0 / cap, beta=cap)

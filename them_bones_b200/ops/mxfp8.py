@@ -134,8 +134,8 @@ def gemm2(aq, sfa, bq, sfb, m, n, k, *, a_major=0, b_major=0, epi=GE_BF16, r=Non
     ldd = d.stride(-2) if d is not None else 0
     sr = r.stride(0) if (r is not None and batch > 1) else 0
     ldr = r.stride(-2) if r is not None else 0
-    dp = [0 if t is None else t.data_ptr() for t in (aq, sfa, bq, sfb, d, r, dq, dsf, dt, dtsf)]
-    L.call("bones_gemm_mxfp8_pair", *dp[:8], dq_group, *dp[8:], dt_group, m, n, k, batch, lda, ldb, ldd, ldr, sa, sb, sd, sr, a_major, b_major, epi,
+    pa, psa, pb, psb, pd, pr, pq, pqs, pt, pts = [0 if t is None else t.data_ptr() for t in (aq, sfa, bq, sfb, d, r, dq, dsf, dt, dtsf)]
+    L.call("bones_gemm_mxfp8_pair", pa, psa, pb, psb, pd, pr, pq, pqs, dq_group, pt, pts, dt_group, m, n, k, batch, lda, ldb, ldd, ldr, sa, sb, sd, sr, a_major, b_major, epi,
            alpha, beta, bn, splits, 0, L.raw_stream())
     COUNTS["mx_gemm"] += 1
     return d, dq, dsf, dt, dtsf
