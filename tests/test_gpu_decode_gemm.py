@@ -9,7 +9,8 @@ I = ctypes.c_int
 
 
 @pytest.mark.parametrize("b,n,k,splits,epi", [(1, 128, 64, 1, 0), (16, 384, 1280, 4, 0), (17, 128, 576, 2, 1), (33, 256, 1280, 4, 2), (64, 1280, 5120, 8, 2),
-                                              (65, 256, 128, 2, 1), (128, 640, 1280, 8, 3), (64, 1024, 1280, 1, 3), (5, 256, 512, 4, 2), (32, 256, 640, 8, 0)])
+                                              (65, 256, 128, 2, 1), (128, 640, 1280, 8, 3), (64, 1024, 1280, 1, 3), (5, 256, 512, 4, 2), (32, 256, 640, 8, 0), (64, 256, 1280, 16, 2),
+                                              (37, 128, 1088, 16, 1), (3, 128, 1024, 16, 2), (9, 256, 640, 8, 0), (128, 128, 1024, 16, 2)])
 def test_projection_epilogues(b, n, k, splits, epi):
     from them_bones_b200.ops import _lib as L
     g = torch.Generator(device="cuda").manual_seed(b + n)

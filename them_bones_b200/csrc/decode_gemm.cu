@@ -12,11 +12,15 @@
 //   * RMSNorm has no gain, so it is one factor per sequence: norm(x) W^T = r (x W^T).  The epilogue that produces x leaves the
 //     squares' sums per 128-column tile, the epilogue that consumes it multiplies by r: no norm kernel, and x enters the MMA
 //     as it is instead of rounded once more;
-//   * launched with programmatic dependence: the weight tiles of the first stages are requested before the wait for the
-//     previous kernel (weights depend on nothing in the step), so their latency hides behind it.
+//   * launched with programmatic dependence, and every kernel lets its successor start as soon as it runs itself: the weight tiles
+//     of the first stages (weights depend on nothing in the step) and the cache rows of the attention are requested before the wait
+//     for the previous kernel, so their latency hides behind it.  Only that wait orders data: nothing is written, and nothing a
+//     kernel of this step writes is read, before it.
 // Warp 0 issues the TMA loads, warp 1 the MMAs, the others run the epilogue.
 //
-// One step of the 20-layer, 1280-wide model at batch 64: 103 kernels and 0.90 ms where 250 kernels took 1.41 ms.  What is left is
+// One step of the 20-layer, 1280-wide model at batch 64: 103 kernels and 0.81 ms where 250 kernels took 1.41 ms.  Of 0.90 ms before,
+// the earlier start took 0.01, the rows requested ahead (residual before the accumulator, cache rows into L2) and clusters of 16
+// for the ten-tile projections 0.07, two CTAs a tile for the others (rule in utils/decode.py) 0.02.  What is left is
 // a chain of latencies: per projection about 1.6 us from the previous kernel's end to this one's start, 1.5 to 4 us until
 // the accumulator is complete, 1.2 + 1 us for the exchange and its barrier, 0.7 to 1.3 us of epilogue.  Measured without gain:
 // bulk prefetches of the next projection's weights into L2 (the issuing warp stalls for 4 us, 1.6 % a step).
@@ -147,8 +151,19 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const uint32_t tmem = *tmem_slot_g;
   const int cols = NB / S, lc = 31 - __clz(cols);        // tokens this CTA finishes (a power of two), and how many of them exist
   const int mine = max(0, min(cols, p.b - rank * cols));
-  pdl_wait();
   pdl_launch();
+  pdl_wait();
+  // residual, x0 and mix factors of an epilogue thread's first four tokens, requested before the wait for the accumulator
+  __nv_bfloat16 rs[4], x0[4];
+  float ma = 0.f, mb = 0.f;
+  auto residual = [&](int c0) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const long long at = (long long)(rank * cols + min(c0 + i, mine - 1)) * p.N + n0 + (warp & 3) * 32 + lane;
+      rs[i] = p.res[at];
+      if (p.x0) x0[i] = p.x0[at];
+    }
+  };
 
   if (warp == 0) {
     bool dead = false;
@@ -182,6 +197,10 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   } else {
     // while the weights are on their way: the norm factors of this CTA's tokens
     const int q = warp & 3, nl = q * 32 + lane;
+    if (EPI == DEC_RES && ((warp - 2) >> 2) * 4 < mine) {
+      residual(((warp - 2) >> 2) * 4);
+      if (p.x0) { ma = *p.mix_a; mb = *p.mix_b; }
+    }
     {
       const int e = threadIdx.x - 64, t = rank * cols + e;
       if (e < cols) {
@@ -218,19 +237,11 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     // four tokens at a time
     const int q = warp & 3, nl = q * 32 + lane, warp_group = (warp - 2) >> 2;
     if (!*abort_flag) {
-      const float ma = EPI == DEC_RES && p.x0 ? *p.mix_a : 0.f, mb = EPI == DEC_RES && p.x0 ? *p.mix_b : 0.f;
 #pragma unroll 1
       for (int c0 = warp_group * 4; c0 < mine; c0 += DG_EW) {
         const long long at0 = (long long)(rank * cols + c0) * p.N + n0 + nl;
-        float v[4] = {0.f, 0.f, 0.f, 0.f}, rs[4], x0[4];
-        if (EPI == DEC_RES) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const long long at = at0 + (long long)min(i, mine - 1 - c0) * p.N;
-            rs[i] = __bfloat162float(p.res[at]);
-            x0[i] = p.x0 ? __bfloat162float(p.x0[at]) : 0.f;
-          }
-        }
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (EPI == DEC_RES && c0 != warp_group * 4) residual(c0);
 #pragma unroll 2
         for (int s = 0; s < S; ++s) {
           const float4 w = *reinterpret_cast<const float4*>(gen + ST * G::kStage + 16u * red_unit(s, nl, c0 >> 2, lc));
@@ -247,8 +258,8 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
             asm("tanh.approx.f32 %0, %1;" : "=f"(th) : "f"(y / p.cap));
             y = p.cap * th;
           } else if (EPI == DEC_RES) {
-            y = __bfloat162float(__float2bfloat16(y + rs[i]));
-            if (p.x0) y = ma * y + mb * x0[i];
+            y = __bfloat162float(__float2bfloat16(y + __bfloat162float(rs[i])));
+            if (p.x0) y = ma * y + mb * __bfloat162float(x0[i]);
           }
           const __nv_bfloat16 o = __float2bfloat16(y);
           if (c0 + i < mine) p.out[at0 + (long long)i * p.N] = o;
@@ -302,6 +313,7 @@ static int launch_dec_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const D
   static bool attr_done = false;
   if (!attr_done) {
     BONES_CHECK(cudaFuncSetAttribute(decode_gemm_kernel<NB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem));
+    BONES_CHECK(cudaFuncSetAttribute(decode_gemm_kernel<NB, EPI>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
     attr_done = true;
   }
   cudaLaunchConfig_t cfg = {};
@@ -312,6 +324,11 @@ static int launch_dec_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const D
   cfg.stream = stream;
   cfg.attrs = at;
   cfg.numAttrs = (unsigned)dec_launch_attrs(at, S, pdl);
+  if (S > 8) {                                 // more than the portable cluster size: a device may have no room for one
+    static int room = -1;
+    if (room < 0) BONES_CHECK(cudaOccupancyMaxActiveClusters(&room, decode_gemm_kernel<NB, EPI>, &cfg));
+    if (room == 0) return launch_dec_gemm<NB, EPI>(tw, tx, p, 8, pdl, stream);
+  }
   return (int)cudaLaunchKernelEx(&cfg, decode_gemm_kernel<NB, EPI>, tw, tx, p);
 }
 template <int NB>
@@ -340,6 +357,7 @@ __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
     f[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
+__device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
 __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
                                                                   const float* __restrict__ sinT, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
                                                                   const int* pos_ptr, const int* doc_start, __nv_bfloat16* __restrict__ y, int H,
@@ -347,12 +365,14 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
   __shared__ __align__(16) __nv_bfloat16 s_new[3][128];
   __shared__ __align__(16) float s_acc[8][128];
   __shared__ float s_l[8];
-  pdl_wait();
   pdl_launch();
   const int h = blockIdx.x, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l16 = lane & 15;
   const int pos = *pos_ptr;
-  if (pos < 0 || pos >= Tmax) return;
+  if (pos < 0 || pos >= Tmax) {
+    pdl_wait();
+    return;
+  }
   int lo = doc_start ? doc_start[b] : 0;
   if (window_tiles > 0) lo = max(lo, (pos / 128 - (window_tiles - 1)) * 128);
   lo = max(lo, 0);
@@ -367,6 +387,11 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
   };
   int j = lo + warp * 2 + (lane >> 4);
   fetch(j);
+  // the cache holds earlier steps' keys: the next ones come to L2 while the projection before this kernel still runs
+  for (int i = 1, n = j + 16; i < 8 && n < pos; ++i, n += 16) {
+    if ((l16 & 3) == 0) prefetch_l2(((l16 & 4) ? vp : kp) - l16 * 8 + (l16 >> 3) * 64 + (long long)n * A);
+  }
+  pdl_wait();
   if (warp < 3) {
     const __nv_bfloat16* src = qkv + (long long)b * 3 * A + warp * A + h * 128;
     float2 x1 = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 2 * lane));
@@ -541,14 +566,14 @@ extern "C" {
 using namespace bones;
 
 // X [b, K], W [N, K], out [b, N], all bf16 and contiguous; N a multiple of 128, K of 64, b <= 128.  `splits`: CTAs of a cluster
-// that share a tile's contraction (1, 2, 4 or 8; at most 4 for b <= 16).  `pdl`: the previous kernel on the stream is one of this file's.
+// that share a tile's contraction (1, 2, 4, 8 or 16; a CTA finishes four tokens or more, so few
+// sequences are padded to 4 * splits).  `pdl`: the previous kernel on the stream is one of this file's.
 int bones_decode_gemm(const void* X, const void* W, void* out, int b, int N, int K, int splits, int epi, const float* ssq_in, int n_ssq,
                       const void* res, const void* x0, const float* mix_a, const float* mix_b, float* ssq_out, float cap, int pdl, void* stream) {
-  if (b < 1 || b > 128 || (N % 128) || (K % 64) || N <= 0 || K <= 0 || (splits != 1 && splits != 2 && splits != 4 && splits != 8) || splits > K / 64)
+  if (b < 1 || b > 128 || (N % 128) || (K % 64) || N <= 0 || K <= 0 || (splits != 1 && splits != 2 && splits != 4 && splits != 8 && splits != 16) || splits > K / 64)
     return -2;
   if (((uintptr_t)X & 15) || ((uintptr_t)W & 15) || (epi == DEC_RES && !res)) return -2;
-  const int nb = b <= 16 ? 16 : b <= 32 ? 32 : b <= 64 ? 64 : 128;
-  if (nb / splits < 4) return -2;
+  const int rows = b > 4 * splits ? b : 4 * splits, nb = rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128;
   DecGemmParams p;
   p.N = N; p.b = b; p.KB = K / 64;
   p.ssq_in = ssq_in; p.n_ssq = n_ssq; p.inv_k = 1.0f / (float)K;

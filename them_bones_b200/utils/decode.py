@@ -192,10 +192,14 @@ class NativeDecoder:
 
     def _proj(self, x, w, out, epi, ssq=None, n_ssq=0, res=None, mix=None, ssq_out=None):
         """One projection of the fused step (``bones_decode_gemm``).  The contraction is split over a cluster until the CTAs
-        cover the SMs: a tile is 128 output columns, so 1280 columns are 10 tiles and 8 CTAs share each."""
+        cover the SMs: a tile is 128 output columns, so 1280 columns are 10 tiles and 8 or 16 CTAs share each.  A CTA finishes at
+        least four sequences: 4, 8 or 16 CTAs for up to 16, 32, 64.  Above 32 sequences the exchange of the partial sums (32 KB
+        a CTA) costs as much as the loads: two CTAs where there are tiles enough, else sixteen, and above 64, where an SM holds one
+        CTA, eight.  Measured a layer (1280 columns), qkv and c_fc in 4 / 2 CTAs: batch 64 38.8 / 37.8 us, batch 24 28.9 / 30.5,
+        batch 8 26.9 / 31.1; out or c_proj in 8 / 16: batch 128 62 / 74, batch 64 38.1 / 36.6, batch 32 28.6 / 30.9."""
         from ..ops import _lib as L
         b, (n, k) = x.shape[0], w.shape
-        splits, most = 1, 4 if b <= 16 else 8
+        splits, most = 1, 4 if b <= 16 else 8 if b <= 32 else 2 if n // 128 > 10 else 16 if b <= 64 else 8
         while splits < most and n // 128 * splits * 2 <= 160 and splits * 2 <= k // 64:
             splits *= 2
         x0, ma, mb = (self.x0, mix[0], mix[1]) if mix is not None else (None, None, None)
