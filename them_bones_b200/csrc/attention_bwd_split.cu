@@ -3,13 +3,14 @@
 //   dkv kernel   one CTA per 128-key tile walks the query tiles that see it, in transposed form so that keys are the
 //                TMEM lanes:  S^T = Kh Qh^T,  dP^T = V dO^T,  P^T = exp2(S^T c1 - lse2) masked,  dV += P^T dO,
 //                dS^T = P^T (dP^T - delta) scale,  dK += dS^T Qh.
-//   dq kernel    one CTA per 128-query tile walks its key tiles (queries are the lanes):  S and dP again, dS, dQ += dS Kh.
+//                dS^T also goes to memory where there is scratch for it.
+//   dq kernel    one CTA per 128-query tile walks its key tiles (queries are the lanes):  dQ += dS Kh with the stored dS^T, or, without
+//                the scratch, S and dP again, dS, dQ += dS Kh.
 //
-// P^T, dS^T and dS never touch shared memory: the compute warps write them back to TMEM as packed bf16 pairs over the
+// P^T, dS^T and dS reach their MMAs without shared memory: the compute warps write them back to TMEM as packed bf16 pairs over the
 // columns of the fp32 tile they were computed from, and the next MMA takes its A operand from TMEM.  Every accumulator
-// (dK, dV, dQ) lives in TMEM for the whole CTA: no atomics, no per-tile drain, deterministic results.  Recomputing S and
-// dP in the second kernel costs two extra GEMMs per tile pair; in the single-kernel form (attention_bwd.cu) TMEM is full
-// and the five GEMMs serialise with the exponentiation and a dQ drain through fp32 atomics.
+// (dK, dV, dQ) lives in TMEM for the whole CTA: no atomics, no per-tile drain, deterministic results.  In the single-kernel
+// form (attention_bwd.cu) TMEM is full and the five GEMMs serialise with the exponentiation and a dQ drain through fp32 atomics.
 // Outputs are bf16: dq-hat | dk-hat as [B*T, 2A] for the RoPE / QK-norm backward, dV straight into its third of dqkv.
 // Operand views, masking and scaling are those of attention_bwd.cu; the saved log-sum-exp is consumed through a
 // pre-pass that also computes delta = rowsum(dO * O).

@@ -3,10 +3,9 @@
 //
 // Bound by launches, not by bytes: at 16384 tokens and 16 experts the logits are 1 MB, and the same arithmetic as PyTorch
 // operators was about 50 kernels forward and backward of 2 to 10 us each (about 200 us of 2050, and 800 us of host time); the two
-// passes take 17 us.  One thread
-// per token; a CTA stages its 128 tokens' logits in shared memory (rows of E + 1 floats: no bank conflicts by row or by
-// column).  Sums over tokens are per-CTA partials added in a fixed order by a second small kernel: results are the same on
-// every run.
+// passes take 17 us.  One thread per token; a CTA stages its 128 tokens' logits in shared memory (rows of E + 1 floats: no bank
+// conflicts by row or by column).  Sums over tokens are per-CTA partials added in a fixed order by a second small kernel: results
+// are the same on every run.
 #include "common.cuh"
 
 namespace bones {
