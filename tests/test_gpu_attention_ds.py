@@ -15,6 +15,17 @@ def test_number_of_tile_pairs(t, window):
     assert ds_tiles(t, window) == sum(1 for q in range(n) for k in range(q + 1) if w == 0 or q - k < w)
 
 
+def test_scratch_is_optional(monkeypatch):
+    from them_bones_b200.ops import attention_bwd as AB
+    assert AB._ds_scratch(4096, "cpu").numel() == 4096 and AB._ds_scratch(AB.DS_LIMIT + 1, "cpu") is None
+
+    def none_left(*args, **kwargs):
+        raise torch.OutOfMemoryError("no memory")
+
+    monkeypatch.setattr(torch, "empty", none_left)
+    assert AB._ds_scratch(4096, "cpu") is None
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("b,t,h,d,window,docs", CASES)
 def test_both_routes_agree(monkeypatch, b, t, h, d, window, docs):
