@@ -502,7 +502,8 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const long long* tok,
 // Last kernel of a step, one CTA per sequence: arg-max of the logits (lowest index of equal values, a NaN above everything),
 // the forced token while the prompt lasts, and the position's advance by the last CTA to finish.
 __global__ void __launch_bounds__(1024) decode_end_kernel(const __nv_bfloat16* __restrict__ logits, long long ldl, int V, int* pos_ptr,
-                                                          const int* __restrict__ prompt_len, long long* out, int L, long long* tok, int* ticket) {
+                                                          const int* __restrict__ prompt_len, long long* out, long long ldo, int L, long long* tok,
+                                                          int* ticket) {
   __shared__ float sv[32];
   __shared__ int si[32];
   pdl_wait();
@@ -547,8 +548,8 @@ __global__ void __launch_bounds__(1024) decode_end_kernel(const __nv_bfloat16* _
       const int pos = *pos_ptr + 1;
       long long nxt = at;
       if (pos < L) {
-        if (pos < *prompt_len) nxt = out[(long long)b * L + pos];
-        else out[(long long)b * L + pos] = nxt;
+        if (pos < *prompt_len) nxt = out[b * ldo + pos];
+        else out[b * ldo + pos] = nxt;
       }
       tok[b] = nxt;
       __threadfence();
@@ -618,9 +619,9 @@ int bones_decode_begin(const long long* tok, const int* pos, int* doc_start, lon
   return (int)cudaGetLastError();
 }
 
-// ticket: one int, zero before the first step
-int bones_decode_end(const void* logits, long long ldl, int V, int* pos, const int* prompt_len, long long* out, int L, long long* tok, int* ticket,
-                     int B, void* stream) {
+// out: rows of L tokens, ldo apart; ticket: one int, zero before the first step
+int bones_decode_end(const void* logits, long long ldl, int V, int* pos, const int* prompt_len, long long* out, long long ldo, int L, long long* tok,
+                     int* ticket, int B, void* stream) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
   cfg.gridDim = dim3((unsigned)B);
@@ -628,6 +629,6 @@ int bones_decode_end(const void* logits, long long ldl, int V, int* pos, const i
   cfg.stream = (cudaStream_t)stream;
   cfg.attrs = at;
   cfg.numAttrs = (unsigned)dec_launch_attrs(at, 1, 1);
-  return (int)cudaLaunchKernelEx(&cfg, decode_end_kernel, (const __nv_bfloat16*)logits, ldl, V, pos, prompt_len, out, L, tok, ticket);
+  return (int)cudaLaunchKernelEx(&cfg, decode_end_kernel, (const __nv_bfloat16*)logits, ldl, V, pos, prompt_len, out, ldo, L, tok, ticket);
 }
 }  // extern "C"

@@ -126,6 +126,13 @@ def _rope_at(x, cos, sin):
     return torch.cat([x1 * c + x2 * s, -x1 * s + x2 * c], -1).to(x.dtype)
 
 
+def _token_rows(out, b, device) -> bool:
+    """Whether ``out`` is what the fused step's last kernel reads forced tokens from and writes generated ones to by address:
+    ``b`` rows of int64 on the model's device, each contiguous, any distance apart that keeps them disjoint."""
+    return (out.dim() == 2 and out.shape[0] == b and out.dtype == torch.int64 and out.device == device and out.stride(1) == 1
+            and (b == 1 or out.stride(0) >= out.shape[1]))
+
+
 class NativeDecoder:
     """One decode step as a CUDA graph over the native kernels: embedding, fused norms, tcgen05 GEMMs, the two decode
     kernels (``csrc/decode.cu``: RoPE + QK-norm + cache append, cached attention), soft-capped logits, arg-max.  The
@@ -179,14 +186,15 @@ class NativeDecoder:
             self.part = torch.empty(max(b * w.shape[0] * (w.shape[1] // 256) for w in ws), dtype=torch.float32, device=dev)
 
     def _fused_ok(self) -> bool:
-        """Whether the step runs on the kernels of ``csrc/decode_gemm.cu``: a plain dense decoder with at most 128 sequences."""
+        """Whether the step runs on the kernels of ``csrc/decode_gemm.cu``: a plain dense decoder with at most 128 sequences.
+        Any other ``out`` goes through the indexed reads and writes of the general step, which take or refuse it."""
         model, cfg = self.model, self.model.config
         ws = [w for blk, dense in zip(model.transformer.h, self.dense) if dense
               for w in (blk.attn.c_q.weight, blk.attn.c_k.weight, blk.attn.c_v.weight, blk.attn.c_proj.weight, blk.mlp.c_fc.weight, blk.mlp.c_proj.weight)]
         ws += [model.lm_head.weight, model.transformer.wte.weight]
         scalars = [v for blk in model.transformer.h for v in (blk.resid_lambda, blk.x0_lambda)]
         return (self.tok.shape[0] <= 128 and all(self.dense) and model.tables is None and model.value_embeds is None and not model.n_skip
-                and len(model.transformer.h) > 0 and cfg.n_embd % 128 == 0
+                and len(model.transformer.h) > 0 and cfg.n_embd % 128 == 0 and _token_rows(self.out, self.tok.shape[0], self.tok.device)
                 and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.shape[0] % 128 == 0 and w.shape[1] % 64 == 0 for w in ws)
                 and all(v.dtype == torch.float32 for v in scalars) and model.cos.dtype == torch.float32 and model.sin.dtype == torch.float32)
 
@@ -233,7 +241,8 @@ class NativeDecoder:
             n_ssq = tiles
         self._proj(self.xa, model.lm_head.weight, self.last_logits, 3, ssq=self.ssq_a, n_ssq=n_ssq)
         L.call("bones_decode_end", L.ptr(self.last_logits), ctypes.c_longlong(self.last_logits.shape[1]), _I(cfg.vocab_size), L.ptr(pos),
-               L.ptr(self.prompt_len), L.ptr(self.out), _I(self.out.shape[1]), L.ptr(tok), L.ptr(self.ticket), _I(b), L.stream())
+               L.ptr(self.prompt_len), L.ptr(self.out), ctypes.c_longlong(self.out.stride(0)), _I(self.out.shape[1]), L.ptr(tok), L.ptr(self.ticket), _I(b),
+               L.stream())
 
     def _lin(self, x, w, mode=0, residual=None):
         """``x [b, k] @ w[n, k]^T`` as ``k / 256`` batched partial products into fp32 slices, then their ordered sum as
