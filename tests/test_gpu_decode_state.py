@@ -58,3 +58,37 @@ def test_token_rows_of_another_type_are_refused():
     assert not dec.fused
     with pytest.raises((RuntimeError, IndexError)):
         dec.run(1)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("b,window", [(64, 0), (7, 128)])
+def test_documents_that_begin_at_many_steps(b, window):
+    """Every step some sequences begin a document: their attention sees nothing before it, from that very step on."""
+    from them_bones_b200.utils import decode as D
+    model, steps = _model(n_layer=3, attn_window=window, attn_long=(2,)), 150
+    toks = torch.randint(1, 1000, (b, steps), device="cuda")
+    toks[torch.rand(b, steps, device="cuda") < 0.2] = 0
+    toks[:, 0] = 0
+    toks[: b // 2, steps - 1] = 0
+    out = torch.cat([toks, torch.zeros(b, 1, dtype=torch.int64, device="cuda")], 1)
+    with torch.no_grad():
+        cache = D.KVCache(model, b, steps + 1)
+        dec = D.NativeDecoder(model, cache, toks[:, 0], out, prompt_len=steps)
+        assert dec.fused
+        dec.run(steps)
+        got = dec.last_logits.float()
+        # a document that begins with the last token: the same logits as that token alone
+        alone = D._forward_cached(model, toks[: b // 2, -1:], _at(D.KVCache(model, b // 2, steps + 1), steps - 1))
+        ref = D._forward_cached(model, toks, D.KVCache(model, b, steps + 1))
+    D.L_check()
+    last = torch.where(toks == 0, torch.arange(steps, device="cuda"), 0).amax(1).int()
+    assert torch.equal(cache.doc_start, last)
+    rel = ((got - ref).norm(dim=1) / ref.norm(dim=1))
+    assert float(rel.max()) < 6e-2, rel            # bf16 activations of three layers, row by row
+    rel = ((got[: b // 2] - alone).norm(dim=1) / alone.norm(dim=1))
+    assert float(rel.max()) < 6e-2, rel
+
+
+def _at(cache, pos):
+    cache.len = pos
+    return cache
