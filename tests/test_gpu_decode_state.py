@@ -92,3 +92,34 @@ def test_documents_that_begin_at_many_steps(b, window):
 def _at(cache, pos):
     cache.len = pos
     return cache
+
+
+@pytest.mark.gpu
+def test_unknown_token_ids_have_zero_rows():
+    """An id outside the embedding gives that sequence a zero row at that step, as in the embedding gather, not what an earlier
+    step or another sequence left."""
+    from them_bones_b200.utils import decode as D
+    model, b, p = _model(), 6, 5
+    for blk in model.transformer.h:
+        blk.resid_lambda.data.fill_(0.9)
+        blk.x0_lambda.data.fill_(0.3)
+    toks = torch.randint(1, 1000, (b, p), device="cuda")
+    toks[:, 0] = 0
+    rows = model.transformer.wte.weight.shape[0]
+    model.transformer.wte.weight.data[777] = 0
+    toks[toks == 777] = 5
+
+    def logits(ids):
+        out = torch.cat([ids, torch.zeros(b, 1, dtype=torch.int64, device="cuda")], 1)
+        with torch.no_grad():
+            dec = D.NativeDecoder(model, D.KVCache(model, b, p + 1), ids[:, 0], out, prompt_len=p)
+            assert dec.fused
+            dec.run(p)
+        return dec.last_logits.clone()
+
+    zero, unknown = toks.clone(), toks.clone()
+    zero[1, 2] = zero[4, p - 1] = zero[3, 1] = 777
+    unknown[1, 2], unknown[4, p - 1], unknown[3, 1] = rows, -1, rows + 12345
+    got, want = logits(unknown), logits(zero)
+    D.L_check()
+    assert torch.equal(got, want)

@@ -497,14 +497,15 @@ __global__ void __launch_bounds__(256) decode_begin_kernel(const long long* tok,
     for (int i = 0; i < 8; ++i) s += red[i];
     return s;
   };
-  if (t < 0 || t >= rows) return;              // uniform over the CTA
-  const __nv_bfloat16* e = wte + t * C;
+  const bool known = t >= 0 && t < rows;       // any other id has a zero row, as in the embedding gather
+  const __nv_bfloat16* e = wte + (known ? t : 0) * C;
+  auto at = [&](int c) { return known ? __bfloat162float(e[c]) : 0.f; };
   float s = 0.f;
-  for (int c = threadIdx.x; c < C; c += 256) { const float f = __bfloat162float(e[c]); s += f * f; }
+  for (int c = threadIdx.x; c < C; c += 256) { const float f = at(c); s += f * f; }
   const float r = rsqrtf(sum(s) / C + 1.1920928955078125e-07f), ma = *mix_a, mb = *mix_b;
   s = 0.f;
   for (int c = threadIdx.x; c < C; c += 256) {
-    const __nv_bfloat16 z = __float2bfloat16(__bfloat162float(e[c]) * r);
+    const __nv_bfloat16 z = __float2bfloat16(at(c) * r);
     const float f = __bfloat162float(z);
     const __nv_bfloat16 m = __float2bfloat16(ma * f + mb * f);
     x0[(long long)b * C + c] = z;
