@@ -35,6 +35,12 @@ def _ds_scratch(nbytes, device):
         return None
 
 
+def _aligned(x):
+    """Contiguous and 16-byte aligned (what the kernels' tensor maps and vector loads need)."""
+    x = x if x.is_contiguous() else x.contiguous()
+    return x if x.data_ptr() % 16 == 0 else x.clone()
+
+
 def length_multiple(head_dim: int) -> int:
     """The sequence length has to be a multiple of this: the split kernels take any length, the fused one whole tiles."""
     return 128 if _IMPL == "fused" and head_dim == 128 else 1
@@ -43,11 +49,9 @@ def length_multiple(head_dim: int) -> int:
 def backward(dy, qkv2, qk, y, lse, cos, sin, ds, b, t, n_head, head_dim, scale, window):
     m, a = b * t, n_head * head_dim
     dev = dy.device
-    dy2 = (dy if dy.is_contiguous() else dy.contiguous()).view(m, a)
+    dy2 = _aligned(dy).view(m, a)
     dqkv = torch.empty(m, 3 * a, dtype=torch.bfloat16, device=dev)
     if _IMPL != "fused" or head_dim != 128:
-        if t % 128 and dy2.data_ptr() % 16:
-            dy2 = dy2.clone()
         # statistics of whole 128-query tiles, and behind them the two kernels' work-item counters
         n = b * n_head * (-(-t // 128) * 128) * 2
         stats = torch.empty(n + 2, dtype=torch.float32, device=dev)

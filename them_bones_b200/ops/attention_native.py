@@ -14,6 +14,7 @@ import ctypes
 import torch
 
 from . import _lib as L
+from .attention_bwd import _aligned
 
 _I, _L, _F = ctypes.c_int, ctypes.c_longlong, ctypes.c_float
 SUPPORTED_HEAD_DIMS = (128, 64)
@@ -62,22 +63,15 @@ def attn_forward(qk, qkv2, doc_start, b, t, n_head, scale, window, head_dim=128)
     return y, lse
 
 
-def _aligned(x):
-    """Contiguous and 16-byte aligned (what the kernels' tensor maps and vector loads need)."""
-    x = x if x.is_contiguous() else x.contiguous()
-    return x if x.data_ptr() % 16 == 0 else x.clone()
-
-
 class _AttnFn(torch.autograd.Function):
     @staticmethod
     def forward(ctx, qkv, cos, sin, n_head, head_dim, scale, doc_start, window):
         b, t, _ = qkv.shape
         a = n_head * head_dim
-        # a tensor of a ragged length may begin anywhere in its storage (one sequence of a packed batch)
-        fix = _aligned if t % 128 else (lambda x: x if x.is_contiguous() else x.contiguous())
-        qkv2 = fix(qkv).view(b * t, -1)
-        cos, sin = fix(cos.float()), fix(sin.float())
-        ds = fix(doc_start.to(torch.int32)) if doc_start is not None else None
+        # a tensor may begin anywhere in its storage (one sequence of a packed batch)
+        qkv2 = _aligned(qkv).view(b * t, -1)
+        cos, sin = _aligned(cos.float()), _aligned(sin.float())
+        ds = _aligned(doc_start.to(torch.int32)) if doc_start is not None else None
         dev = qkv2.device
         qk = torch.empty(b * t, 2 * a, dtype=qkv2.dtype, device=dev)
         y = torch.empty(b, t, a, dtype=qkv2.dtype, device=dev)
