@@ -607,6 +607,7 @@ using namespace bones;
 
 int bones_rope_qknorm_fwd(const void* qkv, const float* cosT, const float* sinT, void* qk, int* counter, long long M, int T, int H, int D,
                           void* stream) {
+  if (misaligned16(qkv, qk, cosT, sinT)) return -3;
   if (D == 128) return launch_rope_fwd<128>(qkv, cosT, sinT, qk, counter, M, T, H, (cudaStream_t)stream);
   if (D == 64) return launch_rope_fwd<64>(qkv, cosT, sinT, qk, counter, M, T, H, (cudaStream_t)stream);
   return -2;
@@ -616,6 +617,7 @@ int bones_rope_qknorm_fwd(const void* qkv, const float* cosT, const float* sinT,
 int bones_rope_qknorm_bwd(const void* qkv, const float* cosT, const float* sinT, const float* dqk, const void* dv, void* dqkv, long long M,
                           int T, int H, int D, void* stream) {
   if (D != 128) return -2;
+  if (misaligned16(qkv, dqk, cosT, sinT, dv, dqkv)) return -3;
   const long long threads = M * 3 * H * 8;
   rope_qknorm_bwd128_kernel<<<(unsigned)((threads + 255) / 256), 256, 0, (cudaStream_t)stream>>>(
       (const __nv_bfloat16*)qkv, cosT, sinT, dqk, (const __nv_bfloat16*)dv, (__nv_bfloat16*)dqkv, M, T, H);
@@ -625,6 +627,7 @@ int bones_rope_qknorm_bwd(const void* qkv, const float* cosT, const float* sinT,
 // dqk: bf16 [M, 2*H*D]; writes the q and k thirds of dqkv [M, 3*H*D]
 int bones_rope_qknorm_bwd_bf16(const void* qkv, const float* cosT, const float* sinT, const void* dqk, void* dqkv, long long M, int T, int H,
                                int D, void* stream) {
+  if (misaligned16(qkv, dqk, cosT, sinT, dqkv)) return -3;
   const long long threads = M * H * (D / 16);
   const unsigned grid = (unsigned)((threads + 255) / 256);
   const auto *x = (const __nv_bfloat16*)qkv, *g = (const __nv_bfloat16*)dqk;

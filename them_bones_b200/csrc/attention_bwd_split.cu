@@ -1013,6 +1013,7 @@ int bones_rope_qknorm_bwd_bf16(const void* qkv, const float* cosT, const float* 
 
 // stats: [B, H, Tp] float2 scratch (Tp: T rounded up to a multiple of 128); counters: two ints, zeroed here
 int bones_attn_bwd_stats(const void* dy, const void* y, const float* lse, void* stats, int* counters, int B, int T, int H, int D, void* stream) {
+  if (misaligned16(dy, y, stats)) return -3;
   const int Tp = (T + ST - 1) / ST * ST;
   const long long threads = (long long)B * H * Tp / 2 * (D / 8);
   const unsigned grid = (unsigned)((threads + 255) / 256);
@@ -1029,9 +1030,7 @@ int bones_attn_bwd_stats(const void* dy, const void* y, const float* lse, void* 
 int bones_attn_bwd_split(const void* qk, const void* qkv, const void* dy, const void* stats, int* counters, void* dqk, void* dv,
                          long long dv_ld, void* ds, const int* doc_start, int B, int T, int H, int D, float scale, int window_tiles, void* stream) {
   if (D != 128 && D != 64) return -2;
-  if ((dv_ld % 16) || ((uintptr_t)dv & 31) || ((uintptr_t)dqk & 31) || ((uintptr_t)stats & 15) ||
-      (doc_start && ((uintptr_t)doc_start & 15)))
-    return -3;
+  if ((dv_ld % 16) || ((uintptr_t)dv & 31) || ((uintptr_t)dqk & 31) || ((uintptr_t)stats & 15)) return -3;
   const long long A = (long long)H * D;
   CUtensorMap tq, tv, td;
   int rc = tmap_rows_3d_s(&tq, qk, B, T, 2 * A);

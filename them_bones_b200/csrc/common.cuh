@@ -390,6 +390,11 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
 EncodeTiledFn get_encode_tiled();
 int* error_word();             // device pointer to the library's error word (allocated on first use per device)
+// whether any of the pointers is not 16-byte aligned: what a kernel with 16-byte accesses asks before its launch
+template <typename... Ptrs>
+inline bool misaligned16(const Ptrs*... p) {
+  return ((((uintptr_t)p & 15) != 0) || ...);
+}
 int make_tmap(CUtensorMap* out, CUtensorMapDataType dt, int rank, const void* base, const uint64_t* dims, const uint64_t* strides_bytes,
               const uint32_t* box, CUtensorMapSwizzle swz);
 }  // namespace bones

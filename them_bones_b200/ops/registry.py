@@ -31,8 +31,8 @@ def attention_fwd(qkv: Tensor, cos: Tensor, sin: Tensor, doc_start: Optional[Ten
                   window: int) -> Tuple[Tensor, Tensor, Tensor]:
     from . import attention_native as AN
     b, t, _ = qkv.shape
-    qkv2 = qkv.contiguous().view(b * t, -1)
-    qk = AN.rope_qknorm(qkv2, cos, sin, t, n_head, head_dim)
+    qkv2 = AN._aligned(qkv).view(b * t, -1)
+    qk = AN.rope_qknorm(qkv2, AN._aligned(cos), AN._aligned(sin), t, n_head, head_dim)
     y, lse = AN.attn_forward(qk, qkv2, doc_start, b, t, n_head, scale, window)
     return y.view(b, t, n_head * head_dim), lse, qk
 
@@ -49,8 +49,8 @@ def attention_bwd(dy: Tensor, qkv: Tensor, qk: Tensor, y: Tensor, lse: Tensor, c
                   n_head: int, head_dim: int, scale: float, window: int) -> Tensor:
     from . import attention_bwd as AB
     b, t, _ = qkv.shape
-    qkv2 = qkv.contiguous().view(b * t, -1)
-    dqkv = AB.backward(dy, qkv2, qk, y.reshape(b * t, -1), lse, cos, sin, doc_start, b, t, n_head, head_dim, scale, window)
+    qkv2 = AB._aligned(qkv).view(b * t, -1)
+    dqkv = AB.backward(dy, qkv2, qk, y.reshape(b * t, -1), lse, AB._aligned(cos), AB._aligned(sin), doc_start, b, t, n_head, head_dim, scale, window)
     return dqkv.view(b, t, -1)
 
 
