@@ -123,3 +123,37 @@ def test_unknown_token_ids_have_zero_rows():
     got, want = logits(unknown), logits(zero)
     D.L_check()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("sms", [64, 132, 148, 160])
+@pytest.mark.parametrize("width", [128, 256, 512, 1024, 1280, 1408, 1536, 1664, 2048, 4096])
+def test_projection_splits_follow_the_device(width, sms):
+    """Powers of two that leave every CTA a K block and fit the device; a projection with few tiles is shared until the CTAs cover
+    a good part of it, at any width."""
+    from them_bones_b200.utils.decode import projection_splits
+    for b in (1, 16, 17, 32, 33, 64, 65, 128):
+        for n, k, res in ((3 * width, width, False), (width, width, True), (4 * width, width, False), (width, 4 * width, True), (65536, width, False)):
+            s = projection_splits(b, n, k, res, sms)
+            tiles, most = n // 128, 4 if b <= 16 else 8 if b <= 32 or b > 64 else 16
+            assert s in (1, 2, 4, 8, 16) and s <= most and s <= k // 64
+            assert s == 1 or tiles * s <= 1.6 * sms and (b <= 64 or tiles * s <= sms)
+            if res and s < most and 2 * s <= k // 64:
+                assert tiles * s > 0.4 * sms, (b, n, k, s)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("width,b", [(384, 40), (1408, 64), (1408, 100), (1536, 24), (2048, 8), (2048, 70)])
+def test_step_at_other_widths(width, b):
+    from them_bones_b200.utils import decode as D
+    model, steps = _model(n_embd=width), 6
+    toks = torch.randint(1, 1000, (b, steps), device="cuda")
+    toks[:, 0] = 0
+    out = torch.cat([toks, torch.zeros(b, 1, dtype=torch.int64, device="cuda")], 1)
+    with torch.no_grad():
+        dec = D.NativeDecoder(model, D.KVCache(model, b, steps + 1), toks[:, 0], out, prompt_len=steps)
+        assert dec.fused
+        dec.run(steps)
+        ref = D._forward_cached(model, toks, D.KVCache(model, b, steps + 1))
+    D.L_check()
+    got = dec.last_logits.float()
+    assert float((got - ref).norm() / ref.norm()) < 3e-2          # bf16 activations of two layers

@@ -133,6 +133,32 @@ def _token_rows(out, b, device) -> bool:
             and (b == 1 or out.stride(0) >= out.shape[1]))
 
 
+def projection_splits(b, n, k, residual, sms):
+    """CTAs of a cluster that share the contraction of each 128-column tile of a decode projection (``n`` columns, ``k`` long).
+
+    Doubled while a CTA keeps a K block of 64, up to what the batch makes worth while and what the ``sms`` SMs take in one go.
+    A CTA finishes at least four sequences: up to 16 of them 4 CTAs (8 pad the sequences to 32), up to 32 8 CTAs.  Above, the exchange
+    of the partial sums (32 KB a CTA) costs as much as the loads: 2 CTAs, except that the residual epilogue (out, c_proj: few columns,
+    and per sequence a residual, x0 and sums of squares to handle) is shorter the fewer sequences a CTA finishes: 16, and 8 above
+    64 sequences, where an SM holds one CTA.  Room: two CTAs of up to 64 sequences fit an SM, but clusters leave gaps: 1.6 CTAs an
+    SM, 1.25 where clusters of 8 meet 17 to 32 sequences, one above 64 sequences and 0.8 of clusters of four or more (16 tiles
+    by 8 CTAs: 524 us where 4 take 480).
+
+    Six layers, us a step, this rule against 2 CTAs for every projection of more than ten tiles and at most 160 CTAs: 1280 wide the
+    same (batch 64 242, batch 24 186, batch 8 171); 1408 wide 256 for 342 at batch 64, 336 for 399 at 128; 2048 wide 349 for 441, 437 for 515,
+    246 for 253 at batch 8; 256 wide 145 for 148 and 204 for 212; 512 to 1152 wide the same.
+    """
+    tiles, kb = n // 128, k // 64
+    most = 4 if b <= 16 else 8 if b <= 32 else 2 if not residual else 16 if b <= 64 else 8
+    splits = 1
+    while splits < most and splits * 2 <= kb:
+        room = 1.6 if b <= 16 or 32 < b <= 64 else 1.25 if b <= 32 else 1.0 if splits == 1 else 0.8
+        if tiles * splits * 2 > room * sms:
+            break
+        splits *= 2
+    return splits
+
+
 class NativeDecoder:
     """One decode step as a CUDA graph over the native kernels: embedding, fused norms, tcgen05 GEMMs, the two decode
     kernels (``csrc/decode.cu``: RoPE + QK-norm + cache append, cached attention), soft-capped logits, arg-max.  The
@@ -175,6 +201,7 @@ class NativeDecoder:
             self.qkv = torch.empty(b, 3 * a, dtype=bf, device=dev)
             self.h = torch.empty(b, cfg.mlp_ratio * c, dtype=bf, device=dev)
             self.ssq_a, self.ssq_b = (torch.empty(c // 128, b, dtype=f32, device=dev) for _ in range(2))
+            self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
             self.ticket = torch.zeros(1, dtype=torch.int32, device=dev)
             self.last_logits = torch.empty(b, model.lm_head.weight.shape[0], dtype=bf, device=dev)
         elif self.split:
@@ -199,17 +226,10 @@ class NativeDecoder:
                 and all(v.dtype == torch.float32 for v in scalars) and model.cos.dtype == torch.float32 and model.sin.dtype == torch.float32)
 
     def _proj(self, x, w, out, epi, ssq=None, n_ssq=0, res=None, mix=None, ssq_out=None):
-        """One projection of the fused step (``bones_decode_gemm``).  The contraction is split over a cluster until the CTAs
-        cover the SMs: a tile is 128 output columns, so 1280 columns are 10 tiles and 8 or 16 CTAs share each.  A CTA finishes at
-        least four sequences: 4, 8 or 16 CTAs for up to 16, 32, 64.  Above 32 sequences the exchange of the partial sums (32 KB
-        a CTA) costs as much as the loads: two CTAs where there are tiles enough, else sixteen, and above 64, where an SM holds one
-        CTA, eight.  Measured a layer (1280 columns), qkv and c_fc in 4 / 2 CTAs: batch 64 38.8 / 37.8 us, batch 24 28.9 / 30.5,
-        batch 8 26.9 / 31.1; out or c_proj in 8 / 16: batch 128 62 / 74, batch 64 38.1 / 36.6, batch 32 28.6 / 30.9."""
+        """One projection of the fused step (``bones_decode_gemm``), its contraction shared as ``projection_splits`` says."""
         from ..ops import _lib as L
         b, (n, k) = x.shape[0], w.shape
-        splits, most = 1, 4 if b <= 16 else 8 if b <= 32 else 2 if n // 128 > 10 else 16 if b <= 64 else 8
-        while splits < most and n // 128 * splits * 2 <= 160 and splits * 2 <= k // 64:
-            splits *= 2
+        splits = projection_splits(b, n, k, res is not None, self.sms)
         x0, ma, mb = (self.x0, mix[0], mix[1]) if mix is not None else (None, None, None)
         L.call("bones_decode_gemm", L.ptr(x), L.ptr(w), L.ptr(out), _I(b), _I(n), _I(k), _I(splits), _I(epi), L.ptr(ssq), _I(n_ssq), L.ptr(res),
                L.ptr(x0), L.ptr(ma), L.ptr(mb), L.ptr(ssq_out), ctypes.c_float(self.model.config.softcap), _I(1),
