@@ -31,3 +31,26 @@ def test_combine_matches_statement(n, k, e, cap, c, with_res, with_tok):
     assert bool((got[0][tok == n] == 0).all()) and bool((got[1][slot == e * cap] == 0).all())
     if with_res:
         assert torch.equal(got[2], dout)
+
+
+@pytest.mark.parametrize("n,k,c", [(1, 0, 8), (37, 3, 264), (64, 8, 128), (50, 9, 264), (5, 13, 1280), (3, 40, 64)])
+def test_any_number_of_choices(n, k, c):
+    """Up to eight choices a token keeps its slots in registers; any other number goes through the general form."""
+    from them_bones_b200 import ops
+    g = torch.Generator(device="cuda").manual_seed(n + k)
+    slots = n * k + 5
+    perm = torch.randperm(slots, generator=g, device="cuda")[: n * k].view(n, k)
+    slot = torch.where(torch.rand(n, k, generator=g, device="cuda") < 0.2, slots, perm)
+    ys, dout = (torch.randn(m, c, generator=g, device="cuda").bfloat16() for m in (slots, n))
+    gates = torch.rand(n, k, generator=g, device="cuda")
+    ys.requires_grad_(True), gates.requires_grad_(True)
+    out = ops.moe_combine(ys, slot, gates)
+    dy, dg = torch.autograd.grad(out, [ys, gates], dout)
+    yp = torch.cat([ys.detach().double(), torch.zeros(1, c, device="cuda", dtype=torch.float64)])
+    want = (gates.detach().double()[..., None] * yp[slot]).sum(1)
+    rel = lambda a, b: float((a.double() - b).norm() / b.norm().clamp_min(1e-30))  # noqa: E731
+    assert rel(out.detach(), want) < 4e-3                      # one bf16 rounding
+    wdg = (yp[slot] * dout.double()[:, None]).sum(-1)
+    wdy = torch.zeros(slots + 1, c, device="cuda", dtype=torch.float64)
+    wdy.index_add_(0, slot.reshape(-1), (gates.detach().double()[..., None] * dout.double()[:, None]).reshape(-1, c))
+    assert rel(dg, wdg) < 1e-5 and rel(dy, wdy[:slots]) < 4e-3

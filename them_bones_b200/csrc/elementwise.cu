@@ -356,34 +356,45 @@ __global__ void scatter_add_rows_kernel(const __nv_bfloat16* dy, const IdxT* idx
 // out[n] = sum_k gates[n,k] * ys[slot[n,k]]   (slot == S: dropped)
 // gates null: all one.  residual: added to the combined row after its rounding, as a separate addition would.  A token's slots and
 // gates are read once and four column groups are in flight together (16384 x 1280 from two slots each, forward with the residual
-// and the dispatch gradient: 54 us; 60 and 20 for the addition before).
+// and the dispatch gradient: 54 us; 60 and 20 for the addition before).  K: topk rounded up to 1, 2 or 8; 0: any topk, its slots
+// and gates read for every column group.
 template <int K>
 __global__ void moe_combine_kernel(const __nv_bfloat16* __restrict__ ys, const long long* __restrict__ slot, const float* __restrict__ gates,
                                    const __nv_bfloat16* __restrict__ residual, __nv_bfloat16* __restrict__ out, int n, int C, int topk, long long S) {
+  constexpr int KR = K ? K : 1;
   const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= n) return;
-  const __nv_bfloat16* src[K];
-  float g[K];
-#pragma unroll
-  for (int k = 0; k < K; ++k) {                // K: topk rounded up to 1, 2 or 8
+  const __nv_bfloat16* src[KR];
+  float g[KR];
+  auto look = [&](int k, int r) {
     const long long s = k < topk ? slot[(size_t)row * topk + k] : -1;
     const bool live = s >= 0 && s < S;
-    src[k] = live ? ys + (size_t)s * C : nullptr;
-    g[k] = live ? (gates ? gates[(size_t)row * topk + k] : 1.0f) : 0.f;
-  }
+    src[r] = live ? ys + (size_t)s * C : nullptr;
+    g[r] = live ? (gates ? gates[(size_t)row * topk + k] : 1.0f) : 0.f;
+  };
+#pragma unroll
+  for (int k = 0; k < K; ++k) look(k, k);
 #pragma unroll 4
   for (int c = lane * 8; c < C; c += 256) {
     float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < K; ++k) {
-      if (!src[k]) continue;
-      const uint4 u = *reinterpret_cast<const uint4*>(src[k] + c);
+    auto add = [&](int r) {
+      if (!src[r]) return;
+      const uint4 u = *reinterpret_cast<const uint4*>(src[r] + c);
       const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
       for (int t = 0; t < 4; ++t) {
         const float2 f = unpack_bf16(w[t]);
-        acc[2 * t] += g[k] * f.x;
-        acc[2 * t + 1] += g[k] * f.y;
+        acc[2 * t] += g[r] * f.x;
+        acc[2 * t + 1] += g[r] * f.y;
+      }
+    };
+    if constexpr (K > 0) {
+#pragma unroll
+      for (int k = 0; k < K; ++k) add(k);
+    } else {
+      for (int k = 0; k < topk; ++k) {
+        look(k, 0);
+        add(0);
       }
     }
     uint4 o;
@@ -973,14 +984,15 @@ int bones_scatter_add_rows(const void* dy, const void* idx, int idx_is_64, float
 // gates, residual: null for all ones, none.  ys, out and residual 16-byte aligned
 int bones_moe_combine(const void* ys, const long long* slot, const float* gates, const void* residual, void* out, int n, int C, int topk, long long S,
                       void* stream) {
-  if ((C % 8) || topk < 1 || topk > 8) return -2;
+  if ((C % 8) || topk < 0) return -2;
   if (n <= 0) return 0;
 #define BONES_COMBINE(K)                                                                                                                  \
   moe_combine_kernel<K><<<ROW_GRID(n), 0, (cudaStream_t)stream>>>((const __nv_bfloat16*)ys, slot, gates, (const __nv_bfloat16*)residual, \
                                                                   (__nv_bfloat16*)out, n, C, topk, S)
   if (topk == 1) BONES_COMBINE(1);
   else if (topk == 2) BONES_COMBINE(2);
-  else BONES_COMBINE(8);
+  else if (topk >= 1 && topk <= 8) BONES_COMBINE(8);
+  else BONES_COMBINE(0);
 #undef BONES_COMBINE
   return (int)cudaGetLastError();
 }
