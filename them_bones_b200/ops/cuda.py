@@ -741,8 +741,8 @@ class _MoeRouterFn(torch.autograd.Function):
 
 
 def moe_router_ok(h, router, topk):
-    """The fused router covers bf16 activations, up to 64 experts and the GEMM's 16-byte rows."""
-    return h.dtype == BF16 and router.shape[0] <= 64 and h.shape[1] % 8 == 0 and topk in (1, 2) and h.shape[0] > 0
+    """The fused router covers bf16 activations, up to 64 experts, one or two different choices and the GEMM's 16-byte rows."""
+    return h.dtype == BF16 and router.shape[0] <= 64 and h.shape[1] % 8 == 0 and topk in (1, 2) and topk <= router.shape[0] and h.shape[0] > 0
 
 
 def moe_router(h, router, topk, aux_w, z_w, want_aux):
