@@ -19,7 +19,7 @@ struct CeAux {
 
 constexpr int CF_ROWS = 32, CF_WARPS = 16;
 
-// nll[row]; with `info` also what the gradient pass needs: (log2 of sum over weight, target weight, auxiliary weights).
+// nll[row]; with `info` also what the gradient pass needs: (log2 of sum over |weight|, target weight, auxiliary weights).
 // 32 rows per CTA, one per lane; the warps share the P partial sums and add them in a fixed order.
 __global__ void __launch_bounds__(CF_WARPS * 32) ce_finish_kernel(const float* __restrict__ part, int P, int M, const __nv_bfloat16* __restrict__ logits,
                                                                   long long ldl, const float* __restrict__ z_target, const long long* __restrict__ targets,
@@ -58,8 +58,9 @@ __global__ void __launch_bounds__(CF_WARPS * 32) ce_finish_kernel(const float* _
   if (aux.nll_aux) aux.nll_aux[row] = oa;
   const float w = valid ? (row_w ? row_w[row] : inv_loss_div / fmaxf(1.0f, *n_valid)) : 0.f;
   const float sum = w + a[0] + a[1];
-  // a row without any live target: lw = +inf makes every probability term exactly 0
-  info[row] = make_float4(sum > 0.f ? lse2 - log2f(sum) : __int_as_float(0x7f800000), w, a[0], a[1]);
+  // weights may be negative (the gradient pass takes the sign from their sum); a row without any live target: +inf makes every
+  // probability term exactly 0
+  info[row] = make_float4(sum != 0.f ? lse2 - log2f(fabsf(sum)) : __int_as_float(0x7f800000), w, a[0], a[1]);
 }
 
 // In place: z -> (w_sum softmax(z) - sum of target weights at their columns) (1 - (z / cap)^2); columns V .. ldl - 1 become 0.
@@ -78,6 +79,7 @@ __global__ void __launch_bounds__(256) ce_grad_kernel(__nv_bfloat16* __restrict_
     if (c < V) u[i] = *reinterpret_cast<const uint4*>(l + c);
   }
   const float4 f = info[row];
+  const bool neg = f.y + f.z + f.w < 0.f;
   const int t1 = f.y != 0.f ? (int)targets[row] : -8, t2 = f.z != 0.f ? (int)tg2[row] : -8, t3 = f.w != 0.f ? (int)tg3[row] : -8;
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -95,6 +97,7 @@ __global__ void __launch_bounds__(256) ce_grad_kernel(__nv_bfloat16* __restrict_
       float p0, p1;
       asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p0) : "f"(fmaf(z0, 1.4426950408889634f, -f.x)));
       asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(p1) : "f"(fmaf(z1, 1.4426950408889634f, -f.x)));
+      if (neg) { p0 = -p0; p1 = -p1; }
       if (own) {
         const int k = c + 2 * j;
         if (k == t1) p0 -= f.y;
