@@ -34,7 +34,7 @@ def test_negative_row_weights(m, c, vocab, padded, n_aux):
     ex, ew = torch.autograd.grad(want, [x64, w64])
     rel = lambda a, b: float((a.double() - b).norm() / b.norm())  # noqa: E731
     # logits are bf16 (2^-9), the logits' gradient and the results are rounded once more each; the loss is a sum of both signs
-    scale = sum(float((lse.abs() * a.abs()).sum()) for a in weights)
+    scale = sum(float((lse.detach().abs() * a.abs()).sum()) for a in weights)
     assert abs(float(loss) - float(want)) < 4e-3 * scale
     assert rel(dx, ex) < 1e-2, rel(dx, ex)
     assert rel(dw[:vocab], ew[:vocab]) < 1e-2 and not dw[vocab:].any()

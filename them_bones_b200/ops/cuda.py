@@ -411,9 +411,21 @@ def _mm_tn_write(dy, x, grad):
     COUNTS["gemm"] += 1
 
 
+def _by_address(t) -> bool:
+    """Whether a kernel can stand in for PyTorch operators on ``t`` inside a backward: it has memory of its own (the batched
+    gradients of ``is_grads_batched`` do not) and no graph is being recorded through it (``create_graph``)."""
+    if torch.is_grad_enabled() and t.requires_grad:
+        return False
+    try:
+        t.data_ptr()
+    except RuntimeError:
+        return False
+    return True
+
+
 def _scale_cast(g32, scale, dtype):
     """``g32`` rounded to ``dtype``, times ``scale`` (a device scalar), rounded again."""
-    if dtype != BF16 or g32.numel() % 8:
+    if dtype != BF16 or g32.numel() % 8 or not _by_address(scale):
         return g32.to(dtype) * scale.to(dtype)
     out = torch.empty(g32.shape, dtype=dtype, device=g32.device)
     L.call("bones_scale_cast", L.ptr(g32), L.ptr(_c(scale.float())), L.ptr(out), _L(g32.numel()), L.stream())
