@@ -522,11 +522,14 @@ def _lmhead_nll(x, w, targets, vocab, cap):
     m = x2.shape[0]
     tg = _c(targets).view(-1).to(torch.int64)
     nll, z = torch.empty(m, dtype=torch.float32, device=x.device), torch.empty(m, dtype=torch.float32, device=x.device)
-    part = torch.empty(-(-w.shape[0] // 256) * 2, m, dtype=torch.float32, device=x.device)
+    # the partial sums are 2 KB a row at 65536 columns: in blocks of rows, as the logits of a training step are
+    part = torch.empty(-(-w.shape[0] // 256) * 2 * min(LOSS_ROWS, m), dtype=torch.float32, device=x.device)
     null = L.ptr(None)
-    _logits_stats(x2, w, None, vocab, cap, part, tg, z)
-    L.call("bones_ce_finish", L.ptr(part), _I(part.shape[0]), _I(m), null, _L(0), L.ptr(z), L.ptr(tg), _I(vocab), _F(cap), L.ptr(nll), null, null, null,
-           _F(1.0), null, null, null, null, null, L.stream())
+    for r0 in range(0, m, LOSS_ROWS):
+        r1 = min(m, r0 + LOSS_ROWS)
+        _logits_stats(x2[r0:r1], w, None, vocab, cap, part, tg[r0:r1], z[r0:r1])
+        L.call("bones_ce_finish", L.ptr(part), _I(-(-w.shape[0] // 256) * 2), _I(r1 - r0), null, _L(0), L.ptr(z[r0:r1]), L.ptr(tg[r0:r1]), _I(vocab),
+               _F(cap), L.ptr(nll[r0:r1]), null, null, null, _F(1.0), null, null, null, null, null, L.stream())
     COUNTS["lmhead_loss"] += 1
     return nll
 
