@@ -6,6 +6,7 @@ import os
 
 import torch
 
+from . import COUNTS
 from . import _lib as L
 
 _I, _L, _F = ctypes.c_int, ctypes.c_longlong, ctypes.c_float
@@ -15,8 +16,9 @@ _IMPL = os.environ.get("BONES_ATTN_BWD", "split")
 
 
 # The dK / dV kernel leaves dS for the dQ kernel (32 KB per pair of 128-token tiles) while that scratch stays below this, 2 % of the
-# device, and can be had; otherwise the dQ kernel computes S, P and dP again.  It is given back when the call returns.  With it the two
-# kernels take 398 instead of 486 us at 16 x 2048 tokens, 10 heads of 128 (0.71 GB); the gain per pair does not depend on the size.
+# device, and can be had; otherwise the dQ kernel computes S, P and dP again, which gives the same bits.  It is given back when the
+# call returns.  With it the two kernels take 398 instead of 486 us at 16 x 2048 tokens, 10 heads of 128 (0.71 GB); the gain per pair
+# does not depend on the size.
 DS_LIMIT = 4 << 30
 
 
@@ -26,8 +28,24 @@ def ds_tiles(t: int, window: int) -> int:
     return n * (n + 1) // 2 if w <= 0 or n <= w else w * (w + 1) // 2 + (n - w) * w
 
 
+# From this size on the scratch is the largest allocation of the call (dqkv takes a third of it at 2048 tokens), and whether it
+# fits is asked first: an allocation that fails makes the allocator give back all it has cached, layer after layer on a device that
+# is nearly full.  The question takes about 70 us of host time (130 where the device itself has no room).
+DS_ASK = 256 << 20
+
+
+def _fits(nbytes, device) -> bool:
+    if torch.cuda.is_current_stream_capturing():         # a graph's memory comes from its own pool
+        return True
+    free = torch.cuda.mem_get_info(device)[0]
+    if nbytes <= free:
+        return True
+    stats = torch.cuda.memory_stats(device)
+    return nbytes <= free + stats["reserved_bytes.all.current"] - stats["allocated_bytes.all.current"]
+
+
 def _ds_scratch(nbytes, device):
-    if nbytes > DS_LIMIT:
+    if nbytes > DS_LIMIT or nbytes >= DS_ASK and not _fits(nbytes, device):
         return None
     try:
         return torch.empty(nbytes, dtype=torch.uint8, device=device)
@@ -57,6 +75,7 @@ def backward(dy, qkv2, qk, y, lse, cos, sin, ds, b, t, n_head, head_dim, scale, 
         stats = torch.empty(n + 2, dtype=torch.float32, device=dev)
         dqk = torch.empty(m, 2 * a, dtype=torch.bfloat16, device=dev)
         scratch = _ds_scratch(b * n_head * ds_tiles(t, window) * 32768, dev)
+        COUNTS["attention_dq_again" if scratch is None else "attention_dq_stored"] += 1
         # dV goes straight into its third of dqkv, rows 3a apart
         L.call("bones_attention_bwd", dy2.data_ptr(), qkv2.data_ptr(), qk.data_ptr(), y.data_ptr(), lse.data_ptr(), cos.data_ptr(), sin.data_ptr(),
                0 if ds is None else ds.data_ptr(), stats.data_ptr(), stats.data_ptr() + 4 * n, 0 if scratch is None else scratch.data_ptr(), dqk.data_ptr(),
