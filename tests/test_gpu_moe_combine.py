@@ -54,3 +54,20 @@ def test_any_number_of_choices(n, k, c):
     wdy = torch.zeros(slots + 1, c, device="cuda", dtype=torch.float64)
     wdy.index_add_(0, slot.reshape(-1), (gates.detach().double()[..., None] * dout.double()[:, None]).reshape(-1, c))
     assert rel(dg, wdg) < 1e-5 and rel(dy, wdy[:slots]) < 4e-3
+
+
+def test_gradient_of_the_residual_alone():
+    """Where only the residual is asked for, its gradient is the incoming one, in every form that an addition takes."""
+    from them_bones_b200 import ops
+    from them_bones_b200.ref import functional as RF
+    slot, tok = RF.moe_slots(torch.randint(0, 4, (12, 1), device="cuda"), 1, 12, 4, 12)
+    ys, res, dout = (torch.randn(n, 64, device="cuda").bfloat16() for n in (48, 12, 12))
+    res.requires_grad_(True)
+    gates = torch.rand(12, 1, device="cuda", requires_grad=True)
+    out = ops.moe_combine(ys, slot, gates, res, tok)
+    (g,) = torch.autograd.grad(out, res, dout, retain_graph=True)
+    assert torch.equal(g, dout)
+    (g,) = torch.autograd.grad(out, res, torch.stack([dout, 2 * dout]), is_grads_batched=True, retain_graph=True)
+    assert torch.equal(g, torch.stack([dout, 2 * dout]))
+    dgates, g = torch.autograd.grad(out, [gates, res], dout)
+    assert torch.equal(g, dout) and dgates.shape == gates.shape

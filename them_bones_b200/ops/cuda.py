@@ -823,8 +823,10 @@ class _CombineFn(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, dout):
+        if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[2]):         # the residual's alone: an addition's
+            return None, None, None, dout, None
         ys, slot, g32, tok = ctx.saved_tensors
-        dout = _c(dout)
+        residual_grad, dout = dout if ctx.has_res else None, _c(dout)
         if tok is None:              # the token in each slot, where the caller did not have it
             n_slots = ys.shape[0]
             s = torch.where((slot < 0) | (slot > n_slots), n_slots, slot).view(-1)
@@ -834,7 +836,7 @@ class _CombineFn(torch.autograd.Function):
         dg = torch.zeros_like(g32)
         L.call("bones_moe_combine_bwd", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(tok), L.ptr(dout), L.ptr(dys), L.ptr(dg), _I(slot.shape[0]),
                _I(ys.shape[1]), _I(slot.shape[1]), _L(ys.shape[0]), L.stream())
-        return dys, None, dg, (dout if ctx.has_res else None), None
+        return dys, None, dg, residual_grad, None
 
 
 def moe_combine(ys, slot, gates, residual=None, tok=None):
