@@ -56,18 +56,25 @@ def test_any_number_of_choices(n, k, c):
     assert rel(dg, wdg) < 1e-5 and rel(dy, wdy[:slots]) < 4e-3
 
 
-def test_gradient_of_the_residual_alone():
-    """Where only the residual is asked for, its gradient is the incoming one, in every form that an addition takes."""
+def test_gradients_that_have_no_address():
+    """Batched gradients, and gradients that are recorded (``create_graph``): the residual's is the incoming one, as an addition's,
+    and the others are those of the kernel."""
     from them_bones_b200 import ops
     from them_bones_b200.ref import functional as RF
-    slot, tok = RF.moe_slots(torch.randint(0, 4, (12, 1), device="cuda"), 1, 12, 4, 12)
-    ys, res, dout = (torch.randn(n, 64, device="cuda").bfloat16() for n in (48, 12, 12))
-    res.requires_grad_(True)
-    gates = torch.rand(12, 1, device="cuda", requires_grad=True)
+    slot, tok = RF.moe_slots(torch.rand(12, 4, device="cuda").topk(2, dim=1).indices, 1, 12, 4, 3)
+    ys, res, dout = (torch.randn(n, 64, device="cuda").bfloat16() for n in (12, 12, 12))
+    ys.requires_grad_(True), res.requires_grad_(True)
+    gates = torch.rand(12, 2, device="cuda", requires_grad=True)
     out = ops.moe_combine(ys, slot, gates, res, tok)
-    (g,) = torch.autograd.grad(out, res, dout, retain_graph=True)
-    assert torch.equal(g, dout)
     (g,) = torch.autograd.grad(out, res, torch.stack([dout, 2 * dout]), is_grads_batched=True, retain_graph=True)
     assert torch.equal(g, torch.stack([dout, 2 * dout]))
-    dgates, g = torch.autograd.grad(out, [gates, res], dout)
-    assert torch.equal(g, dout) and dgates.shape == gates.shape
+    plain = torch.autograd.grad(out, [ys, gates, res], dout, retain_graph=True)
+    batched = torch.autograd.grad(out, [ys, gates, res], torch.stack([dout, -dout]), is_grads_batched=True, retain_graph=True)
+    recorded = torch.autograd.grad(out, [ys, gates, res], dout.clone().requires_grad_(True), create_graph=True, retain_graph=True)
+    rel = lambda a, b: float((a.float() - b.float()).norm() / b.float().norm())  # noqa: E731
+    for p, b, r in zip(plain, batched, recorded):
+        assert rel(b[0], p) < 2 ** -8 and rel(b[1], -p) < 2 ** -8 and rel(r.detach(), p) < 2 ** -8 and r.requires_grad       # one bf16 rounding each
+    with torch.no_grad():
+        fixed = ys.detach()
+    (g,) = torch.autograd.grad(ops.moe_combine(fixed, slot, gates.detach(), res, tok), res, dout)
+    assert torch.equal(g, dout)

@@ -826,12 +826,21 @@ class _CombineFn(torch.autograd.Function):
         if not (ctx.needs_input_grad[0] or ctx.needs_input_grad[2]):         # the residual's alone: an addition's
             return None, None, None, dout, None
         ys, slot, g32, tok = ctx.saved_tensors
-        residual_grad, dout = dout if ctx.has_res else None, _c(dout)
+        residual_grad = dout if ctx.has_res else None
+        n_slots = ys.shape[0]
+        s = torch.where((slot < 0) | (slot > n_slots), n_slots, slot) if tok is None or not _by_address(dout) else None
         if tok is None:              # the token in each slot, where the caller did not have it
-            n_slots = ys.shape[0]
-            s = torch.where((slot < 0) | (slot > n_slots), n_slots, slot).view(-1)
             tok = torch.full((n_slots + 1,), slot.shape[0], dtype=torch.int64, device=ys.device)
-            tok.scatter_(0, s, torch.arange(slot.shape[0], device=ys.device).repeat_interleave(slot.shape[1]))
+            tok.scatter_(0, s.view(-1), torch.arange(slot.shape[0], device=ys.device).repeat_interleave(slot.shape[1]))
+        if not _by_address(dout):    # what is wanted of it is not known here: perhaps only the residual's, an addition's
+            yp = torch.cat([ys, ys.new_zeros(1, ys.shape[1])]).float()
+            d = dout.float()
+            dg = torch.stack([(yp.index_select(0, s[:, k]) * d).sum(-1) for k in range(s.shape[1])], -1) if s.shape[1] else None
+            gate = torch.zeros(n_slots + 1, device=ys.device).scatter_(0, s.view(-1), g32.view(-1))[:n_slots, None]
+            used = torch.zeros(n_slots + 1, dtype=torch.bool, device=ys.device).scatter_(0, s.view(-1), True)[:n_slots, None]
+            rows = d.index_select(0, tok[:n_slots].clamp(0, slot.shape[0] - 1))
+            return torch.where(used, gate * rows, 0.0).to(ys.dtype), None, dg, residual_grad, None
+        dout = _c(dout)
         dys = torch.empty_like(ys)
         dg = torch.zeros_like(g32)
         L.call("bones_moe_combine_bwd", L.ptr(ys), L.ptr(slot), L.ptr(g32), L.ptr(tok), L.ptr(dout), L.ptr(dys), L.ptr(dg), _I(slot.shape[0]),
