@@ -1,4 +1,4 @@
-"""The one-kernel Newton-Schulz iteration against 64 bits and against the launches it replaces, over tile remainders."""
+"""The Newton-Schulz iteration against 64 bits over tile remainders (one kernel, except for two matrices of 400 x 272: batched launches)."""
 import pytest
 import torch
 

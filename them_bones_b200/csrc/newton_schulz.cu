@@ -501,7 +501,10 @@ int bones_newton_schulz(const void* x0, void* x1, void* x2, void* g, void* b, in
   // a contraction of s, a tile takes its contraction and about one more until its result can be read, and a slot's tiles take
   // `slot`.  X' must also be complete when the matrix's next G comes, n slots after the last one, so with few matrices the lags
   // are what fits (5 matrices of 5120 x 1280: 2 and 3 slots 673 us, 3 and 4 slots 797, 1 and 2 slots 715, none 1697).
-  const float kg = (float)(p.tall ? r : c) / (float)p.s, slot = ((float)p.tri * (kg + 1.0f) + (float)p.rect) / 74.0f;
+  int dev = 0, sms = 0;
+  BONES_CHECK(cudaGetDevice(&dev));
+  BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const float kg = (float)(p.tall ? r : c) / (float)p.s, slot = ((float)p.tri * (kg + 1.0f) + (float)p.rect) / (float)(sms / 2);
   auto up = [](float v) { const int i = (int)v; return i + ((float)i < v ? 1 : 0); };
   p.lag_b = up((kg + 1.0f) / slot);
   p.lag_x = p.lag_b + up(2.0f / slot);
@@ -535,9 +538,6 @@ int bones_newton_schulz(const void* x0, void* x1, void* x2, void* g, void* b, in
     BONES_CHECK(cudaFuncSetAttribute(newton_schulz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_done = true;
   }
-  int dev = 0, sms = 0;
-  BONES_CHECK(cudaGetDevice(&dev));
-  BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   BONES_CHECK(cudaMemsetAsync(scratch, 0, sizeof(int) * (1 + 3 * (size_t)steps * n), (cudaStream_t)stream));
   const int pairs = p.total < sms / 2 ? p.total : sms / 2;
   newton_schulz_kernel<<<2 * pairs, NS_THREADS, smem, (cudaStream_t)stream>>>(maps, p);

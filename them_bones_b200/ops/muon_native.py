@@ -3,8 +3,9 @@
 Polar-Express iteration (coefficients and tall/wide forms: reference round2/source/train.py:11755-11761, :11880-11888;
 its on-chip kernel: round2/source/kernels/nki_nsk.py): tall matrices iterate on ``G = X^T X`` and wide ones on
 ``G = X X^T``; ``B = b G + c G^2``; ``X' = a X + X B`` (tall) or ``a X + B X`` (wide).  ``G`` and ``B`` are symmetric, so
-every product is issued as a K-major or MN-major operand view of the same buffers (no transposes): three batched GEMM
-launches per iteration with the ``alpha*acc + beta*R`` epilogue doing the polynomial.
+every product is issued as a K-major or MN-major operand view of the same buffers (no transposes), either inside one kernel
+for the whole iteration or as three batched GEMM launches per iteration, with the ``alpha*acc + beta*R`` epilogue doing the
+polynomial.
 """
 from __future__ import annotations
 
@@ -17,6 +18,15 @@ from . import COUNTS
 from . import _lib as L
 
 
+def in_one_kernel(k: int, r: int, c: int, steps: int, aligned: bool = True) -> bool:
+    """Whether the whole iteration runs as one kernel over an ordered list of tiles (csrc/newton_schulz.cu): where there are
+    matrices enough to run side by side or so little work that launches are what it costs: 5 x 5120 x 1280 751 -> 657 us, 10 x 1280 x 1280
+    660 -> 524, 20 x 1280 x 1280 1025 -> 841, 4 x 1280 x 1280 327 -> 312, 3 x 1024 x 256 232 -> 183.  One to three large
+    matrices have nobody to hide a product's end behind (2 x 5120 x 1280: 405 us in launches, 536 in one kernel).
+    ``aligned``: the stack begins on 32 bytes."""
+    return r % 16 == 0 and c % 16 == 0 and aligned and 0 < steps <= 8 and k > 0 and (k >= 4 or min(r, c) <= 256)
+
+
 def newton_schulz(x: torch.Tensor, steps: int = 5) -> torch.Tensor:
     """``x [k, r, c]`` bf16, Frobenius-normalised.  Returns the orthogonalised stack (bf16, new tensor)."""
     assert x.dtype == torch.bfloat16 and x.is_contiguous()
@@ -24,22 +34,31 @@ def newton_schulz(x: torch.Tensor, steps: int = 5) -> torch.Tensor:
     if r % 8 or c % 8:       # tiny matrices (a 16 x d router): not worth a tensor-core tile, and below the TMA alignment
         from ..ref.functional import newton_schulz as ns_ref
         return ns_ref(x, steps)
+    if in_one_kernel(k, r, c, steps, x.data_ptr() % 32 == 0):
+        return _one_kernel(x, steps)
+    return _launches(x, steps)
+
+
+def _one_kernel(x, steps):
+    k, r, c = x.shape
+    n = min(r, c)
+    co = POLAR_EXPRESS_COEFFS[:steps]
+    bufs = [torch.empty_like(x), torch.empty_like(x) if len(co) > 1 else x]
+    gb = torch.empty(2, k, n, n, dtype=torch.bfloat16, device=x.device)
+    scratch = torch.empty(1 + 3 * len(co) * k, dtype=torch.int32, device=x.device)
+    flat = (ctypes.c_float * (3 * len(co)))(*[v for t in co for v in t])
+    L.call("bones_newton_schulz", L.ptr(x), L.ptr(bufs[0]), L.ptr(bufs[1]), L.ptr(gb[0]), L.ptr(gb[1]), ctypes.c_int(k), ctypes.c_int(r),
+           ctypes.c_int(c), ctypes.c_int(len(co)), flat, L.ptr(scratch), L.stream())
+    COUNTS["ns_gemm"] += 3 * len(co)
+    COUNTS["ns_kernel"] += 1
+    return bufs[0] if len(co) % 2 else bufs[1]
+
+
+def _launches(x, steps):
+    """Three batched GEMM launches an iteration."""
+    k, r, c = x.shape
     tall = r > c
     n = c if tall else r
-    if r % 16 == 0 and c % 16 == 0 and x.data_ptr() % 32 == 0 and 0 < steps <= 8 and k and (k >= 4 or n <= 256):
-        # the whole iteration as one kernel over an ordered list of tiles (csrc/newton_schulz.cu), where there are matrices enough to
-        # run side by side or so little work that launches are what it costs: 5 x 5120 x 1280 751 -> 657 us, 10 x 1280 x 1280
-        # 660 -> 524, 20 x 1280 x 1280 1025 -> 841, 4 x 1280 x 1280 327 -> 312, 3 x 1024 x 256 232 -> 183.  One to three large
-        # matrices have nobody to hide a product's end behind (2 x 5120 x 1280: 405 us in launches, 536 in one kernel).
-        co = POLAR_EXPRESS_COEFFS[:steps]
-        bufs = [torch.empty_like(x), torch.empty_like(x) if len(co) > 1 else x]
-        gb = torch.empty(2, k, n, n, dtype=torch.bfloat16, device=x.device)
-        scratch = torch.empty(1 + 3 * len(co) * k, dtype=torch.int32, device=x.device)
-        flat = (ctypes.c_float * (3 * len(co)))(*[v for t in co for v in t])
-        L.call("bones_newton_schulz", L.ptr(x), L.ptr(bufs[0]), L.ptr(bufs[1]), L.ptr(gb[0]), L.ptr(gb[1]), ctypes.c_int(k), ctypes.c_int(r),
-               ctypes.c_int(c), ctypes.c_int(len(co)), flat, L.ptr(scratch), L.stream())
-        COUNTS["ns_gemm"] += 3 * len(co)
-        return bufs[0] if len(co) % 2 else bufs[1]
     g = torch.empty(k, n, n, dtype=torch.bfloat16, device=x.device)
     b = torch.empty_like(g)
     cur, nxt = x, torch.empty_like(x)
