@@ -104,6 +104,7 @@ def roles(a):
                                                  "maths_and_copy_along_n": per(lead[21], tiles), "copy_along_m": per(lead[22], tiles),
                                                  "read_back_and_stores": per(lead[23], tiles)}}
     else:
+        from . import attention_bwd as AB
         from . import attention_native as AN
         from ..ref import functional as RF
         if not hasattr(lib, "bones_attn_set_prof"):
@@ -122,12 +123,13 @@ def roles(a):
         dqk = torch.empty(m, 2 * ad, dtype=bf, device="cuda")
         dqkv = torch.empty(m, 3 * ad, dtype=bf, device="cuda")
         dv = dqkv[:, 2 * ad:]
+        ds = AB._ds_scratch(b * h * AB.ds_tiles(t, 0) * 32768, "cuda")          # as the backward has it: dQ from the stored dS
         L.call("bones_attn_bwd_stats", L.ptr(dy), L.ptr(y), L.ptr(lse), L.ptr(stats), L.ptr(counters), I(b), I(t), I(h), I(d), L.stream())
 
         def fn():
             counters.zero_()
             L.call("bones_attn_bwd_split", L.ptr(qk), L.ptr(qkv), L.ptr(dy), L.ptr(stats), L.ptr(counters), L.ptr(dqk), L.ptr(dv), LL(3 * ad),
-                   L.ptr(None), L.ptr(None), I(b), I(t), I(h), I(d), F(scale), I(0), L.stream())
+                   L.ptr(ds), L.ptr(None), I(b), I(t), I(h), I(d), F(scale), I(0), L.stream())
 
         ms = timeit(fn, a.iters, a.warmup, not a.no_flush)
         lib.bones_attn_set_prof(ctypes.c_void_p(prof.data_ptr()))
@@ -137,7 +139,7 @@ def roles(a):
         pr = prof.view(sms, 32).double().mean(0)
         tiles = float(pr[8])
         per = lambda v: round(float(v) / max(tiles, 1.0))  # noqa: E731
-        out = {"what": a.what, "shape": [b, t, h, d], "ms_both_kernels": ms, "dkv_tiles_per_cta": tiles,
+        out = {"what": a.what, "shape": [b, t, h, d], "ms_both_kernels": ms, "dq_from_stored_ds": ds is not None, "dkv_tiles_per_cta": tiles,
                "dkv_mma_warp_clocks_per_tile": {"total": per(pr[7]), "wait_item_kv": per(pr[0]), "wait_q": per(pr[1]), "wait_do": per(pr[2]),
                                                 "wait_p_ready": per(pr[3]), "wait_acc_free": per(pr[4]), "wait_ds_ready": per(pr[5]),
                                                 "issue": per(pr[6])},
