@@ -400,14 +400,7 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
     if ((l16 & 3) == 0) prefetch_l2(((l16 & 4) ? vp : kp) - l16 * 8 + (l16 >> 3) * 64 + (long long)n * A);
   }
   pdl_wait();
-  if (doc_start) {
-    const int now = max(ld_relaxed(doc_start + b), band);
-    if (now != lo) {                           // a document begins here
-      lo = now;
-      j = lo + warp * 2 + (lane >> 4);
-      fetch(j);
-    }
-  }
+  const int now = doc_start ? max(ld_relaxed(doc_start + b), band) : band;      // on its way while q, k and v are handled
   if (warp < 3) {
     const __nv_bfloat16* src = qkv + (long long)b * 3 * A + warp * A + h * 128;
     float2 x1 = unpack_bf16(*reinterpret_cast<const uint32_t*>(src + 2 * lane));
@@ -431,6 +424,11 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
       *reinterpret_cast<uint32_t*>(dst + 2 * lane) = w1;
       *reinterpret_cast<uint32_t*>(dst + 64 + 2 * lane) = w2;
     }
+  }
+  if (now != lo) {                             // a document begins here
+    lo = now;
+    j = lo + warp * 2 + (lane >> 4);
+    fetch(j);
   }
   __syncthreads();
   float q[8], acc[8], l = 0.f;
