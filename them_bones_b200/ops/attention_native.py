@@ -68,10 +68,10 @@ class _AttnFn(torch.autograd.Function):
     def forward(ctx, qkv, cos, sin, n_head, head_dim, scale, doc_start, window):
         b, t, _ = qkv.shape
         a = n_head * head_dim
-        # a tensor may begin anywhere in its storage (one sequence of a packed batch)
+        # a tensor may begin anywhere in its storage (one sequence of a packed batch); document starts are read one by one
         qkv2 = _aligned(qkv).view(b * t, -1)
         cos, sin = _aligned(cos.float()), _aligned(sin.float())
-        ds = _aligned(doc_start.to(torch.int32)) if doc_start is not None else None
+        ds = doc_start.to(torch.int32).contiguous() if doc_start is not None else None
         dev = qkv2.device
         qk = torch.empty(b * t, 2 * a, dtype=qkv2.dtype, device=dev)
         y = torch.empty(b, t, a, dtype=qkv2.dtype, device=dev)
