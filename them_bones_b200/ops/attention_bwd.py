@@ -29,19 +29,20 @@ def ds_tiles(t: int, window: int) -> int:
 
 
 # From this size on the scratch is the largest allocation of the call (dqkv takes a third of it at 2048 tokens), and whether it
-# fits is asked first: an allocation that fails makes the allocator give back all it has cached, layer after layer on a device that
-# is nearly full.  The question takes about 70 us of host time (130 where the device itself has no room).
+# fits is looked up first: an allocation that fails makes the allocator give back all it has cached, layer after layer on a device
+# that is nearly full.  The allocator's own figures, about 60 us of host time, leave DS_OTHERS for what it does not know of.  Asking the
+# driver (cudaMemGetInfo) takes as long on a quiet machine and took milliseconds on a busy one.
 DS_ASK = 256 << 20
+DS_OTHERS = 2 << 30
 
 
 def _fits(nbytes, device) -> bool:
     if torch.cuda.is_current_stream_capturing():         # a graph's memory comes from its own pool
         return True
-    free = torch.cuda.mem_get_info(device)[0]
-    if nbytes <= free:
-        return True
     stats = torch.cuda.memory_stats(device)
-    return nbytes <= free + stats["reserved_bytes.all.current"] - stats["allocated_bytes.all.current"]
+    reserved = stats["reserved_bytes.all.current"]
+    cached, unused = reserved - stats["allocated_bytes.all.current"], torch.cuda.get_device_properties(device).total_memory - reserved
+    return nbytes <= max(cached, unused - DS_OTHERS)
 
 
 def _ds_scratch(nbytes, device):
