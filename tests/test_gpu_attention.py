@@ -121,8 +121,8 @@ def test_attention_head_dim_64(b, t, h, window, docs):
 
 
 def test_attention_ragged_length_is_padded_and_unsupported_shapes_raise():
-    """The operator layer pads a length that is not a multiple of 128 (scoring, cache-free decoding) and raises --
-    rather than taking a library path -- for what the kernels do not cover."""
+    """The kernels take a length that is not a multiple of 128 (scoring, cache-free decoding) as it is -- only the single-kernel
+    backward has it padded -- and the operator layer raises, rather than taking a library path, for what they do not cover."""
     from them_bones_b200 import ops
     from them_bones_b200.ref import functional as RF
     b, t, h, d = 2, 200, 2, 128

@@ -53,7 +53,7 @@ def test_both_routes_agree(monkeypatch, b, t, h, d, window, docs):
     assert torch.isfinite(stored).all()
     a = h * d
     assert torch.equal(stored[..., a:], again[..., a:])            # dK, dV come from the same kernel
-    # dQ: two fp32 sums of the same products, whose S and dP may differ in the last bit of the exponential: bf16 roundings of dS
-    # (2^-9 each, in few elements) and of dQ
+    # dQ: two fp32 sums of the same products; were S or dP to differ in a last bit, bf16 roundings of dS would (2^-9 each, in few
+    # elements), and those of dQ.  (They do not: test_gpu_attention_scratch.py.)
     err = (stored[..., :a].float() - again[..., :a].float()).norm() / again[..., :a].float().norm().clamp_min(1e-12)
     assert t == 1 or float(err) < 2 ** -8, float(err)

@@ -2,9 +2,9 @@
 // by half tile.  What remains is the rows' log-sum-exp and loss (8 MB of partial sums for 4096 rows of 65536 logits) and,
 // for training, one element-wise pass that turns the logits into their gradient in place.
 //
-// Bound by the pass over the logits: 0.54 GB in and out per 4096 rows, 164 us at the copy rate, 156 measured (and 8 us for the
-// rows).  Two passes over a row kept in
-// shared memory (sum of exponentials, then gradient: `softcap_ce_row_kernel`, still used with label smoothing) took 327 us,
+// Bound by the pass over the logits: 0.54 GB read and 0.54 GB written per 4096 rows of 65536, 164 us at the copy rate.  Measured 164 us
+// with L2 flushed before and 160 right behind the GEMM, whose last logits are still in L2; and 12 us for the rows.  Two passes over a
+// row kept in shared memory (sum of exponentials, then gradient: `softcap_ce_row_kernel`, still used with label smoothing) took 327 us,
 // because a row's read, its two exponential passes and its write followed one another in the one CTA an SM has room for.  The
 // element-wise pass has no dependence on the rest of the row: small CTAs, many to an SM.
 #include "common.cuh"

@@ -86,13 +86,6 @@ def mm_tn_acc(dy, x, grad, alpha=1.0, push_ptr=None):
     return grad
 
 
-# A weight gradient that autograd gets back (no slab to accumulate into) is written in bf16 by the GEMM itself once it has so
-# many 256 x 256 tiles that the fp32 form would not split its contraction either (4 x 74 CTA pairs, the GEMM's own rule): the
-# same accumulator, rounded once, without the fp32 zero fill, the read-modify-write and the cast.  For 16 experts of
-# 2560 x 1280 a layer spent 400 us on them (4 plain GEMMs 731 -> 479 us, fills and casts 158 us less).
-WGRAD_WHOLE_TILES = 296
-
-
 def _wgrad(dy2, x2, ws):
     """Weight gradient for one or several row-adjacent weights.  Returns the tuple autograd expects."""
     grads = [getattr(w, "main_grad", None) for w in ws]
@@ -852,6 +845,14 @@ def moe_combine(ys, slot, gates, residual=None, tok=None):
     if residual is not None and (residual.dtype != ys.dtype or residual.data_ptr() % 16):
         return _CombineFn.apply(_c(ys), _c(slot), gates, None, tok) + residual
     return _CombineFn.apply(_c(ys), _c(slot), gates, _c(residual) if residual is not None else None, tok)
+
+
+# A weight gradient of the experts, or of the loss head, that autograd gets back (no slab to accumulate into, as the trainer has) is
+# written whole by the GEMM once it has so many 256 x 256 tiles that accumulating would not split its contraction either (4 x 74 CTA
+# pairs, the GEMM's own rule): experts in bf16, the same accumulator rounded once, without the fp32 zero fill, the read-modify-write
+# and the cast; the head's first block of rows in fp32, without the zero fill.  For 16 experts of 2560 x 1280 a layer spent 400 us on
+# them (4 plain GEMMs 731 -> 479 us, fills and casts 158 us less).
+WGRAD_WHOLE_TILES = 296
 
 
 class _ExpertsFn(torch.autograd.Function):
