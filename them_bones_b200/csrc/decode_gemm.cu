@@ -19,22 +19,12 @@
 //     to choose what it requests early, and reads it again behind the wait.)
 // Warp 0 issues the TMA loads, warp 1 the MMAs, the others run the epilogue.
 //
-// One step of the 20-layer, 1280-wide model at batch 64: 103 kernels and 0.81 ms where 250 kernels took 1.41 ms.  Of 0.90 ms before,
-// the earlier start took 0.01, the rows requested ahead (residual before the accumulator, cache rows into L2) and clusters of 16
-// for the ten-tile projections 0.07, two CTAs a tile for the others (rule in utils/decode.py) 0.02.  What is left is
-// a chain of latencies: per projection about 1.6 us from the previous kernel's end to this one's start, 1.5 to 4 us until
-// the accumulator is complete, 1.2 + 1 us for the exchange and its barrier, 0.7 to 1.3 us of epilogue.  Measured without gain:
-// bulk prefetches of the next projection's weights into L2 (the issuing warp stalls for 4 us, 1.6 % a step).
-#include "common.cuh"
+// Up to 64 sequences the layers' projections run on decode_rows.cu, whose tiles exchange no partial sums or small ones; this kernel has the
+// head and more sequences.  What bounds it is a chain of latencies: per projection about 1.1 us from the previous kernel's end to this
+// one's start, 1.5 to 4 us until the accumulator is complete, 1.3 to 2.9 us for the exchange, 0.7 to 1.3 us of epilogue.
+#include "decode_common.cuh"
 
 namespace bones {
-
-enum DecEpi : int {
-  DEC_SCALE = 0,     // bf16( r acc )
-  DEC_RELU2 = 1,     // bf16( relu(r acc)^2 )
-  DEC_RES = 2,       // x = bf16( acc + res ), then with x0: bf16( a x + b x0 ); squares' sums of what is stored
-  DEC_SOFTCAP = 3,   // bf16( cap tanh(r acc / cap) )
-};
 
 struct DecGemmParams {
   int N, b, KB;
@@ -50,29 +40,6 @@ struct DecGemmParams {
   int* err;
 };
 
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ uint32_t cluster_rank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ uint32_t cluster_size() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(r));
-  return r;
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-__device__ __forceinline__ uint32_t map_to_rank(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void st_cluster_v4(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared::cluster.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
 // Where the partial sums of output column n, tokens 4 u .. 4 u + 3 of `1 << lc`, of cluster rank s stand in their owner's buffer
 // (16-byte units; the unit index is turned by the row so that eight lanes of a warp hit different banks).
 __device__ __forceinline__ uint32_t red_unit(int s, int n, int u, int lc) {
@@ -292,22 +259,6 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   }
 }
 
-static int dec_launch_attrs(cudaLaunchAttribute* at, int cluster, int pdl) {
-  int n = 0;
-  if (cluster > 1) {
-    at[n].id = cudaLaunchAttributeClusterDimension;
-    at[n].val.clusterDim.x = (unsigned)cluster;
-    at[n].val.clusterDim.y = at[n].val.clusterDim.z = 1;
-    ++n;
-  }
-  if (pdl) {
-    at[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[n].val.programmaticStreamSerializationAllowed = 1;
-    ++n;
-  }
-  return n;
-}
-
 template <int NB, int EPI>
 static int launch_dec_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const DecGemmParams& p, int S, int pdl, cudaStream_t stream) {
   using G = DgGeom<NB>;
@@ -345,9 +296,14 @@ static int launch_dec_gemm_epi(int epi, const CUtensorMap& tw, const CUtensorMap
 
 // ---------------------------------------------------------------------------------------------------------------
 // Between the projections: RoPE + QK-norm of the new token, cache append and attention over the cache, one CTA per
-// (head, sequence).  Sixteen lanes share a key (8 dims each), a warp handles two keys per step and the CTA sixteen (few registers
-// a thread, so that the 640 CTAs of 64 sequences x 10 heads run in one wave); the loads of the next step (and of the first one,
-// before the new token's q is ready) are in flight while a step is computed.
+// (head, sequence).  Sixteen lanes share a key (8 dims each), a lane has U keys a round: the keys' loads of the next round go out as soon
+// as this round's scores are computed, the values' as soon as its sums are, so 2 U loads a thread are in flight nearly all the time.  The
+// scores of a lane's keys are folded across the sixteen lanes together (four keys: five shuffles, and four to hand the weights back;
+// one key after the other takes sixteen), and a weight is computed by 16 / U lanes instead of sixteen.
+// U = 4 keeps 64 keys and values a CTA in flight and takes 64 registers, so an SM holds four CTAs; above that U = 2 (48 registers, five
+// CTAs), for 640 CTAs of 64 sequences x 10 heads in one wave.  Six layers, 1280 wide, us a step at position 64 / 256 / 1000, with one key a
+// lane in flight and with these: batch 4 194 / 239 / 422 -> 190 / 213 / 292; batch 32 (U = 4) 208 / 263 / 465 -> 205 / 239 / 352, with U = 2
+// 207 / 250 / 400; batch 64 (U = 2) 225 / 295 / 525 -> 222 / 277 / 466, with U = 4 231 / 277 / 465.
 // The fixed soft-max shift of the training kernels applies (q and k are RMS-normalised).
 // ---------------------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void unpack8(const uint4& u, float* f) {
@@ -365,13 +321,17 @@ __device__ __forceinline__ int ld_relaxed(const int* p) {      // from L2: an ea
 }
 __device__ __forceinline__ void st_relaxed(int* p, int v) { asm volatile("st.relaxed.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory"); }
 __device__ __forceinline__ void prefetch_l2(const void* a) { asm volatile("prefetch.global.L2 [%0];" ::"l"(a)); }
-__global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
+constexpr int kDaWarps = 8;
+template <int U, int CTAS>
+__global__ void __launch_bounds__(32 * kDaWarps, CTAS) decode_attn_step_kernel(const __nv_bfloat16* __restrict__ qkv, const float* __restrict__ cosT,
                                                                   const float* __restrict__ sinT, __nv_bfloat16* kcache, __nv_bfloat16* vcache,
                                                                   const int* pos_ptr, const int* doc_start, __nv_bfloat16* __restrict__ y, int H,
                                                                   int Tmax, float scale, int window_tiles) {
+  static_assert(U == 2 || U == 4, "the fold of the scores");
+  constexpr int NW = kDaWarps, ROUND = 2 * U * NW;            // keys of the CTA in a round
   __shared__ __align__(16) __nv_bfloat16 s_new[3][128];
-  __shared__ __align__(16) float s_acc[8][128];
-  __shared__ float s_l[8];
+  __shared__ __align__(16) float s_acc[NW][128];
+  __shared__ float s_l[NW];
   pdl_launch();
   const int h = blockIdx.x, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, l16 = lane & 15;
@@ -386,18 +346,23 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
   int lo = doc_start ? max(ld_relaxed(doc_start + b), band) : band;
   const int A = H * 128;
   const __nv_bfloat16 *kp = kcache + ((long long)b * Tmax * H + h) * 128 + l16 * 8, *vp = vcache + ((long long)b * Tmax * H + h) * 128 + l16 * 8;
-  uint4 k, v;
-  auto fetch = [&](int j) {                    // keys before the new one come from the cache
-    if (j < pos) {
-      k = *reinterpret_cast<const uint4*>(kp + (long long)j * A);
-      v = *reinterpret_cast<const uint4*>(vp + (long long)j * A);
-    }
+  uint4 k[U], v[U];
+  // key u of this lane in the round that begins at j: j + 2 u; keys before the new one come from the cache
+  auto fetch = [&](uint4* to, const __nv_bfloat16* from, int j) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (j + 2 * u < pos) to[u] = *reinterpret_cast<const uint4*>(from + (long long)(j + 2 * u) * A);
   };
-  int j = lo + warp * 2 + (lane >> 4);
-  fetch(j);
+  int j = lo + warp * 2 * U + (lane >> 4);
+  fetch(k, kp, j);
+  fetch(v, vp, j);
   // the cache holds earlier steps' keys: the next ones come to L2 while the projection before this kernel still runs
-  for (int i = 1, n = j + 16; i < 8 && n < pos; ++i, n += 16) {
-    if ((l16 & 3) == 0) prefetch_l2(((l16 & 4) ? vp : kp) - l16 * 8 + (l16 >> 3) * 64 + (long long)n * A);
+  if ((l16 & 3) == 0) {
+    for (int n = j + ROUND; n < min(pos, lo + 128); n += ROUND) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (n + 2 * u < pos) prefetch_l2(((l16 & 4) ? vp : kp) - l16 * 8 + (l16 >> 3) * 64 + (long long)(n + 2 * u) * A);
+    }
   }
   pdl_wait();
   const int now = doc_start ? max(ld_relaxed(doc_start + b), band) : band;      // on its way while q, k and v are handled
@@ -427,8 +392,9 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
   }
   if (now != lo) {                             // a document begins here
     lo = now;
-    j = lo + warp * 2 + (lane >> 4);
-    fetch(j);
+    j = lo + warp * 2 * U + (lane >> 4);
+    fetch(k, kp, j);
+    fetch(v, vp, j);
   }
   __syncthreads();
   float q[8], acc[8], l = 0.f;
@@ -436,29 +402,50 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] = 0.f;
   const float c1 = scale * 1.4426950408889634f, c2 = scale * 128.0f * 1.4426950408889634f;
+  const bool up = (lane & 8) != 0, right = (lane & 4) != 0;
+  const int mine = U == 4 ? 2 * ((up ? 2 : 0) + (right ? 1 : 0)) : (up ? 2 : 0);      // after the fold this lane has the score of key j + mine
 #pragma unroll 1
-  for (int j0 = lo + warp * 2; j0 <= pos; j0 += 16, j += 16) {
-    if (j >= pos) {                            // the new token's own key and value; past it nothing
-      k = *reinterpret_cast<const uint4*>(&s_new[1][l16 * 8]);
-      v = *reinterpret_cast<const uint4*>(&s_new[2][l16 * 8]);
+  for (int j0 = lo + warp * 2 * U; j0 <= pos; j0 += ROUND, j += ROUND) {
+    float s[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      if (j + 2 * u >= pos) {                  // the new token's own key and value; past it nothing
+        k[u] = *reinterpret_cast<const uint4*>(&s_new[1][l16 * 8]);
+        v[u] = *reinterpret_cast<const uint4*>(&s_new[2][l16 * 8]);
+      }
+      float kf[8];
+      unpack8(k[u], kf);
+      float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) { s0 += q[i] * kf[i]; s1 += q[i + 1] * kf[i + 1]; }
+      s[u] = s0 + s1;
     }
-    float kf[8], vf[8];
-    unpack8(k, kf);
-    unpack8(v, vf);
-    fetch(j + 16);
-    float s0 = 0.f, s1 = 0.f;
+    fetch(k, kp, j + ROUND);
+    float r;
+    if (U == 4) {
+      const float t0 = __shfl_xor_sync(0xffffffffu, up ? s[0] : s[U - 2], 8), t1 = __shfl_xor_sync(0xffffffffu, up ? s[1] : s[U - 1], 8);
+      const float r0 = (up ? s[U - 2] : s[0]) + t0, r1 = (up ? s[U - 1] : s[1]) + t1;
+      r = (right ? r1 : r0) + __shfl_xor_sync(0xffffffffu, right ? r0 : r1, 4);
+    } else {
+      r = (up ? s[1] : s[0]) + __shfl_xor_sync(0xffffffffu, up ? s[0] : s[1], 8);
+      r += __shfl_xor_sync(0xffffffffu, r, 4);
+    }
+    r += __shfl_xor_sync(0xffffffffu, r, 2);
+    r += __shfl_xor_sync(0xffffffffu, r, 1);
+    const float w = j + mine <= pos ? exp2f(r * c1 - c2) : 0.f;
+    l += w;
 #pragma unroll
-    for (int i = 0; i < 8; i += 2) { s0 += q[i] * kf[i]; s1 += q[i + 1] * kf[i + 1]; }
-    float s = s0 + s1;
-    s += __shfl_xor_sync(0xffffffffu, s, 1);
-    s += __shfl_xor_sync(0xffffffffu, s, 2);
-    s += __shfl_xor_sync(0xffffffffu, s, 4);
-    s += __shfl_xor_sync(0xffffffffu, s, 8);
-    const float p = j <= pos ? exp2f(s * c1 - c2) : 0.f;
-    l += p;
+    for (int u = 0; u < U; ++u) {
+      const float pu = __shfl_sync(0xffffffffu, w, (lane & 16) | (u * (16 / U)));
+      float vf[8];
+      unpack8(v[u], vf);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) acc[i] += p * vf[i];
+      for (int i = 0; i < 8; ++i) acc[i] += pu * vf[i];
+    }
+    fetch(v, vp, j + ROUND);
   }
+  if (U == 4) l += __shfl_xor_sync(0xffffffffu, l, 4);
+  l += __shfl_xor_sync(0xffffffffu, l, 8);
   l += __shfl_xor_sync(0xffffffffu, l, 16);
 #pragma unroll
   for (int i = 0; i < 8; ++i) acc[i] += __shfl_xor_sync(0xffffffffu, acc[i], 16);
@@ -471,7 +458,7 @@ __global__ void __launch_bounds__(256, 5) decode_attn_step_kernel(const __nv_bfl
   if (threadIdx.x < 128) {
     float o = 0.f, lt = 0.f;
 #pragma unroll
-    for (int w = 0; w < 8; ++w) { o += s_acc[w][threadIdx.x]; lt += s_l[w]; }
+    for (int w = 0; w < NW; ++w) { o += s_acc[w][threadIdx.x]; lt += s_l[w]; }
     y[((long long)b * H + h) * 128 + threadIdx.x] = __float2bfloat16(lt > 0.f ? o / lt : 0.f);
   }
 }
@@ -616,15 +603,20 @@ int bones_decode_gemm(const void* X, const void* W, void* out, int b, int N, int
 
 int bones_decode_attn_step(const void* qkv, const float* cosT, const float* sinT, void* kcache, void* vcache, const int* pos, const int* doc_start,
                            void* y, int B, int H, int Tmax, float scale, int window_tiles, void* stream) {
+  static int sms[64] = {0};
+  int dev = 0;
+  BONES_CHECK(cudaGetDevice(&dev));
+  if (dev < 64 && !sms[dev]) BONES_CHECK(cudaDeviceGetAttribute(&sms[dev], cudaDevAttrMultiProcessorCount, dev));
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[1];
+  const bool four = dev < 64 && (long long)H * B <= 4ll * sms[dev];        // the CTAs of one wave with four keys a lane
   cfg.gridDim = dim3((unsigned)H, (unsigned)B);
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(32 * kDaWarps);
   cfg.stream = (cudaStream_t)stream;
   cfg.attrs = at;
   cfg.numAttrs = (unsigned)dec_launch_attrs(at, 1, 1);
-  return (int)cudaLaunchKernelEx(&cfg, decode_attn_step_kernel, (const __nv_bfloat16*)qkv, cosT, sinT, (__nv_bfloat16*)kcache,
-                                 (__nv_bfloat16*)vcache, pos, doc_start, (__nv_bfloat16*)y, H, Tmax, scale, window_tiles);
+  return (int)cudaLaunchKernelEx(&cfg, four ? decode_attn_step_kernel<4, 4> : decode_attn_step_kernel<2, 5>, (const __nv_bfloat16*)qkv, cosT, sinT,
+                                 (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, pos, doc_start, (__nv_bfloat16*)y, H, Tmax, scale, window_tiles);
 }
 
 int bones_decode_begin(const long long* tok, const int* pos, int* doc_start, long long bos, const void* wte, long long rows, int C,

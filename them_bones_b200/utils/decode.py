@@ -159,6 +159,45 @@ def projection_splits(b, n, k, residual, sms):
     return splits
 
 
+# What a projection brings to L2 ahead of the next one at most: a layer's largest weights with room to spare (13 MB at width 1280); of
+# the head's 168 MB only as much as is read first.
+AHEAD_LIMIT = 16 << 20
+
+
+def rows_plan(b, n, k, sms):
+    """``(columns of a tile, CTAs that share its contraction)`` of a projection on ``csrc/decode_rows.cu``, or None where it does not apply:
+    more than 64 sequences (its MMA has 64 rows), too few or too many columns for one wave.
+
+    A CTA fills an SM's shared memory, so a plan is one wave: at most ``sms`` CTAs, 0.9 of them in clusters of four or more, which leave
+    gaps.  The contraction is shared until a CTA's part is 1536 at most (a chain of 96 MMAs, 2 us) and tiles of 32 columns or more
+    occupy half of the SMs.  Within that, wide tiles (all CTAs read the same rows of X from L2: fewer of them, less traffic), but narrow
+    ones in clusters of four or more, where a CTA's weights and its exchange count for more.  20 layers, 1280 wide, us a step, all else equal:
+    qkv at batch 64 / 40 / 16 / 4 in tiles of 64 637 / 607 / 549 / 528, 48 644 / 607 / 545 / 520, 32 650 / 605 / 560 / 530, 64 by two CTAs
+    654 / 633 / 568 / 523; out 32 by two 636 / 605 / 544 / 520, 16 by one 643 / 593 / 556 / 550; c_fc 64 634 / 597 / 534 / 518, 32 655 / 614 /
+    569 / 543; c_proj 40 by four 634 / 594 / 534 / 517, 64 by four 660 / 597 / 536 / 517, 32 by two 661 / 621 / 560 / 548.
+    """
+    if b > 64 or k % 128:
+        return None
+    for s in (1, 2, 4, 8):
+        if s > k // 128 or (k > 1536 * s and s < 8):
+            continue
+        fit = [nt for nt in (64, 48, 40, 32) if n % nt == 0 and sms // 2 <= n // nt * s <= (sms if s < 4 else int(0.9 * sms))]
+        if fit:
+            return (fit[0] if s < 4 else fit[-1]), s
+    # few columns: the most CTAs with parts of 256 or more (256 wide: 121 us a step of six layers for 150 at batch 64, 107 for 110 at 8)
+    few = [(n // nt * s, -s, nt) for nt in (16, 32, 64) for s in (1, 2, 4, 8) if (s == 1 or k >= 256 * s) and k <= 1536 * s and n // nt * s < sms // 2]
+    return (max(few)[2], -max(few)[1]) if few else None
+
+
+def use_rows(b, c, a, hidden, sms):
+    """Whether the layers' projections run on ``csrc/decode_rows.cu``: all four or none, since two of its CTAs, or one and one of the other
+    kernel's, do not share an SM (2048 wide, ``out`` alone on it: 10 to 15 % slower).  Narrow models with few sequences stay on the
+    other kernel, whose clusters split their short contractions further (512 and 768 wide, up to 16 sequences: 2 to 6 % faster)."""
+    if c < 1024 and b <= 16:
+        return False
+    return all(rows_plan(b, n, k, sms) is not None for n, k in ((3 * a, c), (c, a), (hidden, c), (c, hidden)))
+
+
 class NativeDecoder:
     """One decode step as a CUDA graph over the native kernels: embedding, fused norms, tcgen05 GEMMs, the two decode
     kernels (``csrc/decode.cu``: RoPE + QK-norm + cache append, cached attention), soft-capped logits, arg-max.  The
@@ -200,8 +239,9 @@ class NativeDecoder:
             self.x0, self.xa, self.xb = (torch.empty(b, c, dtype=bf, device=dev) for _ in range(3))
             self.qkv = torch.empty(b, 3 * a, dtype=bf, device=dev)
             self.h = torch.empty(b, cfg.mlp_ratio * c, dtype=bf, device=dev)
-            self.ssq_a, self.ssq_b = (torch.empty(c // 128, b, dtype=f32, device=dev) for _ in range(2))
+            self.ssq_a, self.ssq_b = (torch.empty(c // 16, b, dtype=f32, device=dev) for _ in range(2))
             self.sms = torch.cuda.get_device_properties(dev).multi_processor_count
+            self.rows = use_rows(b, c, a, cfg.mlp_ratio * c, self.sms)
             self.ticket = torch.zeros(1, dtype=torch.int32, device=dev)
             self.last_logits = torch.empty(b, model.lm_head.weight.shape[0], dtype=bf, device=dev)
         elif self.split:
@@ -225,15 +265,25 @@ class NativeDecoder:
                 and all(w.dtype == torch.bfloat16 and w.is_contiguous() and w.data_ptr() % 16 == 0 and w.shape[0] % 128 == 0 and w.shape[1] % 64 == 0 for w in ws)
                 and all(v.dtype == torch.float32 for v in scalars) and model.cos.dtype == torch.float32 and model.sin.dtype == torch.float32)
 
-    def _proj(self, x, w, out, epi, ssq=None, n_ssq=0, res=None, mix=None, ssq_out=None):
-        """One projection of the fused step (``bones_decode_gemm``), its contraction shared as ``projection_splits`` says."""
+    def _proj(self, x, w, out, epi, ssq=None, n_ssq=0, res=None, mix=None, ssq_out=None, nxt=None):
+        """One projection of the fused step, ``nxt`` the weights that it reads next; returns how many partial sums of squares a sequence has in ``ssq_out``."""
         from ..ops import _lib as L
         b, (n, k) = x.shape[0], w.shape
-        splits = projection_splits(b, n, k, res is not None, self.sms)
         x0, ma, mb = (self.x0, mix[0], mix[1]) if mix is not None else (None, None, None)
+        # the head: CTAs that walk its tiles, 0.5 to 1 % of a step from 40 sequences on, as much the other way at 4
+        head = epi == 3
+        plan = None if not self.rows else rows_plan(b, n, k, self.sms) if not head else (64, 1) if b > 16 else None
+        cap = ctypes.c_float(self.model.config.softcap)
+        if plan is not None:
+            nt, splits = plan
+            L.call("bones_decode_rows", L.ptr(x), L.ptr(w), L.ptr(out), _I(b), _I(n), _I(k), _I(nt), _I(splits), _I(self.sms if head else 0), _I(epi), L.ptr(ssq), _I(n_ssq), L.ptr(res),
+                   L.ptr(x0), L.ptr(ma), L.ptr(mb), L.ptr(ssq_out), cap, L.ptr(nxt),
+                   ctypes.c_longlong(0 if nxt is None else min(2 * nxt.numel(), AHEAD_LIMIT)), _I(1), L.stream())
+            return n // nt
+        splits = projection_splits(b, n, k, res is not None, self.sms)
         L.call("bones_decode_gemm", L.ptr(x), L.ptr(w), L.ptr(out), _I(b), _I(n), _I(k), _I(splits), _I(epi), L.ptr(ssq), _I(n_ssq), L.ptr(res),
-               L.ptr(x0), L.ptr(ma), L.ptr(mb), L.ptr(ssq_out), ctypes.c_float(self.model.config.softcap), _I(1),
-               L.stream())
+               L.ptr(x0), L.ptr(ma), L.ptr(mb), L.ptr(ssq_out), cap, _I(1), L.stream())
+        return n // 128
 
     def _step_fused(self):
         """Five kernels a layer (qkv, attention, out, c_fc, c_proj), one before the first and two after the last; the norms,
@@ -241,7 +291,7 @@ class NativeDecoder:
         from ..ops import _lib as L
         model, cache, cfg = self.model, self.cache, self.model.config
         tok, pos, b, c = self.tok, self.pos, self.tok.shape[0], cfg.n_embd
-        tmax, tiles = cache.k.shape[2], c // 128
+        tmax = cache.k.shape[2]
         ds = cache.doc_start if cfg.doc_mask else None
         hs = model.transformer.h
         w = model.transformer.wte.weight
@@ -250,15 +300,15 @@ class NativeDecoder:
         n_ssq = 1
         for i, blk in enumerate(hs):
             at = blk.attn
-            self._proj(self.xa, self.wqkv[i], self.qkv, 0, ssq=self.ssq_a, n_ssq=n_ssq)
+            self._proj(self.xa, self.wqkv[i], self.qkv, 0, ssq=self.ssq_a, n_ssq=n_ssq, nxt=at.c_proj.weight)
             L.call("bones_decode_attn_step", L.ptr(self.qkv), L.ptr(model.cos), L.ptr(model.sin), L.ptr(cache.k[i]), L.ptr(cache.v[i]), L.ptr(pos), L.ptr(ds),
                    L.ptr(self.y), _I(b), _I(at.n_head), _I(tmax), ctypes.c_float(at.scale), _I(at.window // 128), L.stream())
-            self._proj(self.y, at.c_proj.weight, self.xb, 2, res=self.xa, ssq_out=self.ssq_b)
-            self._proj(self.xb, blk.mlp.c_fc.weight, self.h, 1, ssq=self.ssq_b, n_ssq=tiles)
+            n_ssq = self._proj(self.y, at.c_proj.weight, self.xb, 2, res=self.xa, ssq_out=self.ssq_b, nxt=blk.mlp.c_fc.weight)
+            self._proj(self.xb, blk.mlp.c_fc.weight, self.h, 1, ssq=self.ssq_b, n_ssq=n_ssq, nxt=blk.mlp.c_proj.weight)
             nxt = hs[i + 1] if i + 1 < len(hs) else None
             mix = (nxt.resid_lambda, nxt.x0_lambda) if nxt is not None else None
-            self._proj(self.h, blk.mlp.c_proj.weight, self.xa, 2, res=self.xb, mix=mix, ssq_out=self.ssq_a)
-            n_ssq = tiles
+            n_ssq = self._proj(self.h, blk.mlp.c_proj.weight, self.xa, 2, res=self.xb, mix=mix, ssq_out=self.ssq_a,
+                               nxt=self.wqkv[i + 1] if nxt is not None else model.lm_head.weight)
         self._proj(self.xa, model.lm_head.weight, self.last_logits, 3, ssq=self.ssq_a, n_ssq=n_ssq)
         L.call("bones_decode_end", L.ptr(self.last_logits), ctypes.c_longlong(self.last_logits.shape[1]), _I(cfg.vocab_size), L.ptr(pos),
                L.ptr(self.prompt_len), L.ptr(self.out), ctypes.c_longlong(self.out.stride(0)), _I(self.out.shape[1]), L.ptr(tok), L.ptr(self.ticket), _I(b),
