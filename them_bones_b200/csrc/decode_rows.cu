@@ -55,12 +55,6 @@ constexpr int DR_SUMS = 4 * 64 * 4;                   // squares' sums, four par
                : "r"(taddr)                                                                                                 \
                : "memory")
 
-// whether a barrier's phase is complete, without waiting for it
-__device__ __forceinline__ uint32_t mbar_test(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile("{\n.reg .pred p;\nmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-  return ok;
-}
 constexpr int DR_AHEAD = 4096;
 __device__ __forceinline__ void l2_prefetch_bulk(const void* a, uint32_t bytes) {
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(a), "r"(bytes) : "memory");
@@ -176,8 +170,7 @@ decode_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
     int xsl = 0, wsl = 0, it = 0;
     uint32_t xph = 0, wph = 0;
     bool dead = false, ready = false;
-    // A wait takes 100 to 160 clocks although the stage has long landed; two of them are as long as a stage's eight MMAs.  So whether
-    // the next stage is there is asked before this one's MMAs are issued, and the answer read behind them.
+    // Two waits are as long as a stage's eight MMAs: whether the next stage is there is asked before this one's are issued (`mbar_test`).
     for (int tile = first; tile < p.tiles; tile += step, ++it) {
       const int a = it & 1;
       if (it > 1 && !dead) dead = !mbar_wait(tempty(a), ((uint32_t)(it >> 1) & 1u) ^ 1u, abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);

@@ -30,6 +30,8 @@ SIGNATURES = {
     "bones_gemm_bf16": _GEMM + [_I] * 3 + [_P],                     # ..., force_bn, splits, atomic, stream
     "bones_gemm_bf16_pair": _GEMM + [_I] * 2 + [_P],
     "bones_gemm_bf16_auto": _GEMM + [_I] * 2 + [_P],
+    "bones_mlp_bf16_fwd": [_P] * 6 + [_I] * 4 + [_L] * 4 + [_I, _P],     # ..., GEMM_MODE, stream
+    "bones_mlp_bf16_bwd": [_P] * 9 + [_I] * 4 + [_L] * 4 + [_I, _P],
     "bones_attention_fwd": [_P] * 8 + [_I] * 4 + [_F, _I, _P],
     "bones_attention_bwd": [_P] * 13 + [_I] * 4 + [_F, _I, _P],
     "bones_mx2_quant": [_P, _L, _P, _P, _I, _P, _P, _I, _L, _L, _I, _P],
@@ -113,6 +115,7 @@ EPI_BF16, EPI_BF16_RES, EPI_RELU2, EPI_ACC_F32, EPI_MUL_2SQRT, EPI_F32, EPI_F32_
 
 
 PAIR_MODE = os.environ.get("BONES_GEMM_PAIR", "auto")      # auto | 0 | 1
+GEMM_MODE = {"auto": 0, "1": 1}.get(PAIR_MODE, 2)
 
 
 def gemm(a, b, d, *, m, n, k, lda, ldb, ldd, a_major=0, b_major=0, epi=EPI_BF16, r=None, ldr=0, alpha=1.0, beta=1.0,

@@ -86,6 +86,24 @@ def mm_tn_acc(dy, x, grad, alpha=1.0, push_ptr=None):
     return grad
 
 
+def mm_tn(dy, x, out):
+    """``out [N,K] (bf16) = dy[M,N]^T @ x[M,K]`` in one piece: the accumulator is rounded once."""
+    m, n = dy.shape
+    k = x.shape[1]
+    L.gemm(dy, x, out, m=n, n=k, k=m, lda=dy.stride(0), ldb=x.stride(0), ldd=out.stride(0), a_major=1, b_major=1)
+    COUNTS["gemm"] += 1
+    return out
+
+
+def _wgrad_direct(n, k, m):
+    """Whether a weight gradient ``[n, k]`` of ``m`` rows that autograd gets back (no slab to accumulate into) is written as bf16 by the
+    GEMM.  Accumulating in fp32 lets the GEMM split its contraction over idle SMs, but costs a zero fill, a read-modify-write with
+    atomics and a cast.  Those are the longer up to a contraction that grows with the tiles there are to occupy the SMs.  Direct / split, us:
+    5120 x 1280 of 1000 rows 17 / 39, 4096 46 / 56, 8192 86 / 93, 16384 167 / 164; 1280 x 1280 of 2048 15 / 20, 4096 23 / 26, 8192 40 / 40,
+    16384 90 / 56; 256 x 1024 of 2048 13 / 14, 4096 21 / 15."""
+    return 0 < m <= max(2048, 164 * (-(-n // 256)) * (-(-k // 256)))
+
+
 def _wgrad(dy2, x2, ws):
     """Weight gradient for one or several row-adjacent weights.  Returns the tuple autograd expects."""
     grads = [getattr(w, "main_grad", None) for w in ws]
@@ -110,6 +128,12 @@ def _wgrad(dy2, x2, ws):
                 mm_tn_acc(dy2[:, o:o + w.shape[0]], x2, g)
                 o += w.shape[0]
         return tuple(None for _ in ws)
+    if _wgrad_direct(dy2.shape[1], x2.shape[1], dy2.shape[0]) and all(w.dtype == BF16 for w in ws):
+        full = torch.empty(dy2.shape[1], x2.shape[1], dtype=BF16, device=x2.device)
+        mm_tn(dy2, x2, full)
+        if len(ws) == 1:
+            return (full,)
+        return tuple(g.clone() for g in full.split([w.shape[0] for w in ws]))
     full = torch.zeros(dy2.shape[1], x2.shape[1], dtype=torch.float32, device=x2.device)
     mm_tn_acc(dy2, x2, full)
     outs, o = [], 0
@@ -170,9 +194,14 @@ class _MlpFn(torch.autograd.Function):
     def forward(ctx, x, w_fc, w_proj, residual):
         shp = x.shape
         x2 = _c(x).view(-1, shp[-1])
-        h = mm_nt(x2, w_fc, epi=L.EPI_RELU2)
         r2 = _c(residual).view(-1, w_proj.shape[0]) if residual is not None else None
-        y = mm_nt(h, w_proj, epi=L.EPI_BF16_RES if r2 is not None else L.EPI_BF16, r=r2)
+        m, c = x2.shape
+        f, n = w_fc.shape[0], w_proj.shape[0]
+        h, y = torch.empty(m, f, dtype=BF16, device=x.device), torch.empty(m, n, dtype=BF16, device=x.device)
+        L.call("bones_mlp_bf16_fwd", x2.data_ptr(), w_fc.data_ptr(), w_proj.data_ptr(), r2.data_ptr() if r2 is not None else 0, h.data_ptr(), y.data_ptr(),
+               m, c, f, n, x2.stride(0), w_fc.stride(0), w_proj.stride(0), r2.stride(0) if r2 is not None else 0, L.GEMM_MODE, L.raw_stream(),
+               launches=2)
+        COUNTS["gemm"] += 2
         ctx.save_for_backward(x2, h, w_fc, w_proj)
         ctx.has_res, ctx.shp = residual is not None, shp
         ctx.ws = (w_fc, w_proj)
@@ -183,11 +212,21 @@ class _MlpFn(torch.autograd.Function):
     def backward(ctx, dy):
         x2, h, w_fc, w_proj = ctx.saved_tensors
         dy2 = _c(dy).view(-1, w_proj.shape[0])
-        dpre = mm_nn(dy2, w_proj, epi=L.EPI_MUL_2SQRT, r=h)
-        (g_proj,) = _wgrad(dy2, h, (ctx.ws[1],))
-        dx = mm_nn(dpre, w_fc).view(ctx.shp)
-        (g_fc,) = _wgrad(dpre, x2, (ctx.ws[0],))
-        return dx, g_fc, g_proj, (dy if ctx.has_res else None)
+        m, c = x2.shape
+        f, n = w_fc.shape[0], w_proj.shape[0]
+        dpre, dx = torch.empty(m, f, dtype=BF16, device=dy.device), torch.empty(m, c, dtype=BF16, device=dy.device)
+        direct = [_wgrad_direct(*s, m) and w.dtype == BF16 and getattr(w, "main_grad", None) is None for w, s in zip(ctx.ws, ((f, c), (n, f)))]
+        g_fc = torch.empty(f, c, dtype=BF16, device=dy.device) if direct[0] else None
+        g_proj = torch.empty(n, f, dtype=BF16, device=dy.device) if direct[1] else None
+        L.call("bones_mlp_bf16_bwd", dy2.data_ptr(), x2.data_ptr(), h.data_ptr(), w_fc.data_ptr(), w_proj.data_ptr(), dpre.data_ptr(), dx.data_ptr(),
+               g_fc.data_ptr() if direct[0] else 0, g_proj.data_ptr() if direct[1] else 0, m, c, f, n, dy2.stride(0), x2.stride(0), w_fc.stride(0),
+               w_proj.stride(0), L.GEMM_MODE, L.raw_stream(), launches=2 + sum(direct))
+        COUNTS["gemm"] += 2 + sum(direct)
+        if not direct[1]:
+            (g_proj,) = _wgrad(dy2, h, (ctx.ws[1],))
+        if not direct[0]:
+            (g_fc,) = _wgrad(dpre, x2, (ctx.ws[0],))
+        return dx.view(ctx.shp), g_fc, g_proj, (dy if ctx.has_res else None)
 
 
 def mlp(x, w_fc, w_proj, residual=None, precision="bf16"):
