@@ -11,10 +11,7 @@
 // of a running maximum (the reference kernels do the same): P = exp(scale*s - scale*D) never overflows and no rescale of
 // the output accumulator is ever needed.  The row sum is kept in registers and `lse = log(sum) + scale*D` is saved.
 //
-// One CTA per (128-query tile, head, batch).  Warp 0: TMA producer (Q once, K/V tiles through a 2-stage ring).  Warp 1:
-// tcgen05.mma issuer: S = Q K^T into one of two TMEM buffers, then O += P V with P read from shared memory.  Warps 2-5:
-// one query row per thread: tcgen05.ld the scores, mask, exponentiate, write P (bf16) into 128-byte-swizzled shared
-// memory for the second MMA; at the end divide O by the row sum and store.
+// The roles of the persistent forward kernel stand with it below.
 #include "common.cuh"
 
 namespace bones {
@@ -247,14 +244,20 @@ __device__ __forceinline__ int attn_first_tile(const AttnParams& p, int b, int q
 // (head, batch), so the CTAs that run at one time share their K/V tiles through L2 (dealing the heaviest tiles of all
 // heads first made every CTA stream its own K/V from DRAM at once); the tile order is rotated from one (head, batch) to
 // the next so that every CTA sees a mix of lengths.  All barrier phases run on across items: the producer loads the next
-// item's Q and K/V while the current item computes, the MMA thread issues the next item's first S tiles while the softmax
-// warps finish the current one, and the output accumulator is double-buffered in TMEM so the drain of item i happens
-// after the first softmax tile of item i+1.
-//   TMEM: S/P buffers at columns 0 and 128 (by running tile count), O buffers at 256 and 384 (by item parity).
+// item's Q and K/V while the current item computes, the S warp issues the next item's first tiles while the softmax
+// warps finish the current one, and four warps of their own drain the output, so the softmax warps do nothing but exponentials.
+//   TMEM: S/P buffers at columns 0, 128 and 256 (running tile count mod 3), O at 384.  The scores run two tiles ahead of the
+//   exponentials, so S(g + 1) and its latency (PV, S and their hand-overs are 1 400 clocks) lie under two tiles of exponentials.
+// What bounds it now is the special-function units: a 128 x 128 tile's exponentials are 1 024 clocks, with sixteen warps 1 300 of the
+// 1 830 that a tile takes (2 770 with both products issued by one warp, the items drawn behind the last load and the output
+// drained by the softmax warps).  us: 16 x 2048 tokens in documents, 10 heads of 128, 141 -> 121; 8 x 2048 causal 107 -> 90; 8 x 1777 in
+// documents 73 -> 64; a window of 256 42.5 -> 40.5.  With a tile or two a CTA the longer hand-over shows (4 x 256, 4 heads of 64, 7.6 -> 8.3).
+// Tried and slower: two query tiles at a time with four warps each and shared K/V (8 x 2048 causal 129: the two fall in step, both
+// in their exponentials and then both waiting for MMAs), two groups of eight warps with items of their own (127).
 //   smem: Q x 2 (item parity), K x 2 and V x 3 stages (running tile count): a K stage is free again once its S tile is
 //   done, a V stage only after its O MMAs, so K and V rings of different depth keep the loads a full tile ahead.
 struct FwdItem {
-  int qt, h, b, kt0, n;
+  int qt, h, b;
 };
 __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w, int n_tiles) {
   FwdItem it;
@@ -262,16 +265,26 @@ __device__ __forceinline__ FwdItem fwd_item(const AttnParams& p, int w, int n_ti
   it.qt = n_tiles - 1 - (w % n_tiles + grp) % n_tiles;
   it.h = grp % p.H;
   it.b = grp / p.H;
-  it.kt0 = attn_first_tile(p, it.b, it.qt);
-  it.n = it.qt - it.kt0 + 1;
   return it;
 }
 
-// Threads: producer warp, MMA warp and sixteen softmax warps (four per 32-lane TMEM quadrant, 32 keys a thread).
+// Threads: Q and K loads, S warp, sixteen softmax warps (four per 32-lane TMEM quadrant, 32 keys a thread), four drain warps, PV warp, V loads.
 constexpr int FWD_SW = 16;
-constexpr uint32_t FWD_SLACK = 768;           // room for aligning the tiles to 1024 bytes (the seven tiles, the barriers and
+constexpr uint32_t FWD_BARS = 384;            // barriers, item ring, TMEM address, abort flag
+constexpr uint32_t FWD_SLACK = 640;           // room for aligning the tiles to 1024 bytes (the seven tiles, the barriers and
                                              // the scratch fill the rest of the 227 KB)
-constexpr int FWD_THREADS = 64 + 32 * FWD_SW;
+constexpr int FWD_DW = 4;
+constexpr int FWD_PV = 2 + FWD_SW + FWD_DW;
+constexpr int FWD_VW = FWD_PV + 1;
+constexpr int FWD_THREADS = 32 * (FWD_VW + 1);
+
+// The producer hands items to the other roles through a ring of eight (`item_take` in common.cuh has four): with items of a single tile
+// the drain warps may be six behind it, since S(t) needs the buffer of PV(t - 3), whose accumulator the drain before had to leave.
+constexpr int FWD_RING = 8;
+__device__ __forceinline__ int fwd_take(uint32_t bars, volatile int* slots, int it, volatile int* abort_flag, int* err) {
+  if (!mbar_wait(bars + 8u * (uint32_t)(it % FWD_RING), (uint32_t)((it / FWD_RING) & 1), abort_flag, err, ERR_WAIT_AUX)) return -1;
+  return slots[it % FWD_RING];
+}
 
 // D: head dim (64-wide heads on 128-wide tiles with zero halves did twice the MMAs and ten PyTorch passes of padding: a
 // forward and backward of 4 x 256 tokens, 4 heads took 314 us, 155 us natively).  T may have any value (padding the sequences
@@ -282,7 +295,6 @@ template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   constexpr uint32_t TILE_BYTES = (D / 64) * ATOM_BYTES;
-  constexpr int DT = D / 4;                            // output columns a softmax thread drains
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -303,17 +315,16 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   auto v_full = [&](int s) { return bars + 8u * (8 + s); };
   auto v_free = [&](int s) { return bars + 8u * (11 + s); };
   auto s_full = [&](int s) { return bars + 8u * (14 + s); };
-  auto p_full = [&](int s) { return bars + 8u * (16 + s); };
-  auto o_full = [&](int s) { return bars + 8u * (18 + s); };
-  auto o_free = [&](int s) { return bars + 8u * (20 + s); };
-  const uint32_t tmem_slot = bars + 8u * 22;
-  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + kBars + 176);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kBars + 184);
-  float* lsum = reinterpret_cast<float*>(gen + kBars + 256);           // [4 column parts][128 rows]
-  const uint32_t ring_bars = bars + 192u;
-  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + kBars + 224);
+  auto p_full = [&](int s) { return bars + 8u * (17 + s); };
+  auto s_free = [&](int s) { return bars + 336u + 8u * s; };
+  const uint32_t o_full = bars + 8u * 20, o_free = bars + 8u * 21, l_full = bars + 8u * 22, l_free = bars + 8u * 23, ring_bars = bars + 8u * 24;
+  volatile int* ring_slots = reinterpret_cast<volatile int*>(gen + kBars + 256);      // item numbers, and behind them first key tiles
+  const uint32_t tmem_slot = bars + 320u;
+  volatile uint32_t* tmem_slot_g = reinterpret_cast<volatile uint32_t*>(gen + kBars + 320);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(gen + kBars + 328);
+  float* lsum = reinterpret_cast<float*>(gen + kBars + FWD_BARS);           // [4 column parts][128 rows]
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int A = p.H * D;
   const int n_tiles = (p.T + AT - 1) / AT;
   const int total = n_tiles * p.H * p.B;
@@ -324,16 +335,19 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       mbar_init(q_free(s), 1);
       mbar_init(k_full(s), 1);
       mbar_init(k_free(s), 1);
-      mbar_init(s_full(s), 1);
-      mbar_init(p_full(s), FWD_SW);
-      mbar_init(o_full(s), 1);
-      mbar_init(o_free(s), FWD_SW);
     }
     for (int s = 0; s < 3; ++s) {
       mbar_init(v_full(s), 1);
       mbar_init(v_free(s), 1);
+      mbar_init(s_full(s), 1);
+      mbar_init(s_free(s), 1);
+      mbar_init(p_full(s), FWD_SW);
     }
-    for (int s = 0; s < 4; ++s) mbar_init(ring_bars + 8u * s, 1);
+    mbar_init(o_full, 1);
+    mbar_init(o_free, FWD_DW);
+    mbar_init(l_full, FWD_SW);
+    mbar_init(l_free, FWD_DW);
+    for (int s = 0; s < FWD_RING; ++s) mbar_init(ring_bars + 8u * s, 1);
     *abort_flag = 0;
     fence_barrier_init();
     tma_prefetch_desc(&tm_qk);
@@ -347,9 +361,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot_g;
+  const uint32_t tmem = (uint32_t)warp_uniform((int)*tmem_slot_g);
   auto tS = [&](int s) { return tmem + (uint32_t)s * 128u; };
-  auto tO = [&](int s) { return tmem + 256u + (uint32_t)s * 128u; };
+  const uint32_t tO = tmem + 384u;
 
   // The producer and MMA roles run on all 32 lanes of their warp with warp-uniform state and issue from the elected lane
   // (`elect_one` in common.cuh: operands computed under a `lane == 0` branch cost about 80 clocks per `tcgen05.mma`, more
@@ -357,165 +371,179 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   // A lane whose bounded wait ran out turns `dead`: it walks on without waiting or issuing; when lane 0 is dead no
   // further item is drawn and the warp leaves together.
   if (warp == 0) {
-    int g = 0, it = 0;
+    // Q and K loads, and the items: the next one is drawn, its document start read, and it is handed round and its Q requested one step
+    // a tile over the last tiles of the item before, so nobody waits for either latency (drawn and published behind the last
+    // load, it held the scores up for about 3 500 clocks an item).
+    // three tiles ahead, us: 16 x 2048 tokens in documents 121, two ahead 125, one 129; few items: two, so that the next one goes to a
+    // CTA that needs it soon (16 x 512 tokens 26.0 for 26.4)
+    const int ahead = total >= 6 * (int)gridDim.x ? 3 : 2;
+    int g = 0, it = 0, w = 0, kt0 = 0;
     bool dead = false;
-    for (;; ++it) {
-      int w = -1;
-      if (lane == 0 && !dead) w = item_publish(ring_bars, ring_slots, it, p.items, total);
-      w = warp_uniform(w);
-      if (w < 0) break;
-      FwdItem im = fwd_item(p, w, n_tiles);
-      im.kt0 = warp_uniform(im.kt0);
-      im.n = im.qt - im.kt0 + 1;
-      const int qb = it & 1;
-      if (it >= 2 && !dead) dead = !mbar_wait(q_free(qb), (uint32_t)(((it - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
-      if (elect_one() && !dead) {
-        mbar_arrive_expect_tx(q_full(qb), TILE_BYTES);
+    auto draw = [&](int step, int i) {
+      if (step == 0) {
+        if (lane == 0) w = atomicAdd(p.items, 1);
+      } else if (step == 1) {
+        w = warp_uniform(lane == 0 && !dead && w < total ? w : -1);
+        if (lane == 0 && w >= 0) {
+          const FwdItem im = fwd_item(p, w, n_tiles);
+          kt0 = attn_first_tile(p, im.b, im.qt);
+        }
+      } else {
+        if (lane == 0 && !dead) {
+          ring_slots[FWD_RING + i % FWD_RING] = kt0;
+          ring_slots[i % FWD_RING] = w;
+          mbar_arrive(ring_bars + 8u * (uint32_t)(i % FWD_RING));
+        }
+        kt0 = warp_uniform(kt0);
+        if (w < 0) return;
+        const FwdItem im = fwd_item(p, w, n_tiles);
+        const int qb = i & 1;
+        if (i >= 2 && !dead) dead = !mbar_wait(q_free(qb), (uint32_t)(((i - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
+        if (elect_one() && !dead) {
+          mbar_arrive_expect_tx(q_full(qb), TILE_BYTES);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qb) + c * ATOM_BYTES, &tm_qk, q_full(qb), im.h * D + c * 64, im.qt * AT, im.b);
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qb) + c * ATOM_BYTES, &tm_qk, q_full(qb), im.h * D + c * 64, im.qt * AT, im.b);
+        }
       }
-      for (int j = 0; j < im.n; ++j, ++g) {
-        const int ks = g & 1, vs = g % 3;
-        const int r = (im.kt0 + j) * AT;
+    };
+    for (int step = 0; step < 3; ++step) draw(step, 0);
+    for (; w >= 0; ++it) {
+      const FwdItem im = fwd_item(p, w, n_tiles);
+      const int k_first = kt0, n = im.qt - kt0 + 1;
+      int step = 0;
+      for (int j = 0; j < n; ++j, ++g) {
+        const int ks = g & 1;
         if (g >= 2 && !dead) dead = !mbar_wait(k_free(ks), (uint32_t)(((g - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(k_full(ks), TILE_BYTES);
 #pragma unroll
-          for (int c = 0; c < D / 64; ++c) tma_load_3d(sK(ks) + c * ATOM_BYTES, &tm_qk, k_full(ks), A + im.h * D + c * 64, r, im.b);
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sK(ks) + c * ATOM_BYTES, &tm_qk, k_full(ks), A + im.h * D + c * 64, (k_first + j) * AT, im.b);
         }
-        if (g >= 3 && !dead) dead = !mbar_wait(v_free(vs), (uint32_t)(((g - 3) / 3) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
+        if (j >= n - ahead) draw(step++, it + 1);
+      }
+      for (; step < 3; ++step) draw(step, it + 1);
+    }
+  } else if (warp == FWD_VW) {
+    // V loads
+    int g = 0, it = 0, vs = 0;
+    uint32_t vph = 1;
+    bool dead = false;
+    for (;; ++it) {
+      int w = -1;
+      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
+      w = warp_uniform(w);
+      if (w < 0) break;
+      const FwdItem im = fwd_item(p, w, n_tiles);
+      for (int kt = kt0; kt <= im.qt; ++kt, ++g) {
+        if (g >= 3 && !dead) dead = !mbar_wait(v_free(vs), vph, abort_flag, p.err, ERR_WAIT_EMPTY);
         if (elect_one() && !dead) {
           mbar_arrive_expect_tx(v_full(vs), TILE_BYTES);
 #pragma unroll
-          for (int c = 0; c < D / 64; ++c) tma_load_3d(sV(vs) + c * ATOM_BYTES, &tm_v, v_full(vs), 2 * A + im.h * D + c * 64, r, im.b);
+          for (int c = 0; c < D / 64; ++c) tma_load_3d(sV(vs) + c * ATOM_BYTES, &tm_v, v_full(vs), 2 * A + im.h * D + c * 64, kt * AT, im.b);
         }
+        if (++vs == 3) { vs = 0; vph ^= 1u; }
       }
     }
   } else if (warp == 1) {
+    // S = Q K^T of each tile, into the buffer whose O += P V (three tiles before) is done.  The products have a warp each: a wait takes
+    // 100 to 160 clocks even where it finds its barrier complete, and with three or four of them between the MMAs of one warp
+    // the tensor pipe stood still for as long as it worked (2 250 clocks a tile for 1 024 of MMAs).
+    // Everything an MMA takes is in uniform registers and known to be (`warp_uniform`): moved there one by one they cost about
+    // 100 clocks an MMA of 64.
+    constexpr uint32_t kHi = umma_desc_hi(1024, kLayoutSw128);
     const uint32_t idesc_s = umma_idesc_f16(128, 128, 1, 0, 0);   // Q (K-major) x K (K-major)
-    const uint32_t idesc_o = umma_idesc_f16(128, D, 1, 0, 1);   // P (TMEM) x V (MN-major)
-    // the O += P V step of a tile is issued one tile late, behind the next tile's S, so the softmax of tile g runs
-    // under the S MMAs of tile g+1.  P(g) sits in TMEM as packed bf16 pairs over the S(g) columns it was computed
-    // from (each softmax warp packs its 32 columns into the first 16 of its own range).
-    int pg = -1, p_item = 0;
-    bool p_first = false, p_last = false, dead = false;
-    auto issue_pv = [&]() {
-      const int sb = pg & 1, ob = p_item & 1, vs = pg % 3;
-      if (!dead) dead = !mbar_wait(v_full(vs), (uint32_t)((pg / 3) & 1), abort_flag, p.err, ERR_WAIT_FULL);
-      if (!dead) dead = !mbar_wait(p_full(sb), (uint32_t)((pg >> 1) & 1), abort_flag, p.err, ERR_WAIT_AUX);
-      if (p_first && p_item >= 2 && !dead)
-        dead = !mbar_wait(o_free(ob), (uint32_t)(((p_item - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
-      tc_fence_after();
-      const uint64_t vdesc0 = umma_smem_desc(sV(vs), ATOM_BYTES, 1024, kLayoutSw128);     // + a compile-time step per UMMA_K
-      if (elect_one() && !dead) {
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          const uint64_t bd = vdesc0 + (uint64_t)((k * 2048) >> 4);
-          umma_f16_ts(tO(ob), tS(sb) + (uint32_t)((k >> 1) * 32 + (k & 1) * 8), bd, idesc_o, (p_first && k == 0) ? 0u : 1u);
-        }
-        tc_commit(v_free(vs));
-        if (p_last) tc_commit(o_full(ob));
-      }
-    };
-    int g = 0, it = 0;
+    const uint32_t q_lo = (uint32_t)warp_uniform((int)umma_desc_lo(sQ(0), 0)), k_lo = (uint32_t)warp_uniform((int)umma_desc_lo(sK(0), 0));
+    bool dead = false;
+    int g = 0, gs = 0, it = 0;
+    uint32_t fph = 1;
     for (;; ++it) {
       int w = -1;
-      if (!dead) w = item_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
       w = warp_uniform(w);
       if (w < 0) break;
-      FwdItem im = fwd_item(p, w, n_tiles);
-      im.kt0 = warp_uniform(im.kt0);
-      im.n = im.qt - im.kt0 + 1;
-      const int qb = it & 1;
+      const int n = fwd_item(p, w, n_tiles).qt - kt0 + 1, qb = it & 1;
       if (!dead) dead = !mbar_wait(q_full(qb), (uint32_t)((it >> 1) & 1), abort_flag, p.err, ERR_WAIT_FULL);
-      for (int j = 0; j < im.n; ++j, ++g) {
-        const int sb = g & 1;
-        if (!dead) dead = !mbar_wait(k_full(sb), (uint32_t)((g >> 1) & 1), abort_flag, p.err, ERR_WAIT_FULL);
+      for (int j = 0; j < n; ++j, ++g) {
+        const int kb = g & 1;
+        if (!dead) dead = !mbar_wait(k_full(kb), (uint32_t)((g >> 1) & 1), abort_flag, p.err, ERR_WAIT_FULL);
+        if (g >= 3 && !dead) dead = !mbar_wait(s_free(gs), fph, abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
         tc_fence_after();
-        // S(g) overwrites the buffer that held P(g-2): its O MMAs were issued earlier on the same (in-order) pipe
-        const uint64_t qdesc0 = umma_smem_desc(sQ(qb), 0, 1024, kLayoutSw128), kdesc0 = umma_smem_desc(sK(sb), 0, 1024, kLayoutSw128);
+        const uint32_t qd = q_lo + (uint32_t)qb * (TILE_BYTES >> 4), kd = k_lo + (uint32_t)kb * (TILE_BYTES >> 4), sd = tS(gs);
         if (elect_one() && !dead) {
 #pragma unroll
           for (int k = 0; k < D / 16; ++k) {
-            const uint64_t off = (uint64_t)(((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4);
-            umma_f16(tS(sb), qdesc0 + off, kdesc0 + off, idesc_s, k ? 1u : 0u);
+            const uint32_t off = ((k >> 2) * ATOM_BYTES + (k & 3) * 32) >> 4;
+            umma_f16_lh(sd, qd + off, kHi, kd + off, kHi, idesc_s, k ? 1u : 0u);
           }
-          tc_commit(s_full(sb));
-          tc_commit(k_free(sb));
-          if (j == im.n - 1) tc_commit(q_free(qb));
+          tc_commit(s_full(gs));
+          tc_commit(k_free(kb));
+          if (j == n - 1) tc_commit(q_free(qb));
         }
-        if (pg >= 0) issue_pv();
-        pg = g; p_item = it; p_first = j == 0; p_last = j == im.n - 1;
+        if (++gs == 3) { gs = 0; fph ^= 1u; }
       }
     }
-    if (pg >= 0) issue_pv();
-  } else {
-    // Softmax: sixteen warps, four per 32-lane TMEM quadrant; each thread owns one query row and 32 of the tile's 128
-    // keys.  A tile's softmax is a chain -- TMEM load, exponentials, TMEM store -- that every warp runs at the same
-    // time; with eight warps and 64 keys a thread a tile took 2 400 clocks against 1 024 of MMAs, sixteen warps take a
-    // little less (0.207 -> 0.196 ms at B = 16, T = 2048, H = 10).  Two groups of eight warps that take alternate key
-    // tiles (each chain then has two tile periods) were measured as well and were no faster (0.204 ms): with 64 keys a
-    // thread the chain itself is twice as long.
+  } else if (warp == FWD_PV) {
+    // O += P V.  P(g) sits in TMEM as packed bf16 pairs over the S(g) columns it was computed from (each softmax warp packs its 32
+    // columns into the first 16 of its own range).
+    constexpr uint32_t kHi = umma_desc_hi(1024, kLayoutSw128);
+    const uint32_t idesc_o = umma_idesc_f16(128, D, 1, 0, 1);   // P (TMEM) x V (MN-major)
+    const uint32_t v_lo = (uint32_t)warp_uniform((int)umma_desc_lo(sV(0), ATOM_BYTES));
+    bool dead = false;
+    int ps = 0, it = 0;                      // P buffer and V stage
+    uint32_t pph = 0;
+    for (;; ++it) {
+      int w = -1;
+      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
+      w = warp_uniform(w);
+      if (w < 0) break;
+      const int n = fwd_item(p, w, n_tiles).qt - kt0 + 1;
+      for (int j = 0; j < n; ++j) {
+        if (!dead) dead = !mbar_wait(v_full(ps), pph, abort_flag, p.err, ERR_WAIT_FULL);
+        if (j == 0 && it >= 1 && !dead) dead = !mbar_wait(o_free, (uint32_t)((it - 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
+        if (!dead) dead = !mbar_wait(p_full(ps), pph, abort_flag, p.err, ERR_WAIT_AUX);
+        tc_fence_after();
+        const uint32_t vd = v_lo + (uint32_t)ps * (TILE_BYTES >> 4), pd = tS(ps);
+        if (elect_one() && !dead) {
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            umma_f16_ts_lh(tO, pd + (uint32_t)((k >> 1) * 32 + (k & 1) * 8), vd + (uint32_t)((k * 2048) >> 4), kHi, idesc_o, (j == 0 && k == 0) ? 0u : 1u);
+          tc_commit(s_free(ps));
+          tc_commit(v_free(ps));
+          if (j == n - 1) tc_commit(o_full);
+        }
+        if (++ps == 3) { ps = 0; pph ^= 1u; }
+      }
+    }
+  } else if (warp < 2 + FWD_SW) {
+    // Softmax: sixteen warps, four per 32-lane TMEM quadrant; each thread owns one query row and 32 of the tile's 128 keys.
+    // (Two groups of warps on tiles or items of their own were no faster: they fall in step and wait for the MMAs together.)
     const int q = warp & 3, part = (warp - 2) >> 2;
     const int r = q * 32 + lane;            // row within the tile == TMEM lane
     const int c0 = part * 32;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
-    // the drain of an item's output is deferred until the first tile of the next item has been exponentiated
-    bool pend = false, ok = true;
-    int pend_it = 0;
-    float pend_inv = 0.f;
-    __nv_bfloat16* pend_y = nullptr;
-    auto drain = [&]() -> bool {
-      const int ob = pend_it & 1;
-      const bool got = mbar_wait(o_full(ob), (uint32_t)((pend_it >> 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
-      if (!__all_sync(0xffffffffu, got)) return false;
-      tc_fence_after();
-      {
-        uint32_t v[DT];
-        __syncwarp();
-        if constexpr (DT == 32) BONES_TMEM_LD32(tO(ob) + lane_addr + (uint32_t)(part * DT), v);
-        else BONES_TMEM_LD16(tO(ob) + lane_addr + (uint32_t)(part * DT), v);
-        tmem_ld_wait();
-        uint4 u[DT / 8];
-#pragma unroll
-        for (int gq = 0; gq < DT / 8; ++gq) {
-          u[gq].x = pack_bf16(__uint_as_float(v[gq * 8 + 0]) * pend_inv, __uint_as_float(v[gq * 8 + 1]) * pend_inv);
-          u[gq].y = pack_bf16(__uint_as_float(v[gq * 8 + 2]) * pend_inv, __uint_as_float(v[gq * 8 + 3]) * pend_inv);
-          u[gq].z = pack_bf16(__uint_as_float(v[gq * 8 + 4]) * pend_inv, __uint_as_float(v[gq * 8 + 5]) * pend_inv);
-          u[gq].w = pack_bf16(__uint_as_float(v[gq * 8 + 6]) * pend_inv, __uint_as_float(v[gq * 8 + 7]) * pend_inv);
-        }
-        if (pend_y) {
-#pragma unroll
-          for (int gq = 0; gq < DT / 8; gq += 2) st_global_v8(pend_y + gq * 8, u[gq], u[gq + 1]);      // full 32-byte sectors
-        }
-      }
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(o_free(ob));
-      pend = false;
-      return true;
-    };
-    int g = 0, it = 0;
-    for (;; ++it) {
-      const int w = ok ? item_take(ring_bars, ring_slots, it, abort_flag, p.err) : -1;
+    int gs = 0;
+    uint32_t sph = 0;
+    bool ok = true;
+    for (int it = 0; ok; ++it) {
+      const int w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
       if (w < 0) break;
+      const int kt0 = ring_slots[FWD_RING + it % FWD_RING];
       const FwdItem im = fwd_item(p, w, n_tiles);
       const int qpos = im.qt * AT + r;
-      const bool real = qpos < p.T;
-      int lo = 0;
-      if (p.doc_start && real) lo = p.doc_start[(long long)im.b * p.T + qpos];
+      int lo = 0;                                // on its way while the first scores are waited for and exponentiated
+      if (p.doc_start && qpos < p.T) lo = p.doc_start[(long long)im.b * p.T + qpos];
       float l = 0.f;
-      for (int j = 0; j < im.n; ++j, ++g) {
-        const int sb = g & 1;
-        const bool got = mbar_wait(s_full(sb), (uint32_t)((g >> 1) & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
+      for (int kt = kt0; kt <= im.qt; ++kt) {
+        const bool got = mbar_wait(s_full(gs), sph, abort_flag, p.err, ERR_WAIT_TMEM_FULL);
         if (!__all_sync(0xffffffffu, got)) { ok = false; break; }
         tc_fence_after();
-        const int k0 = (im.kt0 + j) * AT + c0;
-        // warp-uniform: does any row of this warp need the element mask for these 32 keys (diagonal or document start)?
-        const bool need_mask = __any_sync(0xffffffffu, (k0 + 31 > qpos) || (k0 < lo));
+        const int k0 = kt * AT + c0;
         uint32_t v0[32], pk[16];
         __syncwarp();
-        BONES_TMEM_LD32(tS(sb) + lane_addr + (uint32_t)c0, v0);
+        BONES_TMEM_LD32(tS(gs) + lane_addr + (uint32_t)c0, v0);
         tmem_ld_wait();
         {
           float e[32];
@@ -524,38 +552,81 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
             const float x = fmaf(__uint_as_float(v0[i]), p.c1, -p.c2);
             asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e[i]) : "f"(x));
           }
-          if (need_mask) {
+          // warp-uniform: does any row of this warp need the element mask for these 32 keys (diagonal or document start)?
+          if (__any_sync(0xffffffffu, (k0 + 31 > qpos) || (k0 < lo))) {
 #pragma unroll
             for (int i = 0; i < 32; ++i) {
               const int kpos = k0 + i;
               if (kpos > qpos || kpos < lo) e[i] = 0.f;
             }
           }
+          float l4[4] = {0.f, 0.f, 0.f, 0.f};              // four chains: one of 32 additions takes as long as a quarter of the exponentials
 #pragma unroll
-          for (int i = 0; i < 32; ++i) l += e[i];
+          for (int i = 0; i < 32; ++i) l4[i & 3] += e[i];
+          l += (l4[0] + l4[1]) + (l4[2] + l4[3]);
 #pragma unroll
           for (int i = 0; i < 16; ++i) pk[i] = pack_bf16(e[2 * i], e[2 * i + 1]);
         }
-        BONES_TMEM_ST16(tS(sb) + lane_addr + (uint32_t)c0, pk);
+        BONES_TMEM_ST16(tS(gs) + lane_addr + (uint32_t)c0, pk);
         tmem_st_wait();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(p_full(sb));
-        if (pend && !drain()) { ok = false; break; }
+        if (lane == 0) mbar_arrive(p_full(gs));
+        if (++gs == 3) { gs = 0; sph ^= 1u; }
       }
       if (!ok) break;
-      // the four threads of a row exchange their partial row sums through shared memory
+      // the partial row sums of the four threads of a row go to the drain warps
+      if (it >= 1 && !__all_sync(0xffffffffu, mbar_wait(l_free, (uint32_t)((it - 1) & 1), abort_flag, p.err, ERR_WAIT_AUX))) break;
       lsum[part * AT + r] = l;
-      asm volatile("bar.sync 1, 512;" ::: "memory");
-      l = (lsum[r] + lsum[AT + r]) + (lsum[2 * AT + r] + lsum[3 * AT + r]);      // the same order in all four threads
-      asm volatile("bar.sync 1, 512;" ::: "memory");      // nobody rewrites the scratch before everybody has read it
-      if (part == 0 && real) p.lse[((long long)im.b * p.H + im.h) * p.T + qpos] = logf(l) + p.shift_ln;
-      pend = true;
-      pend_it = it;
-      pend_inv = 1.0f / l;
-      pend_y = real ? p.y + ((long long)im.b * p.T + qpos) * A + (long long)im.h * D + part * DT : nullptr;
+      __syncwarp();
+      if (lane == 0) mbar_arrive(l_full);
     }
-    if (ok && pend) drain();
+  } else {
+    // Drain: a thread per query row.
+    const int q = warp & 3, r = q * 32 + lane;
+    const uint32_t tOr = tO + ((uint32_t)(q * 32) << 16);
+    for (int it = 0;; ++it) {
+      const int w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      if (w < 0) break;
+      const FwdItem im = fwd_item(p, w, n_tiles);
+      const int qpos = im.qt * AT + r;
+      const bool real = qpos < p.T;
+      bool got = mbar_wait(l_full, (uint32_t)(it & 1), abort_flag, p.err, ERR_WAIT_AUX);
+      if (!__all_sync(0xffffffffu, got)) break;
+      const float l = (lsum[r] + lsum[AT + r]) + (lsum[2 * AT + r] + lsum[3 * AT + r]);
+      __syncwarp();
+      if (lane == 0) mbar_arrive(l_free);
+      if (real) p.lse[((long long)im.b * p.H + im.h) * p.T + qpos] = logf(l) + p.shift_ln;
+      const float inv = 1.0f / l;
+      __nv_bfloat16* y = p.y + ((long long)im.b * p.T + qpos) * A + (long long)im.h * D;
+      got = mbar_wait(o_full, (uint32_t)(it & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
+      if (!__all_sync(0xffffffffu, got)) break;
+      tc_fence_after();
+#pragma unroll
+      for (int c = 0; c < D; c += 32) {
+        uint32_t v[32];
+        __syncwarp();
+        BONES_TMEM_LD32(tOr + (uint32_t)c, v);
+        tmem_ld_wait();
+        if (c + 32 >= D) {                             // the next item's products may have the accumulator
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(o_free);
+        }
+        uint4 u[4];
+#pragma unroll
+        for (int gq = 0; gq < 4; ++gq) {
+          u[gq].x = pack_bf16(__uint_as_float(v[gq * 8 + 0]) * inv, __uint_as_float(v[gq * 8 + 1]) * inv);
+          u[gq].y = pack_bf16(__uint_as_float(v[gq * 8 + 2]) * inv, __uint_as_float(v[gq * 8 + 3]) * inv);
+          u[gq].z = pack_bf16(__uint_as_float(v[gq * 8 + 4]) * inv, __uint_as_float(v[gq * 8 + 5]) * inv);
+          u[gq].w = pack_bf16(__uint_as_float(v[gq * 8 + 6]) * inv, __uint_as_float(v[gq * 8 + 7]) * inv);
+        }
+        if (real) {                                    // full 32-byte sectors
+          st_global_v8(y + c, u[0], u[1]);
+          st_global_v8(y + c + 16, u[2], u[3]);
+        }
+      }
+    }
   }
 
   tc_fence_before();
@@ -579,7 +650,7 @@ static int tmap_rows_3d(CUtensorMap* out, const void* ptr, int B, int T, long lo
 
 template <int D>
 static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tv, const AttnParams& p, int sms, cudaStream_t s) {
-  constexpr size_t smem = (size_t)(D / 64) * ATOM_BYTES * 7 + 256 + 2048 + FWD_SLACK;   // tiles, barriers, row-sum scratch, alignment slack
+  constexpr size_t smem = (size_t)(D / 64) * ATOM_BYTES * 7 + FWD_BARS + 2048 + FWD_SLACK;   // tiles, barriers, row-sum scratch, alignment slack
   static bool attr_done = false;
   if (!attr_done) {
     BONES_CHECK(cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
