@@ -233,11 +233,9 @@ struct AttnParams {
 constexpr int AT = 128;                         // tile edge (queries and keys)
 constexpr uint32_t ATOM_BYTES = AT * 64 * 2;    // 16 KB: one 128-byte-swizzled atom of [128 rows][64 cols]; a tile has D / 64
 
-__device__ __forceinline__ int attn_first_tile(const AttnParams& p, int b, int qt) {
-  int lo = 0;
-  if (p.doc_start) lo = p.doc_start[(long long)b * p.T + qt * AT] / AT;
-  if (p.window_tiles > 0) lo = max(lo, qt - p.window_tiles + 1);
-  return lo;
+// first key tile of query tile `qt`, whose first query's document begins at `doc`
+__device__ __forceinline__ int attn_first_tile(const AttnParams& p, int doc, int qt) {
+  return p.window_tiles > 0 ? max(doc / AT, qt - p.window_tiles + 1) : doc / AT;
 }
 
 // Persistent forward: one CTA per SM walks (query tile, head, batch) items.  Consecutive items are the query tiles of one
@@ -251,7 +249,11 @@ __device__ __forceinline__ int attn_first_tile(const AttnParams& p, int b, int q
 // What bounds it now is the special-function units: a 128 x 128 tile's exponentials are 1 024 clocks, with sixteen warps 1 300 of the
 // 1 830 that a tile takes (2 770 with both products issued by one warp, the items drawn behind the last load and the output
 // drained by the softmax warps).  us: 16 x 2048 tokens in documents, 10 heads of 128, 141 -> 121; 8 x 2048 causal 107 -> 90; 8 x 1777 in
-// documents 73 -> 64; a window of 256 42.5 -> 40.5.  With a tile or two a CTA the longer hand-over shows (4 x 256, 4 heads of 64, 7.6 -> 8.3).
+// documents 73 -> 64; a window of 256 42.5 -> 40.5.
+// With a tile or two a CTA the longer chain of roles cost 0.3 to 0.7 us; what took it back: a CTA's first item is its own number (no
+// counter, no ring), its Q is requested before its document start is known, and an item's coordinates are divided out once, not again before its
+// loads.  us with the counter's zero fill, one warp for both products / drawn first item / now: 4 x 256, 4 heads of 64 8.5 / 9.2 / 8.5; 8 x 100
+// 7.4 / 8.1 / 7.3; 10 heads of 128: 1 x 128 8.4 / 8.8 / 8.0, 8 x 128 8.8 / 9.2 / 8.6, 16 x 512 in documents 28.3 / 25.8 / 22.0.
 // Tried and slower: two query tiles at a time with four warps each and shared K/V (8 x 2048 causal 129: the two fall in step, both
 // in their exponentials and then both waiting for MMAs), two groups of eight warps with items of their own (127).
 //   smem: Q x 2 (item parity), K x 2 and V x 3 stages (running tile count): a K stage is free again once its S tile is
@@ -295,6 +297,10 @@ template <int D>
 __global__ void __launch_bounds__(FWD_THREADS, 1)
 attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant__ CUtensorMap tm_v, const AttnParams p) {
   constexpr uint32_t TILE_BYTES = (D / 64) * ATOM_BYTES;
+  if (threadIdx.x == 32 * FWD_VW) {
+    tma_prefetch_desc(&tm_qk);
+    tma_prefetch_desc(&tm_v);
+  }
   extern __shared__ uint8_t smem_raw[];
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t base = (raw + 1023u) & ~1023u;
@@ -329,32 +335,13 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   const int n_tiles = (p.T + AT - 1) / AT;
   const int total = n_tiles * p.H * p.B;
 
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < 2; ++s) {
-      mbar_init(q_full(s), 1);
-      mbar_init(q_free(s), 1);
-      mbar_init(k_full(s), 1);
-      mbar_init(k_free(s), 1);
-    }
-    for (int s = 0; s < 3; ++s) {
-      mbar_init(v_full(s), 1);
-      mbar_init(v_free(s), 1);
-      mbar_init(s_full(s), 1);
-      mbar_init(s_free(s), 1);
-      mbar_init(p_full(s), FWD_SW);
-    }
-    mbar_init(o_full, 1);
-    mbar_init(o_free, FWD_DW);
-    mbar_init(l_full, FWD_SW);
-    mbar_init(l_free, FWD_DW);
-    for (int s = 0; s < FWD_RING; ++s) mbar_init(ring_bars + 8u * s, 1);
-    *abort_flag = 0;
+  if (warp == 0) {                                     // a barrier a lane, in the order of the list above
+    const bool by_softmax = (lane >= 17 && lane < 20) || lane == 22, by_drain = lane == 21 || lane == 23;
+    mbar_init(bars + 8u * (uint32_t)lane, by_softmax ? FWD_SW : by_drain ? FWD_DW : 1);
+    if (lane < 3) mbar_init(s_free(lane), 1);
+    if (lane == 0) *abort_flag = 0;
     fence_barrier_init();
-    tma_prefetch_desc(&tm_qk);
-    tma_prefetch_desc(&tm_v);
-  }
-  __syncthreads();
-  if (warp == 1) {
+  } else if (warp == 1) {
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
@@ -362,6 +349,18 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = (uint32_t)warp_uniform((int)*tmem_slot_g);
+  // the first item, whose keys every role looks up itself
+  const FwdItem first = fwd_item(p, (int)blockIdx.x, n_tiles);
+  const int doc_first = p.doc_start ? p.doc_start[(long long)first.b * p.T + first.qt * AT] : 0;
+  const int kt_first = warp_uniform(attn_first_tile(p, doc_first, first.qt));
+  // item `it` of this CTA and its first key tile; -1 behind the last one
+  auto take = [&](int it, int* kt0) {
+    *kt0 = kt_first;
+    if (it == 0) return (int)blockIdx.x;
+    const int w = fwd_take(ring_bars, ring_slots, it - 1, abort_flag, p.err);
+    *kt0 = ring_slots[FWD_RING + (it - 1) % FWD_RING];
+    return w;
+  };
   auto tS = [&](int s) { return tmem + (uint32_t)s * 128u; };
   const uint32_t tO = tmem + 384u;
 
@@ -377,38 +376,42 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     // three tiles ahead, us: 16 x 2048 tokens in documents 121, two ahead 125, one 129; few items: two, so that the next one goes to a
     // CTA that needs it soon (16 x 512 tokens 26.0 for 26.4)
     const int ahead = total >= 6 * (int)gridDim.x ? 3 : 2;
-    int g = 0, it = 0, w = 0, kt0 = 0;
+    int g = 0, it = 0, w = (int)blockIdx.x, kt0 = kt_first;
     bool dead = false;
+    FwdItem after = first;
+    auto load_q = [&](const FwdItem& im, int qb) {
+      if (elect_one() && !dead) {
+        mbar_arrive_expect_tx(q_full(qb), TILE_BYTES);
+#pragma unroll
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qb) + c * ATOM_BYTES, &tm_qk, q_full(qb), im.h * D + c * 64, im.qt * AT, im.b);
+      }
+    };
     auto draw = [&](int step, int i) {
       if (step == 0) {
-        if (lane == 0) w = atomicAdd(p.items, 1);
+        if (lane == 0) w = (int)gridDim.x + atomicAdd(p.items, 1);
       } else if (step == 1) {
         w = warp_uniform(lane == 0 && !dead && w < total ? w : -1);
+        if (w >= 0) after = fwd_item(p, w, n_tiles);
         if (lane == 0 && w >= 0) {
-          const FwdItem im = fwd_item(p, w, n_tiles);
-          kt0 = attn_first_tile(p, im.b, im.qt);
+          kt0 = attn_first_tile(p, p.doc_start ? p.doc_start[(long long)after.b * p.T + after.qt * AT] : 0, after.qt);
         }
       } else {
         if (lane == 0 && !dead) {
-          ring_slots[FWD_RING + i % FWD_RING] = kt0;
-          ring_slots[i % FWD_RING] = w;
-          mbar_arrive(ring_bars + 8u * (uint32_t)(i % FWD_RING));
+          const int s = (i - 1) % FWD_RING;
+          ring_slots[FWD_RING + s] = kt0;
+          ring_slots[s] = w;
+          mbar_arrive(ring_bars + 8u * (uint32_t)s);
         }
         kt0 = warp_uniform(kt0);
         if (w < 0) return;
-        const FwdItem im = fwd_item(p, w, n_tiles);
         const int qb = i & 1;
         if (i >= 2 && !dead) dead = !mbar_wait(q_free(qb), (uint32_t)(((i - 2) >> 1) & 1), abort_flag, p.err, ERR_WAIT_EMPTY);
-        if (elect_one() && !dead) {
-          mbar_arrive_expect_tx(q_full(qb), TILE_BYTES);
-#pragma unroll
-          for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ(qb) + c * ATOM_BYTES, &tm_qk, q_full(qb), im.h * D + c * 64, im.qt * AT, im.b);
-        }
+        load_q(after, qb);
       }
     };
-    for (int step = 0; step < 3; ++step) draw(step, 0);
-    for (; w >= 0; ++it) {
-      const FwdItem im = fwd_item(p, w, n_tiles);
+    FwdItem im = first;
+    load_q(first, 0);
+    for (; w >= 0; ++it, im = after) {
       const int k_first = kt0, n = im.qt - kt0 + 1;
       int step = 0;
       for (int j = 0; j < n; ++j, ++g) {
@@ -429,9 +432,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     uint32_t vph = 1;
     bool dead = false;
     for (;; ++it) {
-      int w = -1;
-      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
-      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
+      int w = -1, kt0 = 0;
+      if (!dead) w = take(it, &kt0);
+      kt0 = warp_uniform(kt0);
       w = warp_uniform(w);
       if (w < 0) break;
       const FwdItem im = fwd_item(p, w, n_tiles);
@@ -458,9 +461,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     int g = 0, gs = 0, it = 0;
     uint32_t fph = 1;
     for (;; ++it) {
-      int w = -1;
-      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
-      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
+      int w = -1, kt0 = 0;
+      if (!dead) w = take(it, &kt0);
+      kt0 = warp_uniform(kt0);
       w = warp_uniform(w);
       if (w < 0) break;
       const int n = fwd_item(p, w, n_tiles).qt - kt0 + 1, qb = it & 1;
@@ -494,9 +497,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     int ps = 0, it = 0;                      // P buffer and V stage
     uint32_t pph = 0;
     for (;; ++it) {
-      int w = -1;
-      if (!dead) w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
-      const int kt0 = warp_uniform(ring_slots[FWD_RING + it % FWD_RING]);
+      int w = -1, kt0 = 0;
+      if (!dead) w = take(it, &kt0);
+      kt0 = warp_uniform(kt0);
       w = warp_uniform(w);
       if (w < 0) break;
       const int n = fwd_item(p, w, n_tiles).qt - kt0 + 1;
@@ -528,9 +531,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     uint32_t sph = 0;
     bool ok = true;
     for (int it = 0; ok; ++it) {
-      const int w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      int kt0;
+      const int w = take(it, &kt0);
       if (w < 0) break;
-      const int kt0 = ring_slots[FWD_RING + it % FWD_RING];
       const FwdItem im = fwd_item(p, w, n_tiles);
       const int qpos = im.qt * AT + r;
       int lo = 0;                                // on its way while the first scores are waited for and exponentiated
@@ -586,7 +589,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     const int q = warp & 3, r = q * 32 + lane;
     const uint32_t tOr = tO + ((uint32_t)(q * 32) << 16);
     for (int it = 0;; ++it) {
-      const int w = fwd_take(ring_bars, ring_slots, it, abort_flag, p.err);
+      int kt0;
+      const int w = take(it, &kt0);
       if (w < 0) break;
       const FwdItem im = fwd_item(p, w, n_tiles);
       const int qpos = im.qt * AT + r;
@@ -602,7 +606,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
       got = mbar_wait(o_full, (uint32_t)(it & 1), abort_flag, p.err, ERR_WAIT_TMEM_FULL);
       if (!__all_sync(0xffffffffu, got)) break;
       tc_fence_after();
-#pragma unroll
+#pragma unroll 1
       for (int c = 0; c < D; c += 32) {
         uint32_t v[32];
         __syncwarp();
