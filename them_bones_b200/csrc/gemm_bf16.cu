@@ -64,7 +64,7 @@ __device__ __forceinline__ void decode_tile(int tile, int tiles_m, int tiles_n, 
   nb = in_group / gsz;
 }
 
-template <int BN, int STAGES>
+template <int BN, int STAGES, bool LOOK>
 __global__ void __launch_bounds__(192, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b, const GemmParams p) {
   extern __shared__ uint8_t smem_raw[];
@@ -153,37 +153,36 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
     const uint32_t a_lbo = p.a_major ? BK * 128 : 0, b_lbo = p.b_major ? BK * 128 : 0;
     const uint32_t a_step = p.a_major ? (16 * 128) >> 4 : 32 >> 4;   // descriptor address units of 16 bytes per UMMA_K
     const uint32_t b_step = p.b_major ? (16 * 128) >> 4 : 32 >> 4;
-    // descriptors of stage 0; a stage adds STAGE_BYTES >> 4 to the address field
-    const uint64_t adesc0 = umma_smem_desc(base, a_lbo, 1024, kLayoutSw128);
-    const uint64_t bdesc0 = umma_smem_desc(base + A_BYTES, b_lbo, 1024, kLayoutSw128);
-    // A K block's four MMAs are shorter than its loads in any width; asking for the next stage ahead (`mbar_test`) takes the waits out of
-    // the chain: 1000 x 1280 x 5120 28.0 -> 26.5 us, 64 x 1280 x 5120 25.7 -> 24.2.
+    // descriptors of stage 0, in uniform registers and known to be; a stage adds STAGE_BYTES >> 4 to the address field
+    constexpr uint32_t kHi = umma_desc_hi(1024, kLayoutSw128);
+    const uint32_t a_lo = (uint32_t)warp_uniform((int)umma_desc_lo(base, a_lbo)), b_lo = (uint32_t)warp_uniform((int)umma_desc_lo(base + A_BYTES, b_lbo));
+    const uint32_t d0 = (uint32_t)warp_uniform((int)tmem);
+    // A K block's four MMAs are shorter than its loads in any width; LOOK: asking for the next stage ahead (`mbar_test`) takes the waits out of
+    // the chain (rule in launch_gemm).
     int stage = 0, acc = 0;
     uint32_t phase = 0, acc_phase = 0;
     bool dead = false, ready = false;
     for (int tile = blockIdx.x; tile < total; tile += gridDim.x) {
       if (!dead) dead = !mbar_wait(tempty(acc), acc_phase ^ 1u, abort_flag, p.err, ERR_WAIT_TMEM_EMPTY);
       tc_fence_after();
-      const uint32_t d_tmem = tmem + acc * BN;
+      const uint32_t d_tmem = d0 + acc * BN;
       const int sp = p.splits == 1 ? 0 : tile / base_tiles;
       const int kb0 = p.splits == 1 ? 0 : (int)((long long)KB * sp / p.splits), kb1 = p.splits == 1 ? KB : (int)((long long)KB * (sp + 1) / p.splits);
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!ready && !dead) dead = !mbar_wait(full(stage), phase, abort_flag, p.err, ERR_WAIT_FULL);
         tc_fence_after();
-        const int next = stage + 1 == STAGES ? 0 : stage + 1;
-        const uint32_t next_phase = next ? phase : phase ^ 1u, there = mbar_test(full(next), next_phase);
-        const uint64_t soff = (uint64_t)(stage * (STAGE_BYTES >> 4));
-        const uint64_t adesc = adesc0 + soff, bdesc = bdesc0 + soff;
+        uint32_t there = 0u;
+        if constexpr (LOOK) there = mbar_test(full(stage + 1 == STAGES ? 0 : stage + 1), stage + 1 == STAGES ? phase ^ 1u : phase);
+        const uint32_t ad = a_lo + (uint32_t)(stage * (STAGE_BYTES >> 4)), bd = b_lo + (uint32_t)(stage * (STAGE_BYTES >> 4));
         if (elect_one() && !dead) {
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k)
-            umma_f16(d_tmem, adesc + (uint64_t)(k * a_step), bdesc + (uint64_t)(k * b_step), idesc, ((kb - kb0) | k) ? 1u : 0u);
+            umma_f16_lh(d_tmem, ad + k * a_step, kHi, bd + k * b_step, kHi, idesc, ((kb - kb0) | k) ? 1u : 0u);
           tc_commit(empty(stage));
           if (kb == kb1 - 1) tc_commit(tfull(acc));
         }
-        ready = __all_sync(0xffffffffu, there != 0u);
-        stage = next;
-        phase = next_phase;
+        if constexpr (LOOK) ready = __all_sync(0xffffffffu, there != 0u);
+        if (++stage == STAGES) { stage = 0; phase ^= 1u; }
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1u;
@@ -239,12 +238,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constan
   }
 }
 
-template <int BN, int STAGES>
-static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
+template <int BN, int STAGES, bool LOOK>
+static int launch_one(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
   constexpr size_t smem = (size_t)STAGES * (BM * BK * 2 + BN * BK * 2) + 8 * (2 * STAGES + 4) + 16 + 1024;
   static bool attr_done = false;
   if (!attr_done) {
-    BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_kernel<BN, STAGES, LOOK>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     attr_done = true;
   }
   int dev = 0, sms = 0;
@@ -271,8 +270,15 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams 
   if (p.splits > KB) p.splits = KB;          // every split owns at least one K block (its last block signals the epilogue)
   const int total = base_tiles * p.splits;
   const int grid = total < sms ? total : sms;
-  gemm_bf16_kernel<BN, STAGES><<<grid, 192, smem, stream>>>(ta, tb, p);
+  gemm_bf16_kernel<BN, STAGES, LOOK><<<grid, 192, smem, stream>>>(ta, tb, p);
   return (int)cudaGetLastError();
+}
+// Long contractions run with the look at the next stage, 1000 x 1280 x 5120 27.2 us without it, 25.5 with; 64 x 1280 x 5120 25.7, 24.1;
+// 1000 x 1280 x 2048 13.6, 12.9; at 1024 the two are equal.  Shorter ones without: each tile begins 0.15 to 0.2 us later with it (64 x 65536 x 64
+// 7.2 us without, 7.65 with; 8 x 256 x 64 3.75, 3.9; 8 x 256 x 512 5.9, 6.1).
+template <int BN, int STAGES>
+static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams p, cudaStream_t stream) {
+  return p.K > 1024 ? launch_one<BN, STAGES, true>(ta, tb, p, stream) : launch_one<BN, STAGES, false>(ta, tb, p, stream);
 }
 
 static int operand_tmap(CUtensorMap* out, const void* ptr, int major, long long rows, long long K, long long ld, long long stride,
