@@ -47,8 +47,15 @@ int make_tmap(CUtensorMap* out, CUtensorMapDataType dt, int rank, const void* ba
     estr[i] = 1;
   }
   for (int i = 0; i + 1 < rank; ++i) gstr[i] = strides_bytes[i];
-  CUresult r = fn(out, dt, (cuuint32_t)rank, const_cast<void*>(base), gdim, gstr, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
-                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  auto encode = [&] {
+    return fn(out, dt, (cuuint32_t)rank, const_cast<void*>(base), gdim, gstr, gbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swz,
+              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  };
+  CUresult r = encode();
+  int dev = 0;
+  // This driver call wants the thread's context to be current, which no runtime call may have seen to yet: autograd's device thread, or a
+  // program's, with the allocator's blocks at hand comes here first.  Choosing the device it already has makes it so.
+  if (r == CUDA_ERROR_INVALID_CONTEXT && cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess) r = encode();
   return r == CUDA_SUCCESS ? 0 : -(int)r - 1000;
 }
 
