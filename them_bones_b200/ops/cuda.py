@@ -95,13 +95,27 @@ def mm_tn(dy, x, out):
     return out
 
 
-def _wgrad_direct(n, k, m):
+def _wgrad_direct(n, k, m, sms=148):
     """Whether a weight gradient ``[n, k]`` of ``m`` rows that autograd gets back (no slab to accumulate into) is written as bf16 by the
-    GEMM.  Accumulating in fp32 lets the GEMM split its contraction over idle SMs, but costs a zero fill, a read-modify-write with
-    atomics and a cast.  Those are the longer up to a contraction that grows with the tiles there are to occupy the SMs.  Direct / split, us:
-    5120 x 1280 of 1000 rows 17 / 39, 4096 46 / 56, 8192 86 / 93, 16384 167 / 164; 1280 x 1280 of 2048 15 / 20, 4096 23 / 26, 8192 40 / 40,
-    16384 90 / 56; 256 x 1024 of 2048 13 / 14, 4096 21 / 15."""
-    return 0 < m <= max(2048, 164 * (-(-n // 256)) * (-(-k // 256)))
+    GEMM.  Accumulating in fp32 lets the GEMM share the contraction out over all ``sms`` SMs, from 32 K blocks of 64 rows on, but costs a
+    zero fill, a read-modify-write with atomics and a cast.  us for a K block: 0.27 a wave of single CTAs, 0.31 a wave of pairs, 0.40 for
+    each full set of pair tiles where they are shared out; the fp32 route's passes: 9 (5 for one narrow column of tiles) and 1.8 for each million
+    weights.  Above 13 000 rows the direct form has gained at most 3 % and lost 8.  Direct / shared, us:
+    5120 x 1280 of 1000 rows 17 / 39, 4096 46 / 55, 12288 126 / 131, 16384 179 / 165; 3840 x 1280 (75 tiles, two waves of 74 pairs) of 2048 27 / 40,
+    6144 65 / 63, 8192 84 / 74, 12288 122 / 100; 2560 x 1280 (one wave) 8192 45 / 51, 12288 66 / 68; 1280 x 1280 of 2048 15 / 20, 4096 24 / 25,
+    6144 34 / 30, 16384 77 / 51; 1024 x 1024 of 2048 16 / 17, 4096 25 / 20; 256 x 256 of 2048 13.6 / 14.1, 3072 18 / 15; 256 x 128 of 2048 13.3 / 11.4."""
+    if not 0 < m <= 13312:
+        return False
+    blocks, tiles, pairs = -(-m // 64), -(-n // 256) * -(-k // 256), sms // 2
+    if blocks < 32:
+        return True
+    waves = min(-(-(-(-n // 128) * -(-k // w)) // sms) for w in (128, 192, 256))          # as bones_gemm_bf16_auto chooses
+    direct = 0.27 * waves if waves == 1 or min(n, k) < 256 else 0.31 * -(-tiles // pairs)
+    return blocks * (direct - 0.40 * tiles / pairs) <= (9 if k > 128 else 5) + 1.8e-6 * n * k
+
+
+def _sms(t):
+    return torch.cuda.get_device_properties(t.device).multi_processor_count
 
 
 def _wgrad(dy2, x2, ws):
@@ -128,7 +142,7 @@ def _wgrad(dy2, x2, ws):
                 mm_tn_acc(dy2[:, o:o + w.shape[0]], x2, g)
                 o += w.shape[0]
         return tuple(None for _ in ws)
-    if _wgrad_direct(dy2.shape[1], x2.shape[1], dy2.shape[0]) and all(w.dtype == BF16 for w in ws):
+    if _wgrad_direct(dy2.shape[1], x2.shape[1], dy2.shape[0], _sms(x2)) and all(w.dtype == BF16 for w in ws):
         full = torch.empty(dy2.shape[1], x2.shape[1], dtype=BF16, device=x2.device)
         mm_tn(dy2, x2, full)
         if len(ws) == 1:
@@ -215,7 +229,7 @@ class _MlpFn(torch.autograd.Function):
         m, c = x2.shape
         f, n = w_fc.shape[0], w_proj.shape[0]
         dpre, dx = torch.empty(m, f, dtype=BF16, device=dy.device), torch.empty(m, c, dtype=BF16, device=dy.device)
-        direct = [_wgrad_direct(*s, m) and w.dtype == BF16 and getattr(w, "main_grad", None) is None for w, s in zip(ctx.ws, ((f, c), (n, f)))]
+        direct = [_wgrad_direct(*s, m, _sms(x2)) and w.dtype == BF16 and getattr(w, "main_grad", None) is None for w, s in zip(ctx.ws, ((f, c), (n, f)))]
         g_fc = torch.empty(f, c, dtype=BF16, device=dy.device) if direct[0] else None
         g_proj = torch.empty(n, f, dtype=BF16, device=dy.device) if direct[1] else None
         L.call("bones_mlp_bf16_bwd", dy2.data_ptr(), x2.data_ptr(), h.data_ptr(), w_fc.data_ptr(), w_proj.data_ptr(), dpre.data_ptr(), dx.data_ptr(),
