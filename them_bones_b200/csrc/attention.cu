@@ -655,11 +655,10 @@ static int tmap_rows_3d(CUtensorMap* out, const void* ptr, int B, int T, long lo
 template <int D>
 static int launch_attn_fwd(const CUtensorMap& tq, const CUtensorMap& tv, const AttnParams& p, int sms, cudaStream_t s) {
   constexpr size_t smem = (size_t)(D / 64) * ATOM_BYTES * 7 + FWD_BARS + 2048 + FWD_SLACK;   // tiles, barriers, row-sum scratch, alignment slack
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(attn_fwd_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done = true;
-  }
+  });
   const long long items = (long long)((p.T + AT - 1) / AT) * p.H * p.B;
   const unsigned grid = (unsigned)(items < sms ? items : sms);       // persistent: one CTA per SM
   attn_fwd_kernel<D><<<grid, FWD_THREADS, smem, s>>>(tq, tv, p);

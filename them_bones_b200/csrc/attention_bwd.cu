@@ -382,11 +382,10 @@ int bones_attn_bwd(const void* qk, const void* qkv, const void* dy, const float*
   p.lse = lse; p.delta = delta; p.dqk = dqk; p.dv = (__nv_bfloat16*)dv;
   p.err = error_word();
   constexpr size_t smem = (size_t)BTILE * 7 + 160 + 1024;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(attn_bwd_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done = true;
-  }
+  });
   dim3 grid(T / BT, H, B);
   attn_bwd_kernel<<<grid, 320, smem, s>>>(tq, tv, td, p);
   return (int)cudaGetLastError();

@@ -977,12 +977,11 @@ template <int D>
 static int launch_split(const CUtensorMap& tq, const CUtensorMap& tv, const CUtensorMap& td, SplitParams p, int* counters, int sms, cudaStream_t s) {
   constexpr size_t smem_dkv = (size_t)dkv_bars(D) + 256 + DKV_SLACK;
   constexpr size_t smem_dq = (size_t)dq_bars(D) + 256 + 1024;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dkv_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dkv));
     BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dq_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_dq));
-    attr_done = true;
-  }
+  });
   const long long items = (long long)(p.Tp / ST) * p.H * p.B;
   const unsigned grid = (unsigned)(items < sms ? items : sms);          // persistent: one CTA per SM in both kernels
   p.items = counters;
@@ -991,11 +990,10 @@ static int launch_split(const CUtensorMap& tq, const CUtensorMap& tv, const CUte
   p.items = counters + 1;
   if (p.ds) {
     constexpr size_t smem_g = (size_t)dqg_bars(D) + 8 * (DQG_NBARS + 2) + 16 + 1024;
-    static bool g_done = false;
-    if (!g_done) {
+    static OncePerDevice limit;
+    BONES_ONCE(limit, {
       BONES_CHECK(cudaFuncSetAttribute(attn_bwd_dq_gemm_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_g));
-      g_done = true;
-    }
+    });
     attn_bwd_dq_gemm_kernel<D><<<grid, DQG_THREADS, smem_g, s>>>(tq, p);
   } else {
     attn_bwd_dq_kernel<D><<<grid, STHREADS, smem_dq, s>>>(tq, tv, td, p);

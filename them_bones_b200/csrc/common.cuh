@@ -12,6 +12,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "per_device.h"
+
 namespace bones {
 
 constexpr long long kWaitLimitCycles = 3000000000LL;   // ~1.5 s at 1.9 GHz
@@ -396,6 +398,17 @@ __device__ __forceinline__ bool bones_index_ok(long long i, long long lo, long l
   do {                                                                         \
     cudaError_t e_ = (x);                                                      \
     if (e_ != cudaSuccess) return (int)e_;                                     \
+  } while (0)
+// The statements `...` (BONES_CHECKs) once on each device, by the static OncePerDevice `once`.
+#define BONES_ONCE(once, ...)                                                  \
+  do {                                                                         \
+    int dev_ = 0;                                                              \
+    BONES_CHECK(cudaGetDevice(&dev_));                                         \
+    const int rc_ = once(dev_, [&]() -> int {                                  \
+      __VA_ARGS__                                                              \
+      return 0;                                                                \
+    });                                                                        \
+    if (rc_ != 0) return rc_;                                                  \
   } while (0)
 
 namespace bones {

@@ -262,12 +262,11 @@ decode_gemm_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
 template <int NB, int EPI>
 static int launch_dec_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const DecGemmParams& p, int S, int pdl, cudaStream_t stream) {
   using G = DgGeom<NB>;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(decode_gemm_kernel<NB, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)G::kSmem));
     BONES_CHECK(cudaFuncSetAttribute(decode_gemm_kernel<NB, EPI>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-    attr_done = true;
-  }
+  });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   cfg.gridDim = dim3((unsigned)(p.N / 128 * S));
@@ -277,8 +276,15 @@ static int launch_dec_gemm(const CUtensorMap& tw, const CUtensorMap& tx, const D
   cfg.attrs = at;
   cfg.numAttrs = (unsigned)dec_launch_attrs(at, S, pdl);
   if (S > 8) {                                 // more than the portable cluster size: a device may have no room for one
-    static int room = -1;
-    if (room < 0) BONES_CHECK(cudaOccupancyMaxActiveClusters(&room, decode_gemm_kernel<NB, EPI>, &cfg));
+    static OncePerDevice asked;
+    static int rooms[OncePerDevice::kDevices] = {0};
+    int dev = 0, room = 0;
+    BONES_CHECK(cudaGetDevice(&dev));
+    BONES_ONCE(asked, {
+      BONES_CHECK(cudaOccupancyMaxActiveClusters(&room, decode_gemm_kernel<NB, EPI>, &cfg));
+      if (dev < OncePerDevice::kDevices) rooms[dev] = room;
+    });
+    if (dev < OncePerDevice::kDevices) room = rooms[dev];
     if (room == 0) return launch_dec_gemm<NB, EPI>(tw, tx, p, 8, pdl, stream);
   }
   return (int)cudaLaunchKernelEx(&cfg, decode_gemm_kernel<NB, EPI>, tw, tx, p);

@@ -394,11 +394,10 @@ constexpr int DR_SMEM_AIM = 190 * 1024;
 
 template <int EPI, bool SPLIT>
 static int launch_rows(const CUtensorMap& tw, const CUtensorMap& tx, const DecRowsParams& p, int S, int ctas, int smem, int pdl, cudaStream_t stream) {
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(decode_rows_kernel<EPI, SPLIT>, cudaFuncAttributeMaxDynamicSharedMemorySize, DR_SMEM_MAX));
-    attr_done = true;
-  }
+  });
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at[2];
   cfg.gridDim = dim3((unsigned)ctas);

@@ -1018,12 +1018,11 @@ int bones_softcap_ce(const void* logits, long long ldl, const long long* targets
   aux.tg[0] = tg2; aux.w[0] = w2; aux.tg[1] = tg3; aux.w[1] = w3; aux.nll_aux = nll_aux;
   aux.smooth = label_smoothing;
   if (V <= 65536 && V >= 8192 && ((uintptr_t)logits % 16) == 0) {
-    static bool attr_set = false;
-    if (!attr_set) {
+    static OncePerDevice limit;
+    BONES_ONCE(limit, {
       BONES_CHECK(cudaFuncSetAttribute(softcap_ce_row_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, CE_SMEM_BYTES));
       BONES_CHECK(cudaFuncSetAttribute(softcap_ce_row_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, CE_SMEM_BYTES));
-      attr_set = true;
-    }
+    });
     int dev = 0, sms = 0;
     BONES_CHECK(cudaGetDevice(&dev));
     BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -419,11 +419,10 @@ int bones_gemm_bf16_pair(const void* A, const void* B, void* D, const void* R, i
   if (rc) return rc;
   rc = operand_tmap2(&tb, B, b_major, N, K, ldb, strideB, batch);
   if (rc) return rc;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
-    attr_done = true;
-  }
+  });
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
   BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
@@ -478,11 +477,10 @@ int bones_logits_stats(const void* x, const void* w, void* D, int M, int N, int 
   if (rc) return rc;
   rc = operand_tmap2(&tb, w, 0, N, K, ldw, 0, 1);
   if (rc) return rc;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(gemm_bf16_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
-    attr_done = true;
-  }
+  });
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
   BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

@@ -1055,13 +1055,12 @@ int bones_mx2_quant(const void* x, long long ldx, void* qr, void* sfr, int group
   const unsigned grid = (unsigned)std::min<long long>(sms, (tiles + kWarps - 1) / kWarps);
   int* err = error_word();
   using G = QdGeom<kHalves, kWarps>;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(mx_quant_dual_kernel<true, true, kHalves, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes));
     BONES_CHECK(cudaFuncSetAttribute(mx_quant_dual_kernel<true, false, kHalves, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes));
     BONES_CHECK(cudaFuncSetAttribute(mx_quant_dual_kernel<false, true, kHalves, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::kSmemBytes));
-    attr_set = true;
-  }
+  });
 #define BONES_QUANT_LAUNCH(ROW, COL)                                                                                          \
   mx_quant_dual_kernel<ROW, COL, kHalves, kWarps><<<grid, kWarps * 32, G::kSmemBytes, (cudaStream_t)stream>>>(                 \
       (const __nv_bfloat16*)x, ldx, (uint8_t*)qr, (uint8_t*)sfr, group_r, (uint8_t*)qc, (uint8_t*)sfc, group_c, R, C, (uint32_t)rows_per, \
@@ -1156,14 +1155,13 @@ int bones_gemm_mxfp8_pair(const void* Aq, const void* sfa, const void* Bq, const
     if (rc) return rc;
   }
   constexpr size_t smem = QSMEM_BYTES;
-  static bool attr_set = false;
-  if (!attr_set) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<kEpiWarpsQ, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     BONES_CHECK(cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<kEpiWarpsQ, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     BONES_CHECK(cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<kEpiWarpsQ, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     BONES_CHECK(cudaFuncSetAttribute(gemm_mxfp8_pair_kernel<kEpiWarpsQ, 3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_set = true;
-  }
+  });
   int dev = 0, sms = 0;
   BONES_CHECK(cudaGetDevice(&dev));
   BONES_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));

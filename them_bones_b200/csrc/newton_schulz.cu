@@ -533,11 +533,10 @@ int bones_newton_schulz(const void* x0, void* x1, void* x2, void* g, void* b, in
   rc = ns_tmap(&maps.b, b, p.s, p.s, n, 128);
   if (rc) return rc;
   constexpr size_t smem = (size_t)NSTAGES * NSTAGE_BYTES + 8 * (2 * NSTAGES + 15) + 16 + 1024;
-  static bool attr_done = false;
-  if (!attr_done) {
+  static OncePerDevice limit;
+  BONES_ONCE(limit, {
     BONES_CHECK(cudaFuncSetAttribute(newton_schulz_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    attr_done = true;
-  }
+  });
   BONES_CHECK(cudaMemsetAsync(scratch, 0, sizeof(int) * (1 + 3 * (size_t)steps * n), (cudaStream_t)stream));
   const int pairs = p.total < sms / 2 ? p.total : sms / 2;
   newton_schulz_kernel<<<2 * pairs, NS_THREADS, smem, (cudaStream_t)stream>>>(maps, p);
