@@ -185,7 +185,8 @@ def rows_plan(b, n, k, sms):
         if fit:
             return (fit[0] if s < 4 else fit[-1]), s
     # few columns: the most CTAs with parts of 256 or more (256 wide: 121 us a step of six layers for 150 at batch 64, 107 for 110 at 8)
-    few = [(n // nt * s, -s, nt) for nt in (16, 32, 64) for s in (1, 2, 4, 8) if (s == 1 or k >= 256 * s) and k <= 1536 * s and n // nt * s < sms // 2]
+    few = [(n // nt * s, -s, nt) for nt in (16, 32, 64) for s in (1, 2, 4, 8)
+           if n % nt == 0 and (s == 1 or k >= 256 * s) and k <= 1536 * s and n // nt * s < sms // 2]
     return (max(few)[2], -max(few)[1]) if few else None
 
 
