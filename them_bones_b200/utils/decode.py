@@ -184,7 +184,7 @@ def rows_plan(b, n, k, sms):
         fit = [nt for nt in (64, 48, 40, 32) if n % nt == 0 and sms // 2 <= n // nt * s <= (sms if s < 4 else int(0.9 * sms))]
         if fit:
             return (fit[0] if s < 4 else fit[-1]), s
-    # few columns: the most CTAs with parts of 256 or more (256 wide: 121 us a step of six layers for 150 at batch 64, 107 for 110 at 8)
+    # few columns: the most CTAs with parts of 256 or more (256 wide: 115 us a step of six layers for 145 at batch 64, 103 for 106 at 8)
     few = [(n // nt * s, -s, nt) for nt in (16, 32, 64) for s in (1, 2, 4, 8)
            if n % nt == 0 and (s == 1 or k >= 256 * s) and k <= 1536 * s and n // nt * s < sms // 2]
     return (max(few)[2], -max(few)[1]) if few else None
@@ -192,11 +192,24 @@ def rows_plan(b, n, k, sms):
 
 def use_rows(b, c, a, hidden, sms):
     """Whether the layers' projections run on ``csrc/decode_rows.cu``: all four or none, since two of its CTAs, or one and one of the other
-    kernel's, do not share an SM (2048 wide, ``out`` alone on it: 10 to 15 % slower).  Narrow models with few sequences stay on the
-    other kernel, whose clusters split their short contractions further (512 and 768 wide, up to 16 sequences: 2 to 6 % faster)."""
-    if c < 1024 and b <= 16:
+    kernel's, do not share an SM (2048 wide, ``out`` alone on it: 10 to 15 % slower).  Between 256 and 896 wide, models with few sequences
+    stay on the other kernel, whose clusters split their contractions further.  Six layers, us a step here / there: 128 wide at batch 1 / 8 /
+    16 88 / 93, 92 / 98, 94 / 100; 256 98 / 98, 103 / 106, 105 / 108; 384 113 / 107, 116 / 116, 118 / 118, at 20 121 / 128; 512 121 / 115, 125 / 121,
+    127 / 126, at 20 132 / 132; 640 125 / 124, 129 / 131, 131 / 135; 768 134 / 133, 138 / 141, 137 / 141; 896 138 / 144, 138 / 149, 142 / 153."""
+    if 256 < c < 896 and b <= 16:
         return False
     return all(rows_plan(b, n, k, sms) is not None for n, k in ((3 * a, c), (c, a), (hidden, c), (c, hidden)))
+
+
+def head_on_rows(b, n, k):
+    """Whether the head ``[n, k]`` of a step whose layers run on ``csrc/decode_rows.cu`` runs there too, its tiles walked by one CTA an SM.
+
+    Above 32 sequences the other kernel pads to 64 and holds one CTA an SM; up to 16 it is the faster everywhere.  Between, what counts is
+    the head's bytes.  A tile of a short contraction costs more here than there.  us a step of four layers here / there: 1280 x 65536 at
+    batch 12 142.0 / 141.6, 20 143.8 / 142.5, 28 145.8 / 144.7, 33 148 / 158, 40 149 / 156, 64 157 / 160; 1024 x 32768 at 20 115.5 / 114.5, 33
+    117.6 / 118.9, 64 125 / 127; 1536 x 65536 at 18 164.7 / 165.8, 28 169 / 170.5, 33 166 / 176; 1024 x 131072 at 18 158 / 162, 28 161 / 168, 64 169 /
+    190.  Of six layers: 256 x 65536 at 20 129 / 122, 64 133.5 / 130, 256 x 8192 at 64 the same; 768 x 32768 at 40 160.5 / 158."""
+    return (b > 32 and (k >= 1024 or n <= 16384)) or (b > 16 and n * k >= 100_000_000)
 
 
 class NativeDecoder:
@@ -271,9 +284,8 @@ class NativeDecoder:
         from ..ops import _lib as L
         b, (n, k) = x.shape[0], w.shape
         x0, ma, mb = (self.x0, mix[0], mix[1]) if mix is not None else (None, None, None)
-        # the head: CTAs that walk its tiles, 0.5 to 1 % of a step from 40 sequences on, as much the other way at 4
         head = epi == 3
-        plan = None if not self.rows else rows_plan(b, n, k, self.sms) if not head else (64, 1) if b > 16 else None
+        plan = None if not self.rows else rows_plan(b, n, k, self.sms) if not head else (64, 1) if head_on_rows(b, n, k) else None
         cap = ctypes.c_float(self.model.config.softcap)
         if plan is not None:
             nt, splits = plan
