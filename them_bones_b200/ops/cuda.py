@@ -8,6 +8,7 @@ optimizer's buffer, ``GradFoldIn`` round2/source/train.py:4677-4723 and ``_Linea
 from __future__ import annotations
 
 import ctypes
+import functools
 import os
 
 import torch
@@ -114,8 +115,9 @@ def _wgrad_direct(n, k, m, sms=148):
     return blocks * (direct - 0.40 * tiles / pairs) <= (9 if k > 128 else 5) + 1.8e-6 * n * k
 
 
-def _sms(t):
-    return torch.cuda.get_device_properties(t.device).multi_processor_count
+@functools.lru_cache(maxsize=None)
+def _sms(device):
+    return torch.cuda.get_device_properties(device).multi_processor_count
 
 
 def _wgrad(dy2, x2, ws):
@@ -142,7 +144,7 @@ def _wgrad(dy2, x2, ws):
                 mm_tn_acc(dy2[:, o:o + w.shape[0]], x2, g)
                 o += w.shape[0]
         return tuple(None for _ in ws)
-    if _wgrad_direct(dy2.shape[1], x2.shape[1], dy2.shape[0], _sms(x2)) and all(w.dtype == BF16 for w in ws):
+    if _wgrad_direct(dy2.shape[1], x2.shape[1], dy2.shape[0], _sms(x2.device)) and all(w.dtype == BF16 for w in ws):
         full = torch.empty(dy2.shape[1], x2.shape[1], dtype=BF16, device=x2.device)
         mm_tn(dy2, x2, full)
         if len(ws) == 1:
@@ -229,7 +231,7 @@ class _MlpFn(torch.autograd.Function):
         m, c = x2.shape
         f, n = w_fc.shape[0], w_proj.shape[0]
         dpre, dx = torch.empty(m, f, dtype=BF16, device=dy.device), torch.empty(m, c, dtype=BF16, device=dy.device)
-        direct = [_wgrad_direct(*s, m, _sms(x2)) and w.dtype == BF16 and getattr(w, "main_grad", None) is None for w, s in zip(ctx.ws, ((f, c), (n, f)))]
+        direct = [_wgrad_direct(*s, m, _sms(x2.device)) and w.dtype == BF16 and getattr(w, "main_grad", None) is None for w, s in zip(ctx.ws, ((f, c), (n, f)))]
         g_fc = torch.empty(f, c, dtype=BF16, device=dy.device) if direct[0] else None
         g_proj = torch.empty(n, f, dtype=BF16, device=dy.device) if direct[1] else None
         L.call("bones_mlp_bf16_bwd", dy2.data_ptr(), x2.data_ptr(), h.data_ptr(), w_fc.data_ptr(), w_proj.data_ptr(), dpre.data_ptr(), dx.data_ptr(),
