@@ -19,8 +19,9 @@
 //     to choose what it requests early, and reads it again behind the wait.)
 // Warp 0 issues the TMA loads, warp 1 the MMAs, the others run the epilogue.
 //
-// Up to 64 sequences the layers' projections run on decode_rows.cu, whose tiles exchange no partial sums or small ones; this kernel has the
-// head and more sequences.  What bounds it is a chain of latencies: per projection about 1.1 us from the previous kernel's end to this
+// Up to 64 sequences most layers' projections, and most heads of more than 32, run on decode_rows.cu, whose tiles exchange no partial sums or small
+// ones (`use_rows` and `head_on_rows` in utils/decode.py); this kernel has the rest: more sequences, other heads, models wider than 1536 and
+// narrow ones with few sequences.  What bounds it is a chain of latencies: per projection about 1.1 us from the previous kernel's end to this
 // one's start, 1.5 to 4 us until the accumulator is complete, 1.3 to 2.9 us for the exchange, 0.7 to 1.3 us of epilogue.
 #include "decode_common.cuh"
 

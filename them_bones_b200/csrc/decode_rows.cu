@@ -18,9 +18,11 @@
 //     loads of the residual and stores, squares' sums without shuffles.
 //   * With many tiles the CTAs are persistent with two accumulators, and the rings run on across tiles.
 // 20 layers, 1280 wide, head of 65536, us a step at position 64, with decode_gemm.cu's kernel for all projections and with this one: batch 64
-// 810 -> 640, 40 804 -> 605, 16 603 -> 545, 4 562 -> 520 (two runs within 1 %).  A layer takes 33 us at batch 64: qkv 6.2, attention 10 (its keys and
-// values move at the copy rate), out 4.2, c_fc 5.7, c_proj 7.3; of each about 1.1 us lie between one kernel's last store and the next
-// one's start, 0.8 us until the first rows of X arrive, and the MMAs of K = 1280 take 1.7 us at least (35 clocks each, 64 x nt x 16).
+// 810 -> 640, 40 804 -> 605, 16 603 -> 545, 4 562 -> 520 (two runs within 1 %).  A layer takes 33 us at batch 64: qkv 6.2, attention 10 (21 MB of
+// keys and values, 3.2 us at the copy rate: its chain of waits, rounds of keys and sums is what takes the time there), out 4.2, c_fc 5.7, c_proj
+// 7.3; of each about 1.1 us lie between one kernel's last store and the next one's start, 0.8 us until the first rows of X arrive, and the
+// MMAs of K = 1280 take 1.7 us at least (35 clocks each, 64 x nt x 16).  All CTAs together read X 13 to 20 MB worth from L2, more than the
+// weights of qkv and c_proj.
 #include "decode_common.cuh"
 
 namespace bones {
@@ -99,7 +101,8 @@ decode_rows_kernel(const __grid_constant__ CUtensorMap tm_w, const __grid_consta
   const int first = blockIdx.x / S, step = gridDim.x / S;
   const int k0 = p.KS * rank / S, k1 = p.KS * (rank + 1) / S;
   // The CTAs begin at different places of the contraction and wrap around: they all read the same X, and in step they would all ask
-  // the same few lines of L2 at a time.
+  // the same few lines of L2 at a time.  A column's place follows its CTA, so where CTAs walk several tiles (the head) the order of
+  // its sum, and with it the last bits, depends on the number of SMs; on one device every call gives the same bits.
   const int turn = first % (k1 - k0);
   auto at_k = [&](int k) { return k + turn < k1 ? k + turn : k + turn - (k1 - k0); };
   const uint32_t tcols = p.nt > 32 ? 64u : 32u;                          // columns between the two accumulators

@@ -144,7 +144,8 @@ def projection_splits(b, n, k, residual, sms):
     SM, 1.25 where clusters of 8 meet 17 to 32 sequences, one above 64 sequences and 0.8 of clusters of four or more (16 tiles
     by 8 CTAs: 524 us where 4 take 480).
 
-    Six layers, us a step, this rule against 2 CTAs for every projection of more than ten tiles and at most 160 CTAs: 1280 wide the
+    Six layers, us a step, all layers on this kernel, this rule against 2 CTAs for every projection of more than ten tiles and at most 160
+    CTAs (``use_rows`` takes 1280 and 1408 wide up to 64 sequences to the other kernel, where they are faster still): 1280 wide the
     same (batch 64 242, batch 24 186, batch 8 171); 1408 wide 256 for 342 at batch 64, 336 for 399 at 128; 2048 wide 349 for 441, 437 for 515,
     246 for 253 at batch 8; 256 wide 145 for 148 and 204 for 212; 512 to 1152 wide the same.
     """
