@@ -419,7 +419,7 @@ using namespace bones;
 
 // As bones_decode_gemm for b <= 64 and K a multiple of 128, in tiles of `nt` columns (a multiple of 8 from 16 to 64 that divides N);
 // ssq_out is [N / nt, b].  `splits` (1, 2, 4 or 8, at most K / 128): CTAs of a cluster that share a tile's contraction.  `ctas`: without a split,
-// how many CTAs walk the tiles (0: one for each).
+// how many CTAs walk the tiles (0: one for each).  The soft-cap comes without a split only.
 int bones_decode_rows(const void* X, const void* W, void* out, int b, int N, int K, int nt, int splits, int ctas, int epi, const float* ssq_in, int n_ssq,
                       const void* res, const void* x0, const float* mix_a, const float* mix_b, float* ssq_out, float cap, const void* next_w, long long next_bytes, int pdl, void* stream) {
   if (b < 1 || b > 64 || N <= 0 || K <= 0 || (K % 128) || nt < 16 || nt > 64 || (nt % 8) || (N % nt)) return -2;
@@ -468,7 +468,7 @@ int bones_decode_rows(const void* X, const void* W, void* out, int b, int N, int
     case DEC_SCALE: return BONES_ROWS(DEC_SCALE);
     case DEC_RELU2: return BONES_ROWS(DEC_RELU2);
     case DEC_RES: return BONES_ROWS(DEC_RES);
-    case DEC_SOFTCAP: return BONES_ROWS(DEC_SOFTCAP);
+    case DEC_SOFTCAP: return splits > 1 ? -2 : launch_rows<DEC_SOFTCAP, false>(tw, tx, p, 1, grid, smem, pdl, s);      // a head has tiles enough
   }
 #undef BONES_ROWS
   return -2;
