@@ -248,12 +248,12 @@ __device__ __forceinline__ int attn_first_tile(const AttnParams& p, int doc, int
 //   exponentials, so S(g + 1) and its latency (PV, S and their hand-overs are 1 400 clocks) lie under two tiles of exponentials.
 // What bounds it now is the special-function units: a 128 x 128 tile's exponentials are 1 024 clocks, with sixteen warps 1 300 of the
 // 1 830 that a tile takes (2 770 with both products issued by one warp, the items drawn behind the last load and the output
-// drained by the softmax warps).  us: 16 x 2048 tokens in documents, 10 heads of 128, 141 -> 121; 8 x 2048 causal 107 -> 90; 8 x 1777 in
-// documents 73 -> 64; a window of 256 42.5 -> 40.5.
+// drained by the softmax warps).  us: 16 x 2048 tokens in documents, 10 heads of 128, 133 -> 114; 8 x 2048 causal 104 -> 89; 4 x 2048 in
+// documents 44.7 -> 37.0; a window of 256 at 16 x 2048 67 -> 58.
 // With a tile or two a CTA the longer chain of roles cost 0.3 to 0.7 us; what took it back: a CTA's first item is its own number (no
 // counter, no ring), its Q is requested before its document start is known, and an item's coordinates are divided out once, not again before its
-// loads.  us with the counter's zero fill, one warp for both products / drawn first item / now: 4 x 256, 4 heads of 64 8.5 / 9.2 / 8.5; 8 x 100
-// 7.4 / 8.1 / 7.3; 10 heads of 128: 1 x 128 8.4 / 8.8 / 8.0, 8 x 128 8.8 / 9.2 / 8.6, 16 x 512 in documents 28.3 / 25.8 / 22.0.
+// loads.  us with the counter's zero fill, one warp for both products / drawn first item / now: 4 x 256, 4 heads of 64 8.5 / 9.2 / 8.6; 8 x 100
+// 7.4 / 8.1 / 7.3; 10 heads of 128: 1 x 128 8.4 / 8.8 / 7.9, 8 x 128 8.8 / 9.2 / 8.5, 16 x 512 in documents 28.3 / 25.8 / 22.0.
 // Tried and slower: two query tiles at a time with four warps each and shared K/V (8 x 2048 causal 129: the two fall in step, both
 // in their exponentials and then both waiting for MMAs), two groups of eight warps with items of their own (127).
 //   smem: Q x 2 (item parity), K x 2 and V x 3 stages (running tile count): a K stage is free again once its S tile is
@@ -373,9 +373,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tm_qk, const __grid_constant
     // Q and K loads, and the items: the next one is drawn, its document start read, and it is handed round and its Q requested one step
     // a tile over the last tiles of the item before, so nobody waits for either latency (drawn and published behind the last
     // load, it held the scores up for about 3 500 clocks an item).
-    // three tiles ahead, us: 16 x 2048 tokens in documents 121, two ahead 125, one 129; few items: two, so that the next one goes to a
-    // CTA that needs it soon (16 x 512 tokens 26.0 for 26.4)
-    const int ahead = total >= 6 * (int)gridDim.x ? 3 : 2;
+    // From two tiles ahead on.  One / two / three, us: 16 x 2048 tokens in documents 114.6 / 113.8 / 114.2, with a window of 256 59.2 / 58.3 / 58.4;
+    // calls of few items the same.
+    constexpr int ahead = 2;
     int g = 0, it = 0, w = (int)blockIdx.x, kt0 = kt_first;
     bool dead = false;
     FwdItem after = first;
